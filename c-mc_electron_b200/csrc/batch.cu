@@ -115,10 +115,12 @@ void build_tables(mcb200_batch *b) {
     base.seed = b->cfg[k].seed;
     base.step = b->member_step[k];  // advanced with b->steps after every step
     base.n = c->dev_counts;
+    base.listed = c->tickets + 1 + mcb200_ctx::kGenerations;
     base.capacity = (int)c->capacity;
     for (int par = 0; par < 2; ++par) {
       BatchInstT<R> e = base;
       e.P = store<R>(c, par == 0 ? c->cur : 1 - c->cur);
+      e.list = store<R>(c, par == 0 ? 1 - c->cur : c->cur).uid;  // free until the step's sort
       e.C = children<R>(c, 0);
       t[(size_t)par * n + k] = e;
     }
@@ -219,13 +221,17 @@ void batch_transport(mcb200_batch *b, uint64_t early = 0) {
   if (batched) {
     if (early) {
       ck(cudaMemsetAsync(side_ticket, 0, sizeof(unsigned int), b->side), "memset");
-      ck(cudaEventRecord(b->ev_side0, b->side), "event");  // the side counter is reset
+      if (launch_batch_drift<R>(F, tab + (size_t)flip * n, n, early, sms, b->side))
+        throw std::runtime_error("batched drift launch failed");
+      ck(cudaEventRecord(b->ev_side0, b->side), "event");  // the side counter is reset, the lists are made
       if (launch_batch_flight<R>(F, tab + (size_t)flip * n, n, early, b->steps, false, side_ticket, 1, sms, b->side,
                                  b->smem_table))
         throw std::runtime_error("batched flight launch failed");
       ck(cudaEventRecord(b->ev_side, b->side), "event");
     }
     ck(cudaMemsetAsync(b->tickets, 0, sizeof(unsigned int) * (1 + mcb200_ctx::kGenerations), b->stream), "memset");
+    if (launch_batch_drift<R>(F, tab + (size_t)flip * n, n, batched & ~early, sms, b->stream))
+      throw std::runtime_error("batched drift launch failed");
     if (launch_batch_flight<R>(F, tab + (size_t)flip * n, n, batched & ~early, b->steps, false, b->tickets,
                                b->blocks_per_sm, sms, b->stream, b->smem_table))
       throw std::runtime_error("batched flight launch failed");
@@ -240,6 +246,7 @@ void batch_transport(mcb200_batch *b, uint64_t early = 0) {
       if (launch_batch_flight<R>(F, tab + (size_t)(2 + g) * n, n, batched, b->steps, true, b->tickets + 1 + g,
                                  b->blocks_per_sm, sms, b->stream, b->smem_table))
         throw std::runtime_error("batched copy flight launch failed");
+    // (a drift pass and its flight count as one)
     b->launches += 2 + mcb200_ctx::kGenerations + (early ? 2 : 0);
   }
   ck(cudaEventRecord(b->ev_flight, b->stream), "event");

@@ -59,6 +59,22 @@ struct DevTables32 {
   const float *gamtet, *energy, *sumscatt, *scatte, *dose, *scattiie, *scatth, *dosh, *scattiih, *dostetmax;
 };
 
+// Constants in the flight's arithmetic, each rounded as the reference's
+// expression for it is (host, once): the device would convert, divide and
+// take roots of them at every event.
+template <typename R>
+struct FlightConstT {
+  R a0pi, emax, dtable, dlist, dlists;
+  R grid_lo[3], grid_inv[3], seed_inv[3];
+  // the Brooks-Herring event and its rate's floor
+  R shift;            // 0.85 a0pi, the valley's centre
+  R in_l, in_t;       // sqrt(meld / mell), sqrt(meld / melt)
+  R out_l, out_t;     // sqrt(mell / meld), sqrt(melt / meld)
+  R ml, mt;           // mell / meld, melt / meld
+  R meld, melt, two_meld;
+  R gamma_floor;      // 1 / scrt0
+};
+
 struct DevTables {
   int nt, nk, nbt;
   int nband[3], bandof[3];
@@ -103,6 +119,7 @@ struct DevTables {
   const int *seed_grid;
   // symmetry (copied to shared memory by each block)
   const int *symi;            // [48*6] matsym[c][s] stored as s*6+c
+  const uint32_t *sym_packed; // [48] the same operation in one word (pack_symmetry)
   const int *newisym;         // [5][48]
   const double *bz;           // [3][5][48]  (xbz, ybz, zbz)
   const int *indmat;          // [729]
@@ -110,6 +127,8 @@ struct DevTables {
   // phonon dispersion tables (FullBandTables::dispersion; null when absent)
   const double *disp;
   int disp_off[6];
+  FlightConstT<double> k64;
+  FlightConstT<float> k32;
   DevTables32 f32;            // FP32 flight tables (null until a context selects FP32 flight)
 };
 
@@ -133,6 +152,10 @@ struct DevMesh {
   // bh_b), (bh_emax, bh_beta, bh_ecut, 0) -- the fields and the
   // Brooks-Herring factors in float, rebuilt before each FP32 step
   const float4 *cell32;         // [cells][3]
+  // FP64 flight: per cell the Brooks-Herring factors that depend on the cell
+  // alone, {doping meld (0: no rate), eebeta meld}, {pi (frickel rho)^2, peak
+  // energy}, {beta^2, 0}, rebuilt before each FP64 step
+  const double2 *cell64;        // [cells][3]
   int surface_dir[kMaxSurfaces];
   int surface_scatter;          // Flag_SurfaceScatter
   int surface_impurity;         // Flag_SurfaceImpurityScatter
@@ -234,6 +257,19 @@ struct ChildSetT {
     return at;
   }
 };
+
+// One symmetry operation in a word.  out[c] = sign_c * in[p_c] takes a wedge
+// vector to the zone; bits 0-5: p_0, p_1, p_2; bits 6-11: the inverse
+// permutation (the c with p_c = j); bits 31, 30, 29: set where sign_0, sign_1,
+// sign_2 is -1.
+inline uint32_t pack_symmetry(const int *op) {  // op: {p_0 + 1, p_1 + 1, p_2 + 1, sign_0, sign_1, sign_2}
+  uint32_t w = 0;
+  for (int c = 0; c < 3; ++c) {
+    const uint32_t p = (uint32_t)(op[c] - 1);
+    w |= p << (2 * c) | (uint32_t)c << (6 + 2 * p) | (op[3 + c] < 0 ? 0x80000000u >> c : 0u);
+  }
+  return w;
+}
 
 inline __host__ __device__ uint32_t pack_cell(int i, int j, int k) {
   return (uint32_t)i | ((uint32_t)j << 10) | ((uint32_t)k << 20);

@@ -240,6 +240,31 @@ void upload_tables32(mcb200_ctx *c, const std::vector<TetFlight> &tf, const std:
   d.dostetmax = dupload(to_float(t.dostetmax), c->ts->owned);
 }
 
+template <typename R>
+void flight_constants(const DevTables &d, FlightConstT<R> &k) {
+  k.a0pi = (R)d.a0pi;
+  k.emax = (R)d.emax;
+  k.dtable = (R)d.dtable;
+  k.dlist = (R)d.dlist;
+  k.dlists = (R)d.dlists;
+  for (int a = 0; a < 3; ++a) {
+    k.grid_lo[a] = (R)d.grid_lo[a];
+    k.grid_inv[a] = (R)d.grid_inv[a];
+    k.seed_inv[a] = (R)d.seed_inv[a];
+  }
+  k.shift = (R)0.85 * (R)d.a0pi;
+  k.in_l = std::sqrt((R)(d.meld / d.mell));
+  k.in_t = std::sqrt((R)(d.meld / d.melt));
+  k.out_l = std::sqrt((R)(d.mell / d.meld));
+  k.out_t = std::sqrt((R)(d.melt / d.meld));
+  k.ml = (R)(d.mell / d.meld);
+  k.mt = (R)(d.melt / d.meld);
+  k.meld = (R)d.meld;
+  k.melt = (R)d.melt;
+  k.two_meld = (R)(2.0 * d.meld);
+  k.gamma_floor = (R)(1.0 / d.scrt0);
+}
+
 void upload_tables(mcb200_ctx *c) {
   const FullBandTables &t = c->ts->tab;
   DevTables &d = c->ts->dt;
@@ -316,7 +341,10 @@ void upload_tables(mcb200_ctx *c) {
                        (t.matsym[1][s] - 1)) * 3 + (t.matsym[2][s] - 1);
       refl[axis * 48 + s] = t.indmat[idx];
     }
+  std::vector<uint32_t> packed(48);
+  for (int s = 0; s < 48; ++s) packed[s] = pack_symmetry(&symi[s * 6]);
   d.symi = dupload(symi, c->ts->owned);
+  d.sym_packed = dupload(packed, c->ts->owned);
   d.newisym = dupload(newisym, c->ts->owned);
   d.bz = dupload(bz, c->ts->owned);
   d.indmat = dupload(indmat, c->ts->owned);
@@ -324,6 +352,8 @@ void upload_tables(mcb200_ctx *c) {
   d.disp = t.dispersion.empty() ? nullptr : dupload(t.dispersion, c->ts->owned);
   for (int i = 0; i < kDispTables; ++i) d.disp_off[i] = t.disp_off[i];
   build_kgrid(c, 40);
+  flight_constants(d, d.k64);
+  flight_constants(d, d.k32);
   upload_tables32(c, tf, ts, kn);
   c->ts->vmax = 0;
   for (size_t q = 0; q < t.vt.size(); ++q)
@@ -514,7 +544,7 @@ void init_device_context(mcb200_ctx *c, size_t max_particles) {
   c->append_count = dalloc<unsigned int>(1, c->owned);
   c->bounds = dalloc<unsigned long long>(4, c->owned);
   ck(cudaMemsetAsync(c->bounds, 0, 4 * sizeof(unsigned long long), c->stream), "memset");
-  c->tickets = dalloc<unsigned int>(1 + mcb200_ctx::kGenerations, c->owned);
+  c->tickets = dalloc<unsigned int>(2 + mcb200_ctx::kGenerations, c->owned);
   c->y.counters = dalloc<unsigned long long>(kCntNumCounters, c->owned);
   c->y.contact = dalloc<long long>(kMaxContacts * 6, c->owned);
   c->total = dalloc<unsigned int>(1, c->owned);
@@ -740,6 +770,7 @@ int mcb200_set_mesh(mcb200_ctx *c, int nx, int ny, int nz, const double *lx, con
     c->y.heat_e = dalloc<long long>(nodes, c->mesh_owned);
     c->y.heat_h = dalloc<long long>(nodes, c->mesh_owned);
     c->cell32 = dalloc<float4>(cells * 3, c->mesh_owned);
+    c->cell64 = dalloc<double2>(cells * 3, c->mesh_owned);
     c->sb.nodes = (int)nodes;
     c->sb.node = dalloc<long long>(nodes * 10, c->mesh_owned);
     c->sb.cell_count = dalloc<unsigned long long>(cells, c->mesh_owned);
@@ -758,6 +789,7 @@ int mcb200_set_mesh(mcb200_ctx *c, int nx, int ny, int nz, const double *lx, con
     c->surf_cached = false;
     c->stat_open = false;
     m.cell32 = c->cell32;
+    m.cell64 = c->cell64;
     c->hist = dalloc<unsigned int>(cells, c->mesh_owned);
     ck(cudaMemsetAsync(c->hist, 0, sizeof(unsigned int) * cells, c->stream), "memset");  // zero between sorts
     c->offsets = dalloc<unsigned int>(cells, c->mesh_owned);
@@ -2012,13 +2044,13 @@ void step_prepare(mcb200_ctx *c) {
                            c->ts->dt, c->ib, grid_for(c, c->capacity, 256), s);
     c->launches += 2;
   }
-  StepCounters z{c->tickets, {}, c->append_count};
+  StepCounters z{c->tickets, {}, c->append_count, c->tickets + 1 + mcb200_ctx::kGenerations};
   for (int g = 0; g < mcb200_ctx::kGenerations; ++g) z.count[g] = children<R>(c, g).count;
   z.count[mcb200_ctx::kGenerations] = c->sink_count;
-  if constexpr (sizeof(R) == 4)  // FP32 flight reads the fields as per-cell float records
+  if constexpr (sizeof(R) == 4)  // the per-cell records the flight reads
     launch_records_and_reset(c->ts->dt, c->mesh, c->cell32, c->ncells, z, s);
   else
-    launch_step_reset(z, s);
+    launch_records_and_reset(c->ts->dt, c->mesh, c->cell64, c->ncells, z, s);
   c->launches += 1;
   join_stat(c);  // the flights change the store the statistics read (the records and counters do not)
 }
@@ -2065,11 +2097,13 @@ void enqueue_flights(mcb200_ctx *c, FlightCtxT<R> F, cudaEvent_t *ev) {
   cudaStream_t s = c->stream;
   F.C = children<R>(c, 0);
   if (ev) ck(cudaEventRecord(ev[1], s), "event");
-  launch_flight(F, store<R>(c, c->cur), DevCount{c->dev_counts, nullptr, (int)c->capacity}, c->tickets, c->sm_count,
-                s);
+  // (the list of the particles with events lies in the other buffer, which
+  // the step's sort writes after the flights)
+  launch_flight(F, store<R>(c, c->cur), DevCount{c->dev_counts, nullptr, (int)c->capacity},
+                store<R>(c, 1 - c->cur).uid, c->tickets + 1 + mcb200_ctx::kGenerations, c->tickets, c->sm_count, s);
   ck(cudaGetLastError(), "flight kernel");
   if (ev) ck(cudaEventRecord(ev[2], s), "event");
-  c->launches += 1;
+  c->launches += 2;
   for (int g = 0; g < mcb200_ctx::kGenerations; ++g) {
     if (g + 1 < mcb200_ctx::kGenerations) {
       F.C = children<R>(c, g + 1);

@@ -196,6 +196,7 @@ struct mcb200_ctx {
   unsigned int *finish_blocks = nullptr;  // [2] blocks of the step's scatter / scan done (zero between steps)
   unsigned int *tickets = nullptr;  // work counters of the persistent flight launches (main + generations)
   float4 *cell32 = nullptr;         // FP32 flight's per-cell records (mesh-sized)
+  double2 *cell64 = nullptr;        // FP64 flight's
   // tallies
   DevTallies y{};
   // sort scratch

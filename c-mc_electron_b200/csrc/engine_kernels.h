@@ -13,22 +13,29 @@ template <typename R>
 struct FlightCtxT;
 using FlightCtx = FlightCtxT<double>;
 
-// Persistent flight launches: `ticket` is a zeroed device counter the blocks
-// take particle indices from; the main flight reads its particle count from
-// device memory (n.max sizes the grid), a child generation its own count;
-// n_hint bounds the copies a generation holds.
+// Flight launches: the drift pass over the store's n particles (device
+// count; n.max sizes the grids), which flies those without an event and
+// lists the others (list: room for n.max indices, *listed zeroed), then the
+// persistent flight of the listed ones.  `ticket` is a zeroed device counter
+// the persistent blocks take indices from; a child generation reads its own
+// count; n_hint bounds the copies a generation holds.
 template <typename R>
-void launch_flight(const FlightCtxT<R> &F, const DevParticlesT<R> &P, DevCount n, unsigned int *ticket, int sm_count,
-                   cudaStream_t s);
+void launch_flight(const FlightCtxT<R> &F, const DevParticlesT<R> &P, DevCount n, uint32_t *list,
+                   unsigned int *listed, unsigned int *ticket, int sm_count, cudaStream_t s);
 template <typename R>
 void launch_child_flight(const FlightCtxT<R> &F, const DevChildrenT<R> &in, int n_hint, unsigned int *ticket,
                          int sm_count, cudaStream_t s);
-// One persistent launch flying the particles (child == false) or the copies
+// The drift pass of the simulations k < ninst with bit k of `members` set, in
+// one launch (before their flight).  Returns 0 on success.
+template <typename R>
+struct BatchInstT;
+template <typename R>
+int launch_batch_drift(const FlightCtxT<R> &F, const BatchInstT<R> *inst, int ninst, uint64_t members, int sm_count,
+                       cudaStream_t s);
+// One persistent launch flying the listed particles (child == false) or the copies
 // of one generation (child == true) of the simulations k < ninst with bit k
 // of `members` set (inst: device table of BatchInstT, steps: their step
 // numbers); blocks_per_sm <= 0: as many as fit.  Returns 0 on success.
-template <typename R>
-struct BatchInstT;
 template <typename R>
 int launch_batch_flight(const FlightCtxT<R> &F, const BatchInstT<R> *inst, int ninst, uint64_t members,
                         const uint32_t *steps, bool child, unsigned int *ticket, int blocks_per_sm, int sm_count,
@@ -52,11 +59,13 @@ struct StepCounters {
   unsigned int *tickets;  // [1 + kChildGenerations]
   unsigned int *count[kChildGenerations + 1];
   unsigned int *appended;  // copies appended to the store this step
+  unsigned int *listed;    // particles the drift pass left to the flight
 };
-void launch_step_reset(const StepCounters &z, cudaStream_t s);
-// FP32 flight's per-cell records (DevMesh::cell32), [cells][3] float4, and
-// the step reset of z, in one launch.
+// The flight's per-cell records (DevMesh::cell32, [cells][3] float4, or
+// cell64, [cells][3] double2) and the step reset of z, in one launch.
 void launch_records_and_reset(const DevTables &T, const DevMesh &M, float4 *out, int cells, const StepCounters &z,
+                              cudaStream_t s);
+void launch_records_and_reset(const DevTables &T, const DevMesh &M, double2 *out, int cells, const StepCounters &z,
                               cudaStream_t s);
 // The end of a step, done by the last block of the sort's scatter (n null:
 // none): *particle_steps += *n; *n = *sorted_total; *next_uid += *appended.

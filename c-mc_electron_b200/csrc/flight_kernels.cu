@@ -4,8 +4,10 @@
 //
 // Step structure (replaces MeshQuantities::update_particle +
 // local_migrate, src/mcmodel.cpp:1460-1505 and :1615-1638):
-//   1. flight_kernel: every particle flies dt on its own random stream;
-//      caught particles are marked dead in their meta word.
+//   1. drift_kernel: the particles that have no event in the step fly it
+//      at once and the others are listed; flight_kernel: the listed ones
+//      fly dt on their own random streams; caught particles are marked dead
+//      in their meta word.
 //   2. child_flight_kernel, repeated: copies made by GENERATE / GENREF fly
 //      the rest of the step (they may make copies of their own).
 //   3. append_children_kernel: surviving copies join the store with uids
@@ -43,21 +45,24 @@ constexpr uint32_t kMetaUnfinished = 1u << 17;
 
 template <typename R>
 __device__ void load_sym(SymSmemT<R> &S, const DevTables &T) {
-  for (int i = threadIdx.x; i < 48 * 6; i += blockDim.x) S.symi[i] = T.symi[i];
+  for (int i = threadIdx.x; i < 48; i += blockDim.x) S.sym[i] = T.sym_packed[i];
   for (int i = threadIdx.x; i < 5 * 48; i += blockDim.x) S.newisym[i] = T.newisym[i];
   for (int i = threadIdx.x; i < 3 * 5 * 48; i += blockDim.x) S.bz[i] = (R)T.bz[i];
   for (int i = threadIdx.x; i < 3 * 48; i += blockDim.x) S.refl[i] = T.reflect_isym[i];
   __syncthreads();
 }
 
-// Loading and storing the flown particles of the main store (StoreIO) and
-// of a child generation (ChildIO).
+// Loading and storing the flown particles of the main store (StoreIO: the
+// particles drift_kernel listed) and of a child generation (ChildIO).  load
+// takes the q-th particle to fly and returns where store puts it (-1: none).
 template <typename R>
 struct StoreIO {
   DevParticlesT<R> P;
+  const uint32_t *list;  // the particles to fly
   double dt;
   uint32_t step;  // the particles' step number (their random streams)
-  __device__ bool load(int p, FlyerT<R> &f) const {
+  // particle p of the store; false: not to be flown
+  __device__ __forceinline__ bool read(int p, FlyerT<R> &f) const {
     const uint32_t meta = P.meta[p];
     if (meta & kMetaDead) return false;
     f.step_ = step;
@@ -75,6 +80,10 @@ struct StoreIO {
     f.left_time = dt;
     return true;
   }
+  __device__ int load(int q, FlyerT<R> &f) const {
+    const int p = (int)list[q];
+    return read(p, f) ? p : -1;
+  }
   __device__ void store(int p, const FlyerT<R> &f, int r) const {
     P.x[p] = f.x; P.y[p] = f.y; P.z[p] = f.z;
     P.kx[p] = f.kx; P.ky[p] = f.ky; P.kz[p] = f.kz;
@@ -91,7 +100,7 @@ template <typename R>
 struct ChildIO {
   DevChildrenT<R> C;
   uint32_t step;
-  __device__ bool load(int p, FlyerT<R> &f) const {
+  __device__ int load(int p, FlyerT<R> &f) const {
     f.step_ = step;
     f.x = C.x[p]; f.y = C.y[p]; f.z = C.z[p];
     f.kx = C.kx[p]; f.ky = C.ky[p]; f.kz = C.kz[p];
@@ -105,7 +114,7 @@ struct ChildIO {
     f.start_stream(C.parent_uid[p], C.sub[p]);
     f.nchild = 0;
     f.left_time = C.left_time[p];
-    return true;
+    return p;
   }
   __device__ void store(int p, const FlyerT<R> &f, int r) const {
     C.x[p] = f.x; C.y[p] = f.y; C.z[p] = f.z;
@@ -120,51 +129,97 @@ struct ChildIO {
   }
 };
 
-// Persistent flight: each lane holds one particle at a time and advances it
-// one event per pass; a lane whose particle has finished its step stores it
-// and takes the next particle index from `ticket` (one atomic per warp for
-// all lanes that need work).  Lanes therefore stay busy while the warp's
-// other particles finish, instead of idling until the slowest one is done.
+// Persistent flight: each lane holds one particle at a time; a lane whose
+// particle has finished its step stores it and takes the next index of the
+// warp's chunk of consecutive particles, and the warp takes its next chunk
+// from `ticket` (fetched one chunk ahead, so no lane waits for the atomic).
 // Every particle's draws come from its own stream, so the result does not
 // depend on which lane flies it or when.
+//
+// A pass of the loop advances every lane to its next event and then runs the
+// work that events left: an impurity event's new k and k-space searches by
+// the lanes that have some, final-state draws by the whole warp.  (Keeping
+// the lanes' work back until 8, 16 or 24 lanes have some was measured slower
+// on bulk boxes and no faster on FinFETs: it takes the lanes out of the next
+// advances, and a warp that alternates between two long pieces of code
+// misses the instruction cache more.)
+//
+// With fewer particles than the grid has lanes, a warp uses only as many
+// lanes as it takes to give every particle one: a warp's passes are the
+// union of its lanes' work, so fewer lanes a warp finish sooner.
 //
 // kLaneEvents (launches of one simulation): the event count of each finished
 // particle is summed in the lane and the warp adds its total to the
 // simulation's counter once, at the end, instead of one atomic on that one
 // address per particle.  A batched launch counts per particle (its particles
 // belong to different simulations).
+#ifndef MCB200_FLIGHT_CHUNK
+#define MCB200_FLIGHT_CHUNK 64
+#endif
 template <typename R, bool kLaneEvents, class IO>
 __device__ __forceinline__ void fly_interleaved(const FlightCtxT<R> &F, const SymSmemT<R> &S, const IO &io, int n,
                                                 unsigned int *ticket) {
-  FlyerT<R> f(F, S);
+  static_assert(kFlightThreads == FlyerT<R>::kRingStride, "one ring column a thread");
+  __shared__ R ring[FlyerT<R>::kRing * FlyerT<R>::kRingStride];
+  FlyerT<R> f(F, S, ring + threadIdx.x);
+  f.n_ph = f.n_imp = 0;
   const unsigned lane = threadIdx.x & 31u;
+  const unsigned warps = gridDim.x * (blockDim.x >> 5), count = (unsigned)n;
+  const unsigned lanes = min(32u, (count + warps - 1) / warps);
+  // a warp's chunk: what its lanes hold when there are few particles, else a
+  // quarter of its share, 8 to MCB200_FLIGHT_CHUNK
+  const unsigned chunk = lanes < 32u ? lanes : max(8u, min((unsigned)MCB200_FLIGHT_CHUNK, count / (4u * warps)));
+  const bool working = lane < lanes;
+  auto take = [&]() {
+    unsigned base = 0;
+    if (lane == 0) base = atomicAdd(ticket, chunk);
+    return base;  // lane 0's value counts
+  };
+  unsigned ahead = take(), next = 0, end = 0;
   int p = -1;
+  int state = FlyerT<R>::kGoOn;
   bool exhausted = false;
-  uint32_t events = 0;  // < 2^31 + kMaxEvents: flushed whenever it passes 2^31
+  uint32_t events = 0;  // < 2^31 + kMaxEvents: flushed whenever it passes 2^31 (it bounds n_ph and n_imp)
+  auto flush = [&]() {
+    atomicAdd(&F.Y.counters[kCntEvents], (unsigned long long)events);
+    atomicAdd(&F.Y.counters[kCntPhonon], (unsigned long long)f.n_ph);
+    atomicAdd(&F.Y.counters[kCntImpurity], (unsigned long long)f.n_imp);
+    events = f.n_ph = f.n_imp = 0;
+  };
   auto done = [&]() {
     const int r = f.template finish<!kLaneEvents>();
     if constexpr (kLaneEvents) {
       events += (uint32_t)f.loop;
-      if (events >= 0x80000000u) {
-        atomicAdd(&F.Y.counters[kCntEvents], (unsigned long long)events);
-        events = 0;
-      }
+      if (events >= 0x80000000u) flush();
     }
     return r;
   };
   for (;;) {
     if (!exhausted) {
-      const unsigned need = __ballot_sync(0xffffffffu, p < 0);
+      const bool wants = p < 0 && working;
+      unsigned need = __ballot_sync(0xffffffffu, wants);
       if (need) {
-        const int leader = __ffs(need) - 1;
-        unsigned base = 0;
-        if ((int)lane == leader) base = atomicAdd(ticket, (unsigned)__popc(need));
-        base = __shfl_sync(0xffffffffu, base, leader);
-        if ((unsigned long long)base + __popc(need) >= (unsigned long long)n) exhausted = true;
-        if (p < 0) {
-          const unsigned q = base + __popc(need & ((1u << lane) - 1u));
-          if (q < (unsigned)n && io.load((int)q, f)) {
-            p = (int)q;
+        unsigned mine = __popc(need & ((1u << lane) - 1u)), left = __popc(need);  // rank among those that still need one
+        int q = -1;
+        while (left) {
+          if (next >= end) {
+            next = __shfl_sync(0xffffffffu, ahead, 0);
+            end = min(next + chunk, count);
+            if (next >= count) {
+              exhausted = true;
+              break;
+            }
+            ahead = take();
+          }
+          const unsigned give = min(left, end - next);
+          if (wants && mine < give) q = (int)(next + mine);
+          mine -= give;  // wraps past zero once served: no second turn
+          left -= give;
+          next += give;
+        }
+        if (q >= 0) {
+          p = io.load(q, f);
+          if (p >= 0) {
             f.begin();
             if (!(f.left_time > 0)) {
               io.store(p, f, done());
@@ -174,33 +229,128 @@ __device__ __forceinline__ void fly_interleaved(const FlightCtxT<R> &F, const Sy
         }
       }
     }
-    if (!__any_sync(0xffffffffu, p >= 0)) {
+    const unsigned held = __ballot_sync(0xffffffffu, p >= 0);
+    if (!held) {
       if (exhausted) break;
       continue;
     }
-    if (p >= 0 && f.iterate()) {
+    if (p >= 0) state = f.advance();
+    const unsigned draws = __ballot_sync(0xffffffffu, p >= 0 && state == FlyerT<R>::kDraw);
+    if (draws) f.final_states(draws);
+    if (p >= 0 && state >= FlyerT<R>::kPending) {
+      if (state == FlyerT<R>::kPending) f.run_pending();
+      state = f.settle() ? FlyerT<R>::kStepOver : FlyerT<R>::kGoOn;
+    }
+    if (p >= 0 && state == FlyerT<R>::kStepOver) {
       io.store(p, f, done());
       p = -1;
     }
   }
   if constexpr (kLaneEvents) {
-    unsigned long long sum = events;
+    const uint32_t mine[3] = {events, f.n_ph, f.n_imp};
+    const int to[3] = {kCntEvents, kCntPhonon, kCntImpurity};
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, off);
-    if (lane == 0 && sum) atomicAdd(&F.Y.counters[kCntEvents], sum);
+    for (int c = 0; c < 3; ++c) {
+      unsigned long long sum = mine[c];
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, off);
+      if (lane == 0 && sum) atomicAdd(&F.Y.counters[to[c]], sum);
+    }
   }
+}
+
+// The drift pass: every particle that certainly has no event in the step
+// (FlyerT::no_event) flies it here, on the fields of its cell with the
+// velocity of its tetrahedron, and the others are listed for the flight.
+// About half of the particles of a bulk step and four fifths of a FinFET's
+// have no event; in the flight's loop each costs a whole pass of the general
+// code, here a fifth of its instructions, in a kernel small enough for the
+// instruction cache and without its divergence.  Measured (drift + flight
+// against the flight of every particle): FinFET FP32 25 + 110 against 165 us
+// per launch of 530k particles, bulk FP32 80 + 707 against 823 us per launch
+// of 2M; the drift pass itself is bound by the latency of its loads (its
+// 112 bytes a particle would take 35 us from HBM in the bulk case).
+//
+// n: the store's count; *listed (zeroed by the step reset) counts the list.
+// A block takes 256 consecutive particles at a time and places its
+// unfinished ones with one atomic.
+template <typename R, class IO>
+__device__ __forceinline__ int drift_block(const FlightCtxT<R> &F, FlyerT<R> &f, const IO &io, int p, bool in,
+                                           bool &unfinished) {
+  unfinished = false;
+  if (!in || !io.read(p, f)) return 0;
+  f.load_cell_fields();
+  f.iband = f.tf(f.itet).band;
+  f.GetV();
+  if (f.left_time > kMyZero && f.no_event() && f.drift()) {
+    const DevParticlesT<R> &P = io.P;
+    P.x[p] = f.x; P.y[p] = f.y; P.z[p] = f.z;
+    P.kx[p] = f.kx; P.ky[p] = f.ky; P.kz[p] = f.kz;
+    P.energy[p] = f.energy;
+    return 1;
+  }
+  unfinished = true;
+  return 0;
+}
+
+// Places the block's marked threads: each gets a consecutive index from *counter.
+__device__ __forceinline__ unsigned place_in_list(bool mine, unsigned int *counter) {
+  __shared__ unsigned warp_base[kFlightThreads / 32 + 1];
+  const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const unsigned votes = __ballot_sync(0xffffffffu, mine);
+  if (lane == 0) warp_base[warp] = (unsigned)__popc(votes);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned run = 0;
+#pragma unroll
+    for (int w = 0; w < kFlightThreads / 32; ++w) {
+      const unsigned c = warp_base[w];
+      warp_base[w] = run;
+      run += c;
+    }
+    warp_base[kFlightThreads / 32] = run ? atomicAdd(counter, run) : 0u;
+  }
+  __syncthreads();
+  const unsigned at = warp_base[kFlightThreads / 32] + warp_base[warp] + (unsigned)__popc(votes & ((1u << lane) - 1u));
+  __syncthreads();  // the counts are reused by the next call
+  return at;
+}
+
+template <typename R>
+__global__ void __launch_bounds__(kFlightThreads) drift_kernel(const __grid_constant__ FlightCtxT<R> F,
+                                                               const __grid_constant__ DevParticlesT<R> P, DevCount n,
+                                                               uint32_t *list, unsigned int *listed) {
+  __shared__ SymSmemT<R> S;  // its operations only
+  for (int i = threadIdx.x; i < 48; i += blockDim.x) S.sym[i] = F.T.sym_packed[i];
+  __syncthreads();
+  pdl_wait();
+  const int count = n.get();
+  const uint32_t step = F.step_dev ? *F.step_dev : F.step;
+  const StoreIO<R> io{P, nullptr, F.dt, step};
+  unsigned int done = 0;
+  for (int base = blockIdx.x * kFlightThreads; base < count; base += gridDim.x * kFlightThreads) {
+    const int p = base + (int)threadIdx.x;
+    FlyerT<R> f(F, S, nullptr);
+    bool unfinished;
+    done += drift_block(F, f, io, p, p < count, unfinished);
+    const unsigned at = place_in_list(unfinished, listed);
+    if (unfinished) list[at] = (uint32_t)p;
+  }
+  done = __reduce_add_sync(0xffffffffu, done);
+  if ((threadIdx.x & 31u) == 0 && done) atomicAdd(&F.Y.counters[kCntEvents], (unsigned long long)done);
 }
 
 template <typename R>
 __global__ void __launch_bounds__(kFlightThreads, kFlightBlocks<R>) flight_kernel(FlightCtxT<R> F, DevParticlesT<R> P,
-                                                                       DevCount n, unsigned int *ticket) {
+                                                                       const uint32_t *list, DevCount n,
+                                                                       unsigned int *ticket) {
   __shared__ SymSmemT<R> S;
   load_sym(S, F.T);  // the band tables: nothing the kernel ahead writes
   pdl_wait();
   const int count = n.get();
   if (count == 0) return;
   const uint32_t step = F.step_dev ? *F.step_dev : F.step;
-  fly_interleaved<R, true>(F, S, StoreIO<R>{P, F.dt, step}, count, ticket);
+  fly_interleaved<R, true>(F, S, StoreIO<R>{P, list, F.dt, step}, count, ticket);
 }
 
 // Copies made during the previous pass (buffer `in`) fly the rest of their
@@ -240,19 +390,18 @@ struct BatchIO {
     }
     return lo;
   }
-  __device__ bool load(int q, FlyerT<R> &f) const {
+  __device__ int load(int q, FlyerT<R> &f) const {
     const int k = find(q);
     const BatchInstT<R> &b = I[k];
     f.I = &b;
     const int p = q - prefix[k];
     if constexpr (kChild) return ChildIO<R>{b.in, b.step}.load(p, f);
-    else return StoreIO<R>{b.P, b.dt, b.step}.load(p, f);
+    else return StoreIO<R>{b.P, b.list, b.dt, b.step}.load(p, f);
   }
-  __device__ void store(int q, const FlyerT<R> &f, int r) const {
+  __device__ void store(int p, const FlyerT<R> &f, int r) const {
     const BatchInstT<R> *b = static_cast<const BatchInstT<R> *>(f.I);
-    const int p = q - prefix[b - I];
     if constexpr (kChild) ChildIO<R>{b->in, b->step}.store(p, f, r);
-    else StoreIO<R>{b->P, b->dt, b->step}.store(p, f, r);
+    else StoreIO<R>{b->P, b->list, b->dt, b->step}.store(p, f, r);
   }
 };
 
@@ -302,7 +451,7 @@ __global__ void __launch_bounds__(kFlightThreads, kFlightBlocks<R>) batch_flight
     for (int k = 0; k < ninst; ++k) {
       prefix[k] = run;
       if ((members >> k) & 1ull)
-        run += kChild ? min((int)*I[k].in.count, I[k].in.capacity) : min((int)*I[k].n, I[k].capacity);
+        run += kChild ? min((int)*I[k].in.count, I[k].in.capacity) : (int)*I[k].listed;
     }
     prefix[ninst] = run;
   }
@@ -310,6 +459,47 @@ __global__ void __launch_bounds__(kFlightThreads, kFlightBlocks<R>) batch_flight
   const int total = prefix[ninst];
   if (total == 0) return;
   fly_interleaved<R, false>(F, S, BatchIO<R, kChild>{I, prefix, ninst}, total, ticket);
+}
+
+// The drift pass of many simulations in one launch: the blocks take 256
+// particles of one simulation at a time.
+template <typename R>
+__global__ void __launch_bounds__(kFlightThreads) batch_drift_kernel(const __grid_constant__ FlightCtxT<R> F,
+                                                                     const BatchInstT<R> *inst, int ninst,
+                                                                     uint64_t members) {
+  __shared__ SymSmemT<R> S;
+  __shared__ int first[kMaxBatch + 1];  // the tiles before each simulation's
+  for (int i = threadIdx.x; i < 48; i += blockDim.x) S.sym[i] = F.T.sym_packed[i];
+  for (int k = threadIdx.x; k < ninst; k += blockDim.x)
+    first[k] = (members >> k) & 1ull
+                   ? (min((int)*inst[k].n, inst[k].capacity) + kFlightThreads - 1) / kFlightThreads : 0;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int run = 0;
+    for (int k = 0; k < ninst; ++k) {
+      const int c = first[k];
+      first[k] = run;
+      run += c;
+    }
+    first[ninst] = run;
+  }
+  __syncthreads();
+  const int tiles = first[ninst];
+  for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+    int k = 0;  // uniform over the block
+    while (first[k + 1] <= t) ++k;
+    const BatchInstT<R> &b = inst[k];
+    const int count = min((int)*b.n, b.capacity);
+    const int p = (t - first[k]) * kFlightThreads + (int)threadIdx.x;
+    FlyerT<R> f(F, S, nullptr);
+    f.I = &b;
+    bool unfinished;
+    const StoreIO<R> io{b.P, nullptr, b.dt, b.step};
+    const unsigned done = __reduce_add_sync(0xffffffffu, drift_block(F, f, io, p, p < count, unfinished));
+    if ((threadIdx.x & 31u) == 0 && done) atomicAdd(&b.Y.counters[kCntEvents], (unsigned long long)done);
+    const unsigned at = place_in_list(unfinished, b.listed);
+    if (unfinished) b.list[at] = (uint32_t)p;
+  }
 }
 
 // Step numbers of a batch: steps[k] += 1, and the step field of simulation
@@ -339,7 +529,28 @@ __device__ __forceinline__ void reset_step_counters(const StepCounters &z, int t
     z.tickets[t] = 0u;
     *z.count[t] = 0u;
   }
-  if (t == 0) *z.appended = 0u;
+  if (t == 0) {
+    *z.appended = 0u;
+    *z.listed = 0u;
+  }
+}
+// FP64 flight's records (DevMesh::cell64): the factors of the reference's
+// expressions that hold no particle value, each rounded as there.
+__global__ void cell_records64_kernel(DevTables T, DevMesh M, double2 *out, int cells, StepCounters z) {
+  pdl_wait();
+  if (blockIdx.x == 0) reset_step_counters(z, threadIdx.x);
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= cells) return;
+  const double rho = M.rho[c], da = M.da[c];
+  // a surface-impurity cell: the reference's formula is commented out there
+  // and leaves the rate unset; the engine treats it as zero
+  const bool on = (da * T.conc0 >= 1e22) && !(M.surface_scatter && M.surface_impurity && M.in_surf[c]);
+  const double eebeta = T.frickel * 4 * kPiD * rho / (2.0 * T.meld * T.eps_si);
+  const double fr = T.frickel * rho;
+  out[3 * (size_t)c + 0] = make_double2(on ? da * T.meld : 0.0, eebeta * T.meld);
+  out[3 * (size_t)c + 1] =
+      make_double2(kPiD * (fr * fr), T.frickel * 4 * kPiD * rho / (8.0 * T.melt * T.eps_si));
+  out[3 * (size_t)c + 2] = make_double2(T.frickel * 4 * kPiD * rho / T.eps_si, 0.0);
 }
 __global__ void cell_records32_kernel(DevTables T, DevMesh M, float4 *out, int cells, StepCounters z) {
   pdl_wait();
@@ -654,16 +865,18 @@ __global__ void __launch_bounds__(256) seed_kernel(FlightCtx F, DevParticlesT<R>
                                                    const int *cell_of, const double *charge, int type,
                                                    uint32_t uid0) {
   __shared__ SymSmem S;
+  __shared__ double ring[Flyer::kRing * Flyer::kRingStride];
   load_sym(S, F.T);
   const DevTables &T = F.T;
   const double tmp_const = 1 - exp(-T.emax);
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
-    Flyer f(F, S);
+    Flyer f(F, S, ring + threadIdx.x);
     const int c = cell_of[q];
     const int kc = c % F.M.nz, ic = (c / F.M.nz) % F.M.nx, jc = c / (F.M.nz * F.M.nx);
     f.ic = ic; f.jc = jc; f.kc = kc;
     f.type = type;
     f.start_stream(uid0 + q, 0);
+    f.stock(3);
     double lamda = f.Random();
     f.x = lamda * F.M.lx[ic] + (1 - lamda) * F.M.lx[ic + 1];
     lamda = f.Random();
@@ -674,6 +887,7 @@ __global__ void __launch_bounds__(256) seed_kernel(FlightCtx F, DevParticlesT<R>
     f.kx = f.ky = f.kz = 0;
     bool ok = false;
     for (int attempt = 0; attempt < 100000 && !ok; ++attempt) {
+      f.stock(3);
       f.energy = -log(1 - f.Random() * tmp_const);
       // CALDOSSUM (src/Band.cpp:2267-2295) and CALDOS (:2234-2264)
       const TabPos p = tab_pos(T, f.energy);
@@ -714,7 +928,7 @@ void launch_seed(const FlightCtx &F, const DevParticlesT<R> &P, int offset, int 
   if (n > 0) seed_kernel<R><<<grid, 256, 0, s>>>(F, P, offset, n, cell_of, charge, type, uid0);
 }
 // Blocks of the persistent flight kernels: enough to fill every SM at the
-// kernel's occupancy, fewer when there are fewer particles than threads.
+// kernel's occupancy, fewer when there are fewer particles than warps.
 // Launch settings are looked up once per device (the current device at the
 // launch) and kept: a process may drive several GPUs.
 constexpr int kMaxDevices = 64;
@@ -732,21 +946,43 @@ int flight_grid(int n, int block, int sm_count) {
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, flight_kernel<R>, block, 0) != cudaSuccess || b < 1) b = 1;
     per_sm = b;
   }
-  const long long want = ((long long)n + block - 1) / block;
+  const long long want = ((long long)n + block / 32 - 1) / (block / 32);
   return (int)std::max<long long>(1, std::min<long long>(want, (long long)per_sm * sm_count));
 }
 
 template <typename R>
-void launch_flight(const FlightCtxT<R> &F, const DevParticlesT<R> &P, DevCount n, unsigned int *ticket, int sm_count,
-                   cudaStream_t s) {
-  launch_pdl(flight_kernel<R>, flight_grid<R>(n.max, kFlightThreads, sm_count), kFlightThreads, 0, s, F, P, n, ticket);
+int drift_grid(long long tiles, int sm_count) {
+  static int per_sm_of[kMaxDevices] = {};
+  int &per_sm = per_sm_of[current_device()];
+  if (per_sm == 0) {
+    int b = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, drift_kernel<R>, kFlightThreads, 0) != cudaSuccess || b < 1)
+      b = 1;
+    per_sm = b;
+  }
+  return (int)std::max<long long>(1, std::min<long long>(tiles, (long long)per_sm * sm_count));
+}
+template <typename R>
+void launch_flight(const FlightCtxT<R> &F, const DevParticlesT<R> &P, DevCount n, uint32_t *list,
+                   unsigned int *listed, unsigned int *ticket, int sm_count, cudaStream_t s) {
+  launch_pdl(drift_kernel<R>, drift_grid<R>(((long long)n.max + kFlightThreads - 1) / kFlightThreads, sm_count),
+             kFlightThreads, 0, s, F, P, n, list, listed);
+  launch_pdl(flight_kernel<R>, flight_grid<R>(n.max, kFlightThreads, sm_count), kFlightThreads, 0, s, F, P,
+             (const uint32_t *)list, DevCount{listed, nullptr, n.max}, ticket);
+}
+template <typename R>
+int launch_batch_drift(const FlightCtxT<R> &F, const BatchInstT<R> *inst, int ninst, uint64_t members, int sm_count,
+                       cudaStream_t s) {
+  if (ninst < 1 || ninst > kMaxBatch) return 1;
+  batch_drift_kernel<R><<<drift_grid<R>(1 << 30, sm_count), kFlightThreads, 0, s>>>(F, inst, ninst, members);
+  return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
 template <typename R>
 void launch_child_flight(const FlightCtxT<R> &F, const DevChildrenT<R> &in, int n_hint, unsigned int *ticket,
                          int sm_count, cudaStream_t s) {
   // One block per SM: a step's copies are few (their lanes refill from the
   // same counter however many there are), and most generations are empty.
-  const int n = (int)std::min<long long>(n_hint, (long long)sm_count * kFlightThreads);
+  const int n = (int)std::min<long long>(n_hint, (long long)sm_count * (kFlightThreads / 32));
   launch_pdl(child_flight_kernel<R>, flight_grid<R>(n, kFlightThreads, sm_count), kFlightThreads, 0, s, F, in, ticket);
 }
 template <typename R>
@@ -780,14 +1016,16 @@ void launch_records_and_reset(const DevTables &T, const DevMesh &M, float4 *out,
                               cudaStream_t s) {
   launch_pdl(cell_records32_kernel, std::max((cells + 255) / 256, 1), 256, 0, s, T, M, out, cells, z);
 }
+void launch_records_and_reset(const DevTables &T, const DevMesh &M, double2 *out, int cells, const StepCounters &z,
+                              cudaStream_t s) {
+  launch_pdl(cell_records64_kernel, std::max((cells + 255) / 256, 1), 256, 0, s, T, M, out, cells, z);
+}
 template <typename R>
 void launch_append_children(const ChildSetT<R> &set, unsigned int *next_uid, const DevParticlesT<R> &dst,
                             const unsigned int *n, int capacity, unsigned int *appended, unsigned int *overflow,
                             int grid, cudaStream_t s) {
   launch_pdl(append_children_kernel<R>, grid, 256, 0, s, set, next_uid, dst, n, capacity, appended, overflow);
 }
-__global__ void step_reset_kernel(StepCounters z) { reset_step_counters(z, threadIdx.x); }
-void launch_step_reset(const StepCounters &z, cudaStream_t s) { step_reset_kernel<<<1, 32, 0, s>>>(z); }
 void launch_exclusive_scan(const unsigned int *in, unsigned int *out, unsigned int *tile_sums, unsigned int *total,
                            int n, cudaStream_t s) {
   const int tiles = (n + 1023) / 1024;
@@ -823,8 +1061,10 @@ void launch_cell_sort(const DevParticlesT<R> &src, DevCount n, const DevParticle
 #define MCB200_INSTANTIATE(R)                                                                                   \
   template void launch_seed<R>(const FlightCtx &, const DevParticlesT<R> &, int, int, const int *,            \
                                const double *, int, uint32_t, int, cudaStream_t);                             \
-  template void launch_flight<R>(const FlightCtxT<R> &, const DevParticlesT<R> &, DevCount, unsigned int *, int, \
-                                 cudaStream_t);                                                                 \
+  template void launch_flight<R>(const FlightCtxT<R> &, const DevParticlesT<R> &, DevCount, uint32_t *,         \
+                                 unsigned int *, unsigned int *, int, cudaStream_t);                            \
+  template int launch_batch_drift<R>(const FlightCtxT<R> &, const BatchInstT<R> *, int, uint64_t, int,          \
+                                     cudaStream_t);                                                             \
   template void launch_child_flight<R>(const FlightCtxT<R> &, const DevChildrenT<R> &, int, unsigned int *, int, \
                                        cudaStream_t);                                                           \
   template void launch_append_children<R>(const ChildSetT<R> &, unsigned int *, const DevParticlesT<R> &,     \

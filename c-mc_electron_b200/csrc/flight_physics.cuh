@@ -41,6 +41,7 @@ namespace mcb200 {
 constexpr double kMyZero = 1e-13;          // MY_ZERO, include/defs.h
 constexpr double kPiD = 3.141592653589793238462643e0;
 constexpr int kMaxEvents = 1000000;
+constexpr int kMaxStateTries = 10000;
 // FP32 flight: consecutive zero-length events after which a particle is
 // taken as stuck (counted in kCntZeroTime and caught).
 constexpr int kMaxZeroTimeEvents = 64;
@@ -84,8 +85,38 @@ __device__ __forceinline__ double m_log(double v) { return log(v); }
 __device__ __forceinline__ float m_log(float v) { return logf(v); }
 __device__ __forceinline__ double m_floor(double v) { return floor(v); }
 __device__ __forceinline__ float m_floor(float v) { return floorf(v); }
-__device__ __forceinline__ void m_sincos(double v, double *s, double *c) { *s = sin(v); *c = cos(v); }
+__device__ __forceinline__ void m_sincos(double v, double *s, double *c) { sincos(v, s, c); }
 __device__ __forceinline__ void m_sincos(float v, float *s, float *c) { sincosf(v, s, c); }
+
+// v times +-1: the sign flipped where the top bit of `neg` is set.
+__device__ __forceinline__ float m_flip(float v, uint32_t neg) {
+  return __uint_as_float(__float_as_uint(v) ^ (neg & 0x80000000u));
+}
+__device__ __forceinline__ double m_flip(double v, uint32_t neg) {
+  return __hiloint2double(__double2hiint(v) ^ (int)(neg & 0x80000000u), __double2loint(v));
+}
+template <typename R>
+__device__ __forceinline__ R m_pick3(uint32_t which, R a, R b, R c) {
+  which &= 3u;
+  return which == 0u ? a : (which == 1u ? b : c);
+}
+
+// mcb200_philox4x32_10 (include/mcb200_rng.h) unrolled, for the stream's one
+// hot place.
+__device__ __forceinline__ void philox_rounds(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3, uint32_t k0,
+                                              uint32_t k1, uint32_t *w) {
+#pragma unroll
+  for (int round = 0; round < 10; ++round) {
+    const uint64_t p0 = (uint64_t)MCB200_PHILOX_M0 * c0, p1 = (uint64_t)MCB200_PHILOX_M1 * c2;
+    c0 = (uint32_t)(p1 >> 32) ^ c1 ^ k0;
+    c1 = (uint32_t)p1;
+    c2 = (uint32_t)(p0 >> 32) ^ c3 ^ k1;
+    c3 = (uint32_t)p0;
+    k0 += MCB200_PHILOX_W0;
+    k1 += MCB200_PHILOX_W1;
+  }
+  w[0] = c0; w[1] = c1; w[2] = c2; w[3] = c3;
+}
 
 // Table views per precision (the FP64 tables or their FP32 copies).
 template <typename R> struct Tab;
@@ -93,7 +124,7 @@ template <> struct Tab<double> {
   static __device__ __forceinline__ const TetFlightT<double> *tf(const DevTables &T) { return T.tf; }
   static __device__ __forceinline__ const TetShapeT<double> *ts(const DevTables &T) { return T.ts; }
   static __device__ __forceinline__ const double4 *knode(const DevTables &T) { return T.knode; }
-  static __device__ __forceinline__ const double *gamtet(const DevTables &T) { return T.gamtet; }
+  static __device__ __forceinline__ const FlightConstT<double> &k(const DevTables &T) { return T.k64; }
   static __device__ __forceinline__ const double *energy(const DevTables &T) { return T.energy; }
   static __device__ __forceinline__ const double *sumscatt(const DevTables &T) { return T.sumscatt; }
   static __device__ __forceinline__ const double *scatte(const DevTables &T) { return T.scatte; }
@@ -108,7 +139,7 @@ template <> struct Tab<float> {
   static __device__ __forceinline__ const TetFlightT<float> *tf(const DevTables &T) { return T.f32.tf; }
   static __device__ __forceinline__ const TetShapeT<float> *ts(const DevTables &T) { return T.f32.ts; }
   static __device__ __forceinline__ const float4 *knode(const DevTables &T) { return T.f32.knode; }
-  static __device__ __forceinline__ const float *gamtet(const DevTables &T) { return T.f32.gamtet; }
+  static __device__ __forceinline__ const FlightConstT<float> &k(const DevTables &T) { return T.k32; }
   static __device__ __forceinline__ const float *energy(const DevTables &T) { return T.f32.energy; }
   static __device__ __forceinline__ const float *sumscatt(const DevTables &T) { return T.f32.sumscatt; }
   static __device__ __forceinline__ const float *scatte(const DevTables &T) { return T.f32.scatte; }
@@ -123,7 +154,7 @@ template <> struct Tab<float> {
 // Symmetry tables staged in shared memory (one copy per block).
 template <typename R>
 struct SymSmemT {
-  int symi[48 * 6];   // matsym[c][s] at s*6+c
+  uint32_t sym[48];   // DevTables::sym_packed
   int newisym[5 * 48];
   R bz[3 * 5 * 48];
   int refl[3 * 48];
@@ -155,6 +186,8 @@ struct BatchInstT : FlightInstT<R> {
   DevParticlesT<R> P;
   DevChildrenT<R> in;
   const unsigned int *n;
+  uint32_t *list;        // the particles the drift pass leaves to the flight, and their count
+  unsigned int *listed;
   int capacity;
   int pad_;
 };
@@ -175,81 +208,79 @@ struct FlyerT {
   const SymSmemT<R> &S;
   const FlightInstT<R> *I;     // the simulation of the current particle (F itself unless batched)
   // random stream (uid, step_, sub; step_ set by the launch's IO from the
-  // simulation's step) and the cached Philox block (index rblk, words rw0..rw3)
-  uint32_t uid, sub, n, step_;
-  uint32_t rblk, rw0, rw1, rw2, rw3;
+  // simulation's step): n draws made, draws [n, stocked) ready in the lane's
+  // ring of kRing entries (shared memory, entry d % kRing of thread t at
+  // [d % kRing * kRingStride + t])
+  uint32_t uid, sub, n, step_, stocked;
+  R *ring;
   // particle registers (MeshQuantities members, include/mcmodel.h:215-233)
   R x, y, z, kx, ky, kz;
   double energy, charge, left_time;
   int ic, jc, kc, itet, isym, type, iband;
   R Ex, Ey, Ez, vx, vy, vz;
-  double Rho, DA;                                // FP64: cell screening and doping densities
-  R imp_a, imp_b, imp_ecut, imp_emax, imp_beta;  // FP32: the cell's Brooks-Herring constants
+  // The cell's Brooks-Herring constants (its record): FP32 the rate is
+  // imp_a sqrt(e) / (1 + imp_b e) below imp_ecut; FP64 imp_a = doping meld (0:
+  // no rate), imp_b = eebeta meld, imp_c = pi (frickel rho)^2
+  R imp_a, imp_b, imp_c, imp_ecut, imp_emax, imp_beta;
   int itetdir, idir;
   bool catch_, self;
   R rough_rate, sphon_rate, surf_gamma, imp_gamma;
   int nchild;
-  // Work left by an event handler for the shared tails of the event loop
-  // (one call site each for the mechanism search, the final-state draw and
-  // the k-point search; see run_pick / run_final_state / run_locate).
-  bool pick_pending;
+  uint32_t n_ph, n_imp;  // real phonon and impurity events since they were last added to the counters
+  int ev;                // the event that ended the last advance()
+  // Work an event left: an impurity event's new k and / or a k-point search
+  // (run_pending, lane by lane), or a final-state draw (final_states, by the
+  // whole warp): for a phonon or surface event whose mechanism is to be
+  // searched with pick_drand or with a draw of its own, or for Diffuse.
+  bool imp_pending;
+  int loc_mode;
+  int draw_kind;
   R pick_drand;
-  int fs_kind, fs_tal;  // pending final-state draw: kind and wedge rule
-  double fs_eeold;      // state before the draw (restored on self-scattering)
-  R fs_kx, fs_ky, fs_kz;
-  int fs_ib, fs_it, fs_is;
-  int loc_mode;         // pending k-point search
-  enum : int { kFsNone = 0, kFsPhonon = 1, kFsIonize = 2, kFsDiffuse = 3 };
   enum : int { kLocNone = 0, kLocBZ = 1, kLocImpurity = 2 };
+  enum : int { kDrawNone = 0, kDrawPick = 1, kDrawPickSurface = 2, kDrawDiffuse = 3 };
 
-  __device__ FlyerT(const FlightCtxT<R> &f, const SymSmemT<R> &s) : F(f), S(s), I(&f), step_(f.step) {}
+  __device__ FlyerT(const FlightCtxT<R> &f, const SymSmemT<R> &s, R *r) : F(f), S(s), I(&f), step_(f.step), ring(r) {}
 
   __device__ __forceinline__ void start_stream(uint32_t u, uint32_t sb) {
     uid = u;
     sub = sb;
     n = 0;
-    rblk = 0xffffffffu;
+    stocked = 0;
   }
 
   // Draw n of the particle's stream (include/mcb200_rng.h).  FP64: the
   // 52-bit uniforms of mcb200_uniform, two per Philox block; FP32: the
-  // 23-bit uniforms of mcb200_uniform_f32, four per block.  A block is
-  // computed once and kept for the draws that follow.
-  __device__ __forceinline__ R Random() {
-    if constexpr (sizeof(R) == 8) {
-      const uint32_t b = n >> 1;
-      double u;
-      if ((n & 1u) && b == rblk) {
-        u = mcb200_bits_to_unit(rw3, rw2);
+  // 23-bit uniforms of mcb200_uniform_f32, four per block.  stock(k) makes
+  // sure of the next k <= kRing / 2 draws, Random takes one of them.  The
+  // draws of an event pass come at several places, where other lanes may or
+  // may not draw; one stock per pass computes the block once for all lanes
+  // that need one, instead of at each place for the lanes that do there.
+  static constexpr uint32_t kRing = 8, kRingStride = 256;
+  static constexpr uint32_t kBlockDraws = sizeof(R) == 4 ? 4 : 2;
+  __device__ __forceinline__ void stock(uint32_t k) {
+#pragma unroll 1
+    while (n + k > stocked) {
+      uint32_t w[4];
+      philox_rounds(stocked / kBlockDraws, uid, step_, sub, (uint32_t)I->seed, (uint32_t)(I->seed >> 32), w);
+      R *e = ring + (stocked & (kRing - 1u)) * kRingStride;
+      if constexpr (sizeof(R) == 8) {
+        e[0] = mcb200_bits_to_unit(w[1], w[0]);
+        e[kRingStride] = mcb200_bits_to_unit(w[3], w[2]);
       } else {
-        const mcb200_philox_block w =
-            mcb200_philox4x32_10(b, uid, step_, sub, (uint32_t)I->seed, (uint32_t)(I->seed >> 32));
-        rblk = b;
-        rw2 = w.w[2];
-        rw3 = w.w[3];
-        u = (n & 1u) ? mcb200_bits_to_unit(w.w[3], w.w[2]) : mcb200_bits_to_unit(w.w[1], w.w[0]);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) e[q * kRingStride] = mcb200_bits_to_unit_f32(w[q]);
       }
-      ++n;
-      return u;
-    } else {
-      const uint32_t b = n >> 2;
-      if (b != rblk) {
-        const mcb200_philox_block w =
-            mcb200_philox4x32_10(b, uid, step_, sub, (uint32_t)I->seed, (uint32_t)(I->seed >> 32));
-        rblk = b;
-        rw0 = w.w[0];
-        rw1 = w.w[1];
-        rw2 = w.w[2];
-        rw3 = w.w[3];
-      }
-      const uint32_t q = n & 3u;
-      const uint32_t w = q == 0 ? rw0 : (q == 1 ? rw1 : (q == 2 ? rw2 : rw3));
-      ++n;
-      return mcb200_bits_to_unit_f32(w);
+      stocked += kBlockDraws;
     }
   }
+  __device__ __forceinline__ R Random() { return ring[(n++ & (kRing - 1u)) * kRingStride]; }
+  // Draws up to n - 1 were made elsewhere (final_states): what the ring
+  // holds from n on is still good.
+  __device__ __forceinline__ void skip_to(uint32_t at) {
+    n = at;
+    if (n > stocked) stocked = n & ~(kBlockDraws - 1u);
+  }
 
-  __device__ __forceinline__ int ms(int c, int s) const { return S.symi[s * 6 + c]; }
   __device__ __forceinline__ int cell_index() const { return (jc * I->M.nx + ic) * I->M.nz + kc; }
   __device__ __forceinline__ int cell_index(int i, int j, int k) const { return (j * I->M.nx + i) * I->M.nz + k; }
   __device__ __forceinline__ const TetFlightT<R> &tf(int it) const { return TB::tf(F.T)[it]; }
@@ -257,18 +288,20 @@ struct FlyerT {
 
   // in_wedge, src/ParticleUtils.cpp:295-305: BZ vector -> irreducible wedge of isym.
   __device__ __forceinline__ void in_wedge(R &xo, R &yo, R &zo, R xi, R yi, R zi) const {
-    const int p0 = ms(0, isym) - 1, p1 = ms(1, isym) - 1;
-    const R a = xi * (R)ms(3, isym), b = yi * (R)ms(4, isym), c = zi * (R)ms(5, isym);
-    xo = p0 == 0 ? a : (p1 == 0 ? b : c);
-    yo = p0 == 1 ? a : (p1 == 1 ? b : c);
-    zo = p0 == 2 ? a : (p1 == 2 ? b : c);
+    const uint32_t w = S.sym[isym];
+    const R a = m_flip(xi, w), b = m_flip(yi, w << 1), c = m_flip(zi, w << 2);
+    xo = m_pick3(w >> 6, a, b, c);
+    yo = m_pick3(w >> 8, a, b, c);
+    zo = m_pick3(w >> 10, a, b, c);
   }
-  // Band::OutWedge, src/Band.cpp:555-570: wedge vector -> BZ.
+  // Band::OutWedge, src/Band.cpp:555-570: wedge vector -> BZ, with operation `w`.
+  static __device__ __forceinline__ void out_wedge(uint32_t w, R &xo, R &yo, R &zo, R xi, R yi, R zi) {
+    xo = m_flip(m_pick3(w, xi, yi, zi), w);
+    yo = m_flip(m_pick3(w >> 2, xi, yi, zi), w << 1);
+    zo = m_flip(m_pick3(w >> 4, xi, yi, zi), w << 2);
+  }
   __device__ __forceinline__ void out_wedge(R &xo, R &yo, R &zo, R xi, R yi, R zi) const {
-    const int p0 = ms(0, isym) - 1, p1 = ms(1, isym) - 1, p2 = ms(2, isym) - 1;
-    xo = (p0 == 0 ? xi : (p0 == 1 ? yi : zi)) * (R)ms(3, isym);
-    yo = (p1 == 0 ? xi : (p1 == 1 ? yi : zi)) * (R)ms(4, isym);
-    zo = (p2 == 0 ? xi : (p2 == 1 ? yi : zi)) * (R)ms(5, isym);
+    out_wedge(S.sym[isym], xo, yo, zo, xi, yi, zi);
   }
   // GetV, src/ParticleUtils.cpp:307-313.
   __device__ __forceinline__ void GetV() {
@@ -303,25 +336,72 @@ struct FlyerT {
     in_wedge(xkl, ykl, zkl, kx, ky, kz);
     in_wedge(xfl, yfl, zfl, Ex, Ey, Ez);
     const TetFlightT<R> &t = tf(itet);
-    R best = 0;
-    itetdir = 0;
+    R num[4], den[4];
 #pragma unroll
     for (int f = 0; f < 4; ++f) {
-      const R nf = t.n[f][0] * xfl + t.n[f][1] * yfl + t.n[f][2] * zfl;
-      R tfp;
-      if (nf < 0) {
-        tfp = (t.n[f][3] - (t.n[f][0] * xkl + t.n[f][1] * ykl + t.n[f][2] * zkl)) / nf;
-        if (tfp < 0) tfp = 0;
-      } else {
-        tfp = Real::kBig;
-      }
-      if (f == 0) best = tfp;
-      else if (tfp < best) {
-        best = tfp;
-        itetdir = f;
-      }
+      den[f] = t.n[f][0] * xfl + t.n[f][1] * yfl + t.n[f][2] * zfl;
+      num[f] = t.n[f][3] - (t.n[f][0] * xkl + t.n[f][1] * ykl + t.n[f][2] * zkl);
     }
-    return best;
+    const unsigned valid = (den[0] < 0 ? 1u : 0u) | (den[1] < 0 ? 2u : 0u) | (den[2] < 0 ? 4u : 0u) |
+                           (den[3] < 0 ? 8u : 0u);
+    itetdir = 0;
+    return least_quotient<4>(num, den, valid, (R)0, itetdir);
+  }
+
+  // The least of the quotients num / den of the `valid` indices, each taken
+  // as at least `low`, and its index (the lowest of equal ones); kBig and
+  // `which` unchanged when none is valid.  FP64 divides only those that a
+  // fast estimate (a few ulp of float) leaves in question, one division's
+  // code in place of N: bulk flight 1446 -> 1326 us per launch of 2M
+  // electrons (in FP32, whose divisions are short, 707 -> 750 us: all are
+  // divided there).
+  template <int N>
+  static __device__ __forceinline__ R least_quotient(const R *num, const R *den, unsigned valid, R low, int &which) {
+    R best = Real::kBig;
+    if constexpr (sizeof(R) == 4) {
+      bool any = false;
+#pragma unroll
+      for (int q = 0; q < N; ++q) {
+        if (!((valid >> q) & 1u)) continue;
+        R v = num[q] / den[q];
+        if (v < low) v = low;
+        if (!any || v < best) {
+          best = v;
+          which = q;
+        }
+        any = true;
+      }
+      return best;
+    } else {
+      float est[N], least = 3.0e38f;
+#pragma unroll
+      for (int q = 0; q < N; ++q) {
+        est[q] = fmaxf(__fdividef((float)num[q], (float)den[q]), (float)low);
+        if ((valid >> q) & 1u) least = fminf(least, est[q]);
+      }
+      const float bar = least + fabsf(least) * 1e-4f + 1e-25f;
+      unsigned open = 0;
+#pragma unroll
+      for (int q = 0; q < N; ++q)
+        if (((valid >> q) & 1u) && !(est[q] > bar)) open |= 1u << q;
+      bool any = false;
+#pragma unroll 1
+      for (; open; open &= open - 1u) {
+        const int q = __ffs(open) - 1;
+        R a = num[0], b = den[0];
+#pragma unroll
+        for (int w = 1; w < N; ++w)
+          if (q == w) { a = num[w]; b = den[w]; }
+        R v = a / b;
+        if (v < low) v = low;
+        if (!any || v < best) {
+          best = v;
+          which = q;
+        }
+        any = true;
+      }
+      return best;
+    }
   }
 
   // CellTime, src/CellHit.cpp:4-93: time to the real-space cell face.  FP32
@@ -329,33 +409,22 @@ struct FlyerT {
   // (width - x) and x.
   __device__ R CellTime() {
     const DevMesh &M = I->M;
-    int idx, idy, idz;
-    R tx, ty, tz;
+    R gap[3];
     if constexpr (Real::kCellRelative) {
-      if (vx > 0) { idx = kDown; tx = (M.dxf[ic] - x) / vx; }
-      else if (vx < 0) { idx = kUp; tx = -x / vx; }
-      else { idx = kUp; tx = Real::kBig; }
-      if (vy > 0) { idy = kRight; ty = (M.dyf[jc] - y) / vy; }
-      else if (vy < 0) { idy = kLeft; ty = -y / vy; }
-      else { idy = kRight; ty = Real::kBig; }
-      if (vz > 0) { idz = kBack; tz = (M.dzf[kc] - z) / vz; }
-      else if (vz < 0) { idz = kFront; tz = -z / vz; }
-      else { idz = kFront; tz = Real::kBig; }
+      gap[0] = vx > 0 ? M.dxf[ic] - x : -x;
+      gap[1] = vy > 0 ? M.dyf[jc] - y : -y;
+      gap[2] = vz > 0 ? M.dzf[kc] - z : -z;
     } else {
-      if (vx > 0) { idx = kDown; tx = (M.lx[ic + 1] - x) / vx; }
-      else if (vx < 0) { idx = kUp; tx = -(x - M.lx[ic]) / vx; }
-      else { idx = kUp; tx = Real::kBig; }
-      if (vy > 0) { idy = kRight; ty = (M.ly[jc + 1] - y) / vy; }
-      else if (vy < 0) { idy = kLeft; ty = -(y - M.ly[jc]) / vy; }
-      else { idy = kRight; ty = Real::kBig; }
-      if (vz > 0) { idz = kBack; tz = (M.lz[kc + 1] - z) / vz; }
-      else if (vz < 0) { idz = kFront; tz = -(z - M.lz[kc]) / vz; }
-      else { idz = kFront; tz = Real::kBig; }
+      gap[0] = vx > 0 ? M.lx[ic + 1] - x : -(x - M.lx[ic]);
+      gap[1] = vy > 0 ? M.ly[jc + 1] - y : -(y - M.ly[jc]);
+      gap[2] = vz > 0 ? M.lz[kc + 1] - z : -(z - M.lz[kc]);
     }
-    idir = idx;
-    R t = tx;
-    if (ty < t) { idir = idy; t = ty; }
-    if (tz < t) { idir = idz; t = tz; }
+    const R v[3] = {vx, vy, vz};
+    const unsigned moving = (vx > 0 || vx < 0 ? 1u : 0u) | (vy > 0 || vy < 0 ? 2u : 0u) | (vz > 0 || vz < 0 ? 4u : 0u);
+    int axis = 0;
+    R t = least_quotient<3>(gap, v, moving, -Real::kBig, axis);
+    // faces come in pairs per axis, the odd one towards larger coordinates
+    idir = 2 * axis + (m_pick3((uint32_t)axis, vx, vy, vz) > 0 ? 1 : 0);
     if constexpr (Real::kCellRelative) {
       if (t < 0) t = 0;  // a position rounded just past the face
     } else {
@@ -366,7 +435,8 @@ struct FlyerT {
 
   // Band::CONFBZ, src/Band.cpp:573-616: fold k back into the first BZ.
   __device__ void CONFBZ(R &a, R &b, R &c) const {
-    const R p = (R)F.T.a0pi;
+    const R p = TB::k(F.T).a0pi;
+#pragma unroll 1
     for (int guard = 0; guard < 64; ++guard) {
       bool out = m_abs(a) > p || m_abs(b) > p || m_abs(c) > p || m_abs(a) + m_abs(b) + m_abs(c) > (R)1.50 * p;
       if (!out) return;
@@ -383,6 +453,7 @@ struct FlyerT {
   // does not settle within the step cap; the caller then uses the k-grid.
   __device__ int walk_to(int start, R a, R b, R c) const {
     int it = start;
+#pragma unroll 1
     for (int s = 0; s < 64; ++s) {
       if constexpr (MCB200_FLIGHT_EVENT_STATS != 0) count(I->Y, kStatWalkSteps);
       int fmin = -1;
@@ -438,9 +509,9 @@ struct FlyerT {
     int start = same_band ? itet : -1;
     if (iband == F.T.bandof[0]) {  // lowest conduction band: start next to the point
       const int sg = kSeedGridN;
-      const int si = min(max((int)m_floor((a - (R)F.T.grid_lo[0]) * (R)F.T.seed_inv[0]), 0), sg - 1);
-      const int sj = min(max((int)m_floor((b - (R)F.T.grid_lo[1]) * (R)F.T.seed_inv[1]), 0), sg - 1);
-      const int sk = min(max((int)m_floor((c - (R)F.T.grid_lo[2]) * (R)F.T.seed_inv[2]), 0), sg - 1);
+      const int si = min(max((int)m_floor((a - TB::k(F.T).grid_lo[0]) * TB::k(F.T).seed_inv[0]), 0), sg - 1);
+      const int sj = min(max((int)m_floor((b - TB::k(F.T).grid_lo[1]) * TB::k(F.T).seed_inv[1]), 0), sg - 1);
+      const int sk = min(max((int)m_floor((c - TB::k(F.T).grid_lo[2]) * TB::k(F.T).seed_inv[2]), 0), sg - 1);
       const int s0 = F.T.seed_grid[((size_t)si * sg + sj) * sg + sk];
       if (s0 >= 0) start = s0;
     }
@@ -452,14 +523,15 @@ struct FlyerT {
       }
     }
     const int g = F.T.grid_n;
-    int gi = (int)m_floor((a - (R)F.T.grid_lo[0]) * (R)F.T.grid_inv[0]);
-    int gj = (int)m_floor((b - (R)F.T.grid_lo[1]) * (R)F.T.grid_inv[1]);
-    int gk = (int)m_floor((c - (R)F.T.grid_lo[2]) * (R)F.T.grid_inv[2]);
+    int gi = (int)m_floor((a - TB::k(F.T).grid_lo[0]) * TB::k(F.T).grid_inv[0]);
+    int gj = (int)m_floor((b - TB::k(F.T).grid_lo[1]) * TB::k(F.T).grid_inv[1]);
+    int gk = (int)m_floor((c - TB::k(F.T).grid_lo[2]) * TB::k(F.T).grid_inv[2]);
     gi = min(max(gi, 0), g - 1);
     gj = min(max(gj, 0), g - 1);
     gk = min(max(gk, 0), g - 1);
     const int *st = F.T.grid_start + (size_t)iband * (g * g * g + 1);
     const int cell = (gi * g + gj) * g + gk;
+#pragma unroll 1
     for (int q = st[cell]; q < st[cell + 1]; ++q) {
       const int it = F.T.grid_tets[q];
       if (tet_contains(it, a, b, c)) {
@@ -482,6 +554,7 @@ struct FlyerT {
     if (ie < 0) ie = 0;
     if (ie >= kMWLE) ie = kMWLE - 1;
     const int p = F.T.pslist[ie * kMNB + iband], cnt = F.T.nslist[ie * kMNB + iband];
+#pragma unroll 1
     for (int itl = p; itl <= p + cnt - 1; ++itl) {
       const int it = F.T.slist[itl];
       if (iband == tf(it).band && tet_contains(it, a, b, c)) {
@@ -522,66 +595,43 @@ struct FlyerT {
     GetEnergy();
   }
 
-  // TALIND, src/ParticleUtils.cpp:626-748: final valley (and a random wedge
-  // in it).  The reference's talend[] lookups are written as arithmetic on
-  // the drawn index (1..4); an index of 5 (u*4+1 rounding up to 5, possible
-  // only for u within 2^-51 of 1) reads past the reference's table and is
-  // clamped to 4 here.
-  __device__ __forceinline__ int talend_index() { return min((int)(Random() * (R)4.0 + (R)1.0), 4); }
-  __device__ void TALIND(int ityp) {
-    int ital = 1;
-    const R ax = m_abs(kx), ay = m_abs(ky), az = m_abs(kz);
-    if (ax >= ay && ax >= az) {
-      if (kx >= (R)0) {
-        if (ityp == 1) ital = 1;
-        if (ityp == 2) ital = 2;
-        if (ityp == 3) ital = talend_index() + 2;  // {3,4,5,6}
-      }
-      if (kx < (R)0) {
-        if (ityp == 1) ital = 2;
-        if (ityp == 2) ital = 1;
-        if (ityp == 3) ital = talend_index() + 2;
-      }
-    }
-    if (ay >= az && ay >= ax) {
-      if (ky >= (R)0) {
-        if (ityp == 1) ital = 3;
-        if (ityp == 2) ital = 4;
-        if (ityp == 3) { const int i = talend_index(); ital = i <= 2 ? i : i + 2; }  // {1,2,5,6}
-      }
-      if (ky < (R)0) {
-        if (ityp == 1) ital = 4;
-        if (ityp == 2) ital = 3;
-        if (ityp == 3) { const int i = talend_index(); ital = i <= 2 ? i : i + 2; }
+  // TALIND, src/ParticleUtils.cpp:626-748: the final valley (1..6) of a
+  // transition of type ityp (1: the same valley, 2: the opposite one, 3: one
+  // of the four others) from k.  The reference's talend[] lookups are
+  // written as arithmetic on the drawn index (1..4); an index of 5 (u*4+1
+  // rounding up to 5, possible only for u within 2^-51 of 1) reads past the
+  // reference's table and is clamped to 4 here.
+  template <class Draw>
+  static __device__ __forceinline__ int final_valley(int ityp, R qx, R qy, R qz, Draw &&draw) {
+    const R ax = m_abs(qx), ay = m_abs(qy), az = m_abs(qz);
+    int valley = 1;
+#pragma unroll 1
+    for (int axis = 0; axis < 3; ++axis) {
+      const bool here = axis == 0 ? ax >= ay && ax >= az : (axis == 1 ? ay >= az && ay >= ax : az > ay && az > ax);
+      if (!here) continue;
+      const R q = axis == 0 ? qx : (axis == 1 ? qy : qz);
+      if (ityp == 3) {  // {3,4,5,6}, {1,2,5,6}, {1,2,3,4}
+        const int i = min((int)(draw() * (R)4.0 + (R)1.0), 4);
+        valley = i > 2 * axis ? i + 2 : i;
+      } else {
+        valley = 2 * axis + ((q >= (R)0) == (ityp == 1) ? 1 : 2);
       }
     }
-    if (az > ay && az > ax) {
-      if (kz >= (R)0) {
-        if (ityp == 1) ital = 5;
-        if (ityp == 2) ital = 6;
-        if (ityp == 3) ital = talend_index();  // {1,2,3,4}
-      }
-      if (kz < (R)0) {
-        if (ityp == 1) ital = 6;
-        if (ityp == 2) ital = 5;
-        if (ityp == 3) ital = talend_index();
-      }
-    }
-    isym = (int)(Random() * (R)8.0) + 8 * (ital - 1);
+    return valley;
   }
 
   // Band::CALDOSTETMAX, src/Band.cpp:2298-2320.
   __device__ R CALDOSTETMAX(R eed, int ib) const {
     const R *d = TB::dostetmax(F.T) + (size_t)ib * kNT;
     if (eed <= (R)0) return d[0];
-    if (eed >= (R)F.T.emax) return d[kNT - 1];
-    const int itab = min((int)(eed / (R)F.T.dtable), kNT - 2);  // eed just below emax may round to the last point
+    if (eed >= TB::k(F.T).emax) return d[kNT - 1];
+    const int itab = min((int)(eed / TB::k(F.T).dtable), kNT - 2);  // eed just below emax may round to the last point
     return d[itab] > d[itab + 1] ? d[itab] : d[itab + 1];
   }
 
   // Band::SURF, src/Band.cpp:194-332 (only reached by FASTSURF for
   // tetrahedra whose two lowest nodes are degenerate).
-  __device__ R SURF(R eps, int it) const;
+  static __device__ R SURF(const DevTables &T, R eps, int it);
   // Band::FASTSURF, src/Band.cpp:665-704.
   __device__ R FASTSURF(R eps, int it) const {
     const TetShapeT<R> &s = ts(it);
@@ -590,79 +640,76 @@ struct FlyerT {
       if (eps <= e1) return s.fac[0] * (eps - e0) * (eps - e0);
       if (eps < e2) {
         if (e1 - e0 > (R)1e-10) return s.fac[0] * (eps - e0) * (eps - e0) - s.fac[1] * (eps - e1) * (eps - e1);
-        return SURF(eps, it);
+        return SURF(F.T, eps, it);
       }
       return s.fac[2] * (eps - e3) * (eps - e3);
     }
     return 0;
   }
 
-  // get_state, src/ParticleUtils.cpp:48-120: random final state on the
-  // iso-energy surface of band iband (rejection on the tet's DOS share).
-  __device__ void get_state() {
-    if (energy <= 0.0) {
-      self = true;
-      return;
-    }
-    const R e = (R)energy;
-    const R maxdostet = CALDOSTETMAX(e, iband);
-    int itab = (int)(e * (R)F.T.dlists);
-    bool small_ = itab < kMWLES;
-    if (!small_) {
-      itab = (int)(e * (R)F.T.dlist);
+  // The tetrahedra of band ib whose energy bin holds e: lst[0, count).
+  __device__ __forceinline__ const int *energy_list(R e, int ib, int &count) const {
+    int itab = (int)(e * TB::k(F.T).dlists);
+    const bool fine = itab < kMWLES;
+    if (!fine) {
+      itab = (int)(e * TB::k(F.T).dlist);
       if (itab >= kMWLE) itab = kMWLE - 1;
     }
-    const int nted = small_ ? F.T.ntlists[itab * kMNB + iband] : F.T.ntlist[itab * kMNB + iband];
-    const int base = small_ ? F.T.ptlists[itab * kMNB + iband] : F.T.ptlist[itab * kMNB + iband];
-    const int *lst = small_ ? F.T.tlists : F.T.tlist;
-    if (nted == 0) {
-      self = true;
-      return;
-    }
-    int count2 = 0;
-    for (;;) {
-      int pick = (int)(nted * Random());
-      if constexpr (sizeof(R) == 4) pick = min(pick, nted - 1);
-      itet = lst[pick + base];
-      count2++;
-      const TetShapeT<R> &s = ts(itet);
-      if ((count2 < 10000) && !((s.e[0] < e) && (s.e[3] > e))) continue;
-      const R dostet = FASTSURF(e, itet) / s.vgt;
-      if (((Random() * maxdostet) > dostet) && (count2 < 10000)) continue;
-      break;
-    }
-    if constexpr (MCB200_FLIGHT_EVENT_STATS != 0)
-      atomicAdd(&I->Y.counters[kStatStateTries], (unsigned long long)count2);
-    if (count2 >= 10000) {
-      self = true;
-    } else {
-      self = false;
-      getK();
-    }
+    const int at = itab * kMNB + ib;
+    count = fine ? F.T.ntlists[at] : F.T.ntlist[at];
+    return fine ? F.T.tlists + F.T.ptlists[at] : F.T.tlist + F.T.ptlist[at];
+  }
+  static __device__ __forceinline__ int list_pick(R u, int count) {
+    const int pick = (int)(count * u);
+    return sizeof(R) == 4 ? min(pick, count - 1) : pick;
   }
 
-  // getK, src/ParticleUtils.cpp:122-284: uniform point on the iso-energy
-  // triangle / quadrangle of tet itet, mapped out of the wedge.
-  __device__ void getK();
+  // get_state, src/ParticleUtils.cpp:48-120: random final state on the
+  // iso-energy surface of band iband (rejection on the tet's DOS share),
+  // one lane for itself (seeding); the flight draws with the whole warp
+  // (final_states).
+  __device__ void get_state() {
+    self = true;
+    if (energy <= 0.0) return;
+    const R e = (R)energy;
+    const R maxdostet = CALDOSTETMAX(e, iband);
+    int nted;
+    const int *lst = energy_list(e, iband, nted);
+    if (nted == 0) return;
+    int count2 = 0;
+    for (;;) {
+      stock(2);
+      itet = lst[list_pick(Random(), nted)];
+      count2++;
+      const TetShapeT<R> &s = ts(itet);
+      if ((count2 < kMaxStateTries) && !((s.e[0] < e) && (s.e[3] > e))) continue;
+      const R dostet = FASTSURF(e, itet) / s.vgt;
+      if (((Random() * maxdostet) > dostet) && (count2 < kMaxStateTries)) continue;
+      break;
+    }
+    if (count2 >= kMaxStateTries) return;
+    self = false;
+    R a, b, c;
+    stock(4);
+    point_on_surface(itet, energy, [this]() { return Random(); }, a, b, c);
+    out_wedge(kx, ky, kz, a, b, c);
+  }
+
+  // getK, src/ParticleUtils.cpp:122-284: uniform point (in the wedge) on the
+  // iso-energy triangle / quadrangle of tet it.
+  template <class Draw>
+  __device__ void point_on_surface(int it, double &en, Draw &&draw, R &xo, R &yo, R &zo) const;
 
   // Band::CALSCATTSUM, src/Band.cpp:1999-2033.
   __device__ R CALSCATTSUM(R eed, int ib) const {
     const R *s = TB::sumscatt(F.T);
     const R *E = TB::energy(F.T);
     if (eed <= (R)0) return s[ib];
-    if (eed >= (R)F.T.emax) return s[(size_t)(kNT - 1) * kMNB + ib];
-    const int itab = min((int)(eed / (R)F.T.dtable), kNT - 2);
+    if (eed >= TB::k(F.T).emax) return s[(size_t)(kNT - 1) * kMNB + ib];
+    const int itab = min((int)(eed / TB::k(F.T).dtable), kNT - 2);
     const R intp = (eed - E[itab]) / (E[itab + 1] - E[itab]);
     return s[(size_t)itab * kMNB + ib] + intp * (s[(size_t)(itab + 1) * kMNB + ib] - s[(size_t)itab * kMNB + ib]);
   }
-
-  // Electron mechanism choice by a running sum over Band::CALSCATTE
-  // (src/Band.cpp:2165-2231) entries, without materialising the 56-entry
-  // array: returns the chosen index or -1 (self-scattering).
-  __device__ int pick_electron_mechanism(R drand) const;
-  __device__ R electron_rate_sum() const;
-  __device__ int pick_hole_mechanism(R drand) const;
-  __device__ R hole_rate_sum() const;
 
   // heat_to_point, src/heat.cpp:169-196 (CIC onto the cell's 8 nodes).
   __device__ void heat_to_point(double e, long long *heat) const {
@@ -678,35 +725,20 @@ struct FlyerT {
       rz = (z - M.lz[kc]) / M.dz[kc];
     }
     const int px = M.nx + 1, pz = M.nz + 1;
-    auto node = [&](int i, int j, int k) { return ((size_t)j * px + i) * pz + k; };
-    tally_add_i64(heat + node(ic, jc, kc), e * (1 - ry) * (1 - rx) * (1 - rz), kEnergyScale);
-    tally_add_i64(heat + node(ic + 1, jc, kc), e * (1 - ry) * rx * (1 - rz), kEnergyScale);
-    tally_add_i64(heat + node(ic, jc, kc + 1), e * (1 - ry) * (1 - rx) * rz, kEnergyScale);
-    tally_add_i64(heat + node(ic + 1, jc, kc + 1), e * (1 - ry) * rx * rz, kEnergyScale);
-    tally_add_i64(heat + node(ic, jc + 1, kc), e * ry * (1 - rx) * (1 - rz), kEnergyScale);
-    tally_add_i64(heat + node(ic + 1, jc + 1, kc), e * ry * rx * (1 - rz), kEnergyScale);
-    tally_add_i64(heat + node(ic, jc + 1, kc + 1), e * ry * (1 - rx) * rz, kEnergyScale);
-    tally_add_i64(heat + node(ic + 1, jc + 1, kc + 1), e * ry * rx * rz, kEnergyScale);
+#pragma unroll 1
+    for (int c = 0; c < 8; ++c) {
+      const int dx = c & 1, dz = (c >> 1) & 1, dy = c >> 2;
+      const R wx = dx ? rx : 1 - rx, wy = dy ? ry : 1 - ry, wz = dz ? rz : 1 - rz;
+      tally_add_i64(heat + ((size_t)(jc + dy) * px + ic + dx) * pz + kc + dz, e * wy * wx * wz, kEnergyScale);
+    }
   }
 
   // ---- final states ----------------------------------------------------
   // The reference draws a final state inside EPSCAT / ESCATII (electrons),
-  // HPSCAT / HSCATII (holes) and Diffuse.  Here the event handlers set up the
-  // mechanism's band, energy and wedge rule (request_scatter,
-  // request_diffuse) and one shared tail, run_final_state, makes the draws
-  // in the reference's order (the wedge: TALIND or a random isym; then
-  // get_state) and applies the routine's epilogue.  One call site of
-  // get_state / TALIND / getK keeps the event loop small enough for the
-  // instruction cache.
-  __device__ void save_old() {
-    fs_eeold = energy;
-    fs_kx = kx; fs_ky = ky; fs_kz = kz;
-    fs_ib = iband; fs_it = itet; fs_is = isym;
-  }
-  __device__ void restore_k() {
-    kx = fs_kx; ky = fs_ky; kz = fs_kz;
-    iband = fs_ib; itet = fs_it; isym = fs_is;
-  }
+  // HPSCAT / HSCATII (holes) and Diffuse.  Here the event handlers only say
+  // which draw is due (draw_kind), and final_states makes it with the whole
+  // warp, in the reference's order: the mechanism, the wedge (TALIND or a
+  // random isym), get_state, and the routine's epilogue.
 
   // FEKLOEM / FEKLOAB / FEKTOEM / FEKTOAB / FEKLAEM / FEKLAAB
   // (src/ElectronPhononScatter.cpp:633-1022), table-driven: the final energy
@@ -716,7 +748,8 @@ struct FlyerT {
   // cumulative sum to a row i, and the final energy is the phonon energy
   // shifted by +-(i / 2) steps of c * edeta.  Below one quantum the emission
   // tables return at once, without a draw.  `which` follows kDispNames.
-  __device__ double fek(int which, double eet) {
+  template <class Draw>
+  __device__ double fek(int which, double eet, Draw &&draw) const {
     const DevTables &T = F.T;
     const bool emit = (which & 1) == 0;
     const int phon = which >> 1;  // 0 LO, 1 TO, 2 LA
@@ -761,16 +794,18 @@ struct FlyerT {
     const int cols = phon == 0 ? (emit ? 120 : 110) : (emit ? 160 : 150);
     const int rows = phon == 0 ? 201 : 51;
     const double *tab = T.disp + T.disp_off[which] + (ei - 1);
-    const double ran = (double)Random();
+    const double ran = (double)draw();
     int i = 0;
     double ksum = 0.0;
     if (which == 0) {  // FEKLOEM wraps before adding: rows 0..199
+#pragma unroll 1
       while (ksum < ran) {
         ++i;
         if (i == rows) { ksum = 1.1; i = 1; }
         ksum += tab[(size_t)(i - 1) * cols];
       }
     } else {
+#pragma unroll 1
       while (ksum < ran) {
         ++i;
         ksum += tab[(size_t)(i - 1) * cols];
@@ -790,137 +825,48 @@ struct FlyerT {
   // Flag_QuantumCorrection the LO / LA / TO events take their final energy
   // from fek, :152-167), ESCATII (:406-497, seciifl = false), HPSCAT
   // (src/HolePhononScatter.cpp:86-146) and HSCATII (:149-234) for mechanism
-  // iscat: the final band and energy, and the wedge rule of the draw
-  // (fs_tal: 1..3 = TALIND(ityp), 0 = a random isym, -1 = none).
-  __device__ void request_scatter(int iscat) {
-    save_old();
+  // iscat: the final band and energy, and the wedge rule of the draw (tal:
+  // 1..3 = TALIND(tal), 0 = a random isym, -1 = none).  Returns whether the
+  // event is a phonon's.
+  template <class Draw>
+  __device__ __forceinline__ bool scatter_setup(int iscat, int carrier, bool quantum, double &en, int &ib, int &tal,
+                                                Draw &&draw) const {
     const DevTables &T = F.T;
-    if (type == 0) {
-      iband = iscat / T.scpre + T.bandof[0];
-      const int m = iscat % T.scpre;
-      if (m + 1 == T.scpre) {  // ESCATII
-        fs_kind = kFsIonize;
-        fs_tal = 0;
-        energy = (energy - T.sieg) / 3.0;
-        return;
-      }
-      fs_kind = kFsPhonon;
-      switch (m) {
-        case 0: fs_tal = 1; break;
-        case 1: energy = energy + T.temptag; fs_tal = 2; break;
-        case 2: energy = energy - T.temptag; fs_tal = 2; break;
-        case 3: energy = energy + T.templag; fs_tal = 2; break;
-        case 4: energy = energy - T.templag; fs_tal = 2; break;
-        case 5: energy = energy + T.templog; fs_tal = 2; break;
-        case 6: energy = energy - T.templog; fs_tal = 2; break;
-        case 7: energy = energy + T.temptaf; fs_tal = 3; break;
-        case 8: energy = energy - T.temptaf; fs_tal = 3; break;
-        case 9: energy = energy + T.templaf; fs_tal = 3; break;
-        case 10: energy = energy - T.templaf; fs_tal = 3; break;
-        case 11: energy = energy + T.temptof; fs_tal = 3; break;
-        case 12: energy = energy - T.temptof; fs_tal = 3; break;
-        default: fs_tal = -1; break;
-      }
-      if (I->M.quantum && (m == 5 || m == 6 || (m >= 9 && m <= 12))) {
-        // the dispersion table of the event: LO 5 / 6, LA 9 / 10, TO 11 / 12
-        // (absorption / emission); the energy before the event
-        static constexpr signed char kTable[13] = {-1, -1, -1, -1, -1, 1, 0, -1, -1, 5, 4, 3, 2};
-        energy = fek(kTable[m], fs_eeold);
-      }
-    } else {
-      iband = iscat / T.scprh + T.bandof[1];
-      const int m = iscat % T.scprh;
-      fs_tal = 0;
-      if (m + 1 == T.scprh) {  // HSCATII
-        fs_kind = kFsIonize;
-        energy = (energy - T.sieg) / 3.0;
-        return;
-      }
-      fs_kind = kFsPhonon;
-      if (m == 1) energy = energy + T.temphop;
-      else if (m == 2) energy = energy - T.temphop;
+    const int per = carrier == 0 ? T.scpre : T.scprh;
+    ib = iscat / per + T.bandof[carrier == 0 ? 0 : 1];
+    const int m = iscat % per;
+    tal = 0;
+    if (m + 1 == per) {  // ESCATII, HSCATII
+      en = (en - T.sieg) / 3.0;
+      return false;
     }
-  }
-  // Set-up of Diffuse, src/CellHit.cpp:243-386 (TALIND(1), get_state, then
-  // the mirror that points the velocity back into the device).
-  __device__ void request_diffuse() {
-    save_old();
-    fs_kind = kFsDiffuse;
-    fs_tal = 1;
-  }
-  // The draws and epilogue of the pending final state.
-  __device__ void run_final_state() {
-    const int kind = fs_kind;
-    fs_kind = kFsNone;
-    if (fs_tal == 0) isym = ((int)((R)48 * Random()) % 48);
-    else if (fs_tal > 0) TALIND(fs_tal);
-    get_state();
-    if (kind == kFsDiffuse) {
-      if (self) restore_k();
-      GetV();
-      switch (idir) {
-        case kUp:
-          if (vx == (R)0) restore_k();
-          if (vx < (R)0) reflect_axis(0);
-          break;
-        case kRight:
-          if (vy == (R)0) restore_k();
-          if (vy > (R)0) reflect_axis(1);
-          break;
-        case kDown:
-          if (vx == (R)0) restore_k();
-          if (vx > (R)0) reflect_axis(0);
-          break;
-        case kLeft:
-          if (vy == (R)0) restore_k();
-          if (vy < (R)0) reflect_axis(1);
-          break;
-        case kFront:
-          if (vz == (R)0) restore_k();
-          if (vz < (R)0) reflect_axis(2);
-          break;
-        case kBack:
-          if (vz == (R)0) restore_k();
-          if (vz > (R)0) reflect_axis(2);
-          break;
-      }
-      return;
+    if (carrier != 0) {
+      if (m == 1) en = en + T.temphop;
+      else if (m == 2) en = en - T.temphop;
+      return true;
     }
-    if (self) {
-      energy = fs_eeold;
-      restore_k();
+    if (m == 0) {
+      tal = 1;
+      return true;
     }
-    if (kind == kFsPhonon && I->M.heat)
-      heat_to_point((energy - fs_eeold) * fabs(charge), type == 0 ? I->Y.heat_e : I->Y.heat_h);
+    tal = m > 12 ? -1 : (m <= 6 ? 2 : 3);
+    if (m > 12) return true;
+    if (quantum && (m == 5 || m == 6 || m >= 9)) {
+      // the dispersion table of the event: LO 5 / 6, LA 9 / 10, TO 11 / 12
+      // (absorption / emission); the energy before the event
+      en = fek(m <= 6 ? 6 - m : 14 - m, en, draw);
+      return true;
+    }
+    const int q = (m - 1) >> 1;  // absorption (m odd) and emission of each phonon
+    const double ph = q == 0 ? T.temptag : q == 1 ? T.templag : q == 2 ? T.templog : q == 3 ? T.temptaf
+                      : q == 4 ? T.templaf : T.temptof;
+    en = (m & 1) ? en + ph : en - ph;
+    return true;
   }
 
-  // ElectronPhononScatter (src/ElectronPhononScatter.cpp:5-95) and
-  // HolePhononScatter (src/HolePhononScatter.cpp:4-83): real or
-  // self-scattering against the variable-gamma majorant; a real event
-  // leaves the mechanism search to run_pick.
-  __device__ void phonon_event() {
-    const R scasum = CALSCATTSUM((R)energy, iband);
-    const R g = tf(itet).gam;
-    const R drand = scasum > g ? Random() * scasum : Random() * g;
-    if (scasum < drand) {
-      self = true;
-      return;
-    }
-    self = false;
-    pick_drand = drand;
-    pick_pending = true;
-  }
-  // The mechanism search of ElectronPhononScatter / HolePhononScatter
-  // (src/ElectronPhononScatter.cpp:47-63, src/HolePhononScatter.cpp:49-66).
-  __device__ void run_pick() {
-    pick_pending = false;
-    const int iscat = type == 0 ? pick_electron_mechanism(pick_drand) : pick_hole_mechanism(pick_drand);
-    if (iscat < 0) {
-      self = true;
-      return;
-    }
-    request_scatter(iscat);
-  }
+  // The final-state draws of the lanes in `owners` (draw_kind), one owner at
+  // a time by the whole warp; every lane of the warp calls it.
+  __device__ __forceinline__ void final_states(unsigned owners);
 
   // GetImpScRate, src/ElectronImpurityScatter.cpp:62-126 (Brooks-Herring,
   // bhmrtfl = false).  FP32: the same rate written as
@@ -930,18 +876,8 @@ struct FlyerT {
       return eel < imp_ecut ? imp_a * m_sqrt(eel) / ((R)1 + imp_b * eel) : (R)0;
     } else {
       const DevTables &T = F.T;
-      if ((eel * T.eV0 < 0.120) && (DA * T.conc0 >= 1e22)) {
-        const double eebeta = T.frickel * 4 * kPiD * Rho / (2.0 * T.meld * T.eps_si);
-        if (I->M.surface_scatter && I->M.surface_impurity && I->M.in_surf[cell_index()]) {
-          // The reference's surface-impurity formula is commented out there and
-          // leaves the rate unset; the engine treats it as zero.
-          return 0.0;
-        }
-        const double fr = T.frickel * Rho;
-        return DA * T.meld * sqrt(2.0 * T.meld * eel) /
-               (kPiD * (fr * fr) * (1.0 + 4.0 * eel * T.melt / (eebeta * T.meld)));
-      }
-      return 0.0;
+      if (!(eel * T.eV0 < 0.120) || imp_a == 0.0) return 0.0;
+      return imp_a * sqrt(2.0 * T.meld * eel) / (imp_c * (1.0 + 4.0 * eel * T.melt / imp_b));
     }
   }
 
@@ -949,30 +885,16 @@ struct FlyerT {
   // BH rate over the tet's energy span.
   __device__ R GetImpScGamma() const {
     const DevTables &T = F.T;
-    R eemax;
-    if constexpr (sizeof(R) == 4) eemax = imp_emax;
-    else eemax = T.frickel * 4 * kPiD * Rho / (8.0 * T.melt * T.eps_si);
+    const R eemax = imp_emax;
     const TetFlightT<R> &s = tf(itet);
-    R gammax;
-    if (eemax < s.e0) gammax = GetImpScRate(s.e0);
-    else if (eemax > s.e3) gammax = GetImpScRate(s.e3);
-    else gammax = GetImpScRate(eemax);
-    const R floor_ = (R)(1.0 / T.scrt0);
+    // the rate at the energy of the span nearest its peak (one evaluation)
+    const R gammax = GetImpScRate(eemax < s.e0 ? s.e0 : (eemax > s.e3 ? s.e3 : eemax));
+    const R floor_ = TB::k(T).gamma_floor;
     return gammax > floor_ ? gammax : floor_;
   }
 
   // EleImpScUpdateK, src/ElectronImpurityScatter.cpp:188-306.
   __device__ void EleImpScUpdateK();
-
-  // ElectronImpurityScatter, src/ElectronImpurityScatter.cpp:128-185.
-  __device__ void ElectronImpurityScatter() {
-    const R gamimp = GetImpScRate((R)energy);
-    if (gamimp < Random() * imp_gamma) {
-      self = true;
-    } else {
-      EleImpScUpdateK();
-    }
-  }
 
   // GetSurfScRate, src/ParSurfaceScatter.cpp:3-45.
   __device__ void GetSurfScRate() {
@@ -1008,42 +930,25 @@ struct FlyerT {
       catch_ = true;
       return;
     }
+    // the face, in the new cell's frame (FP32) or absolute; faces come in
+    // pairs per axis, the odd one towards larger coordinates
     const DevMesh &M = I->M;
-    if constexpr (Real::kCellRelative) {  // the face, in the new cell's frame
-      switch (idir) {
-        case kUp: x = M.dxf[ic - 1]; ic--; break;
-        case kDown: x = 0; ic++; break;
-        case kRight:
-          y = 0;
-          jc++;
-          tally_add_i64(I->Y.rcurrent + jc, charge, kChargeScale);
-          break;
-        case kLeft:
-          y = M.dyf[jc - 1];
-          tally_add_i64(I->Y.lcurrent + jc, charge, kChargeScale);
-          jc--;
-          break;
-        case kFront: z = M.dzf[kc - 1]; kc--; break;
-        case kBack: z = 0; kc++; break;
-      }
+    const int axis = idir >> 1, up = idir & 1;
+    const int old = axis == 0 ? ic : (axis == 1 ? jc : kc), to = up ? old + 1 : old - 1;
+    R at;
+    if constexpr (Real::kCellRelative) {
+      const float *w = axis == 0 ? M.dxf : (axis == 1 ? M.dyf : M.dzf);
+      at = up ? (R)0 : w[to];
     } else {
-      switch (idir) {
-        case kUp: x = M.lx[ic]; ic--; break;
-        case kDown: x = M.lx[ic + 1]; ic++; break;
-        case kRight:
-          y = M.ly[jc + 1];
-          jc++;
-          tally_add_i64(I->Y.rcurrent + jc, charge, kChargeScale);
-          break;
-        case kLeft:
-          y = M.ly[jc];
-          tally_add_i64(I->Y.lcurrent + jc, charge, kChargeScale);
-          jc--;
-          break;
-        case kFront: z = M.lz[kc]; kc--; break;
-        case kBack: z = M.lz[kc + 1]; kc++; break;
-      }
+      const double *l = axis == 0 ? M.lx : (axis == 1 ? M.ly : M.lz);
+      at = l[old + up];
     }
+    if (axis == 0) { x = at; ic = to; }
+    else if (axis == 1) {
+      y = at;
+      jc = to;
+      tally_add_i64((up ? I->Y.rcurrent : I->Y.lcurrent) + old + up, charge, kChargeScale);
+    } else { z = at; kc = to; }
   }
   // Period, src/CellHit.cpp:416-432.
   __device__ void Period() {
@@ -1148,8 +1053,15 @@ struct FlyerT {
       Ex = f[0];
       Ey = f[1];
       Ez = f[2];
-      Rho = M.rho[c];
-      DA = M.da[c];
+      if (type == 0) {
+        const double2 *r = M.cell64 + 3 * (size_t)c;
+        const double2 a = r[0], b = r[1], m = r[2];
+        imp_a = a.x;
+        imp_b = a.y;
+        imp_c = b.x;
+        imp_emax = b.y;
+        imp_beta = m.x;
+      }
     } else {
       const float4 *r = M.cell32 + 3 * (size_t)c;
       if (type == 0) {
@@ -1168,8 +1080,8 @@ struct FlyerT {
   }
   // HitCell, src/CellHit.cpp:96-211.  Returns false when the particle would
   // leave the device through a PASS / GENERATE face on the outer y boundary.
-  __device__ bool HitCell() {
-    const int imot = I->M.motion[(size_t)cell_index() * 6 + idir];
+  // imot: the face's rule; u: the draw of a SCATTOX face without surface scattering.
+  __device__ bool HitCell(int imot, R u) {
     if (imot == kPass || imot == kGenerate || imot == kGenRef) {
       if ((idir == kLeft && jc == 0) || (idir == kRight && jc == I->M.ny - 1)) return false;
     }
@@ -1178,8 +1090,8 @@ struct FlyerT {
     else if (imot == kScattOx) {
       if (I->M.surface_scatter) Reflect();
       else {
-        if (Random() > (R)F.T.difpr[type]) Reflect();
-        else request_diffuse();
+        if (u > (R)F.T.difpr[type]) Reflect();
+        else draw_kind = kDrawDiffuse;
       }
     } else if (imot == kPeriod) Period();
     else if (imot == kGenerate || imot == kGenRef) {
@@ -1198,23 +1110,13 @@ struct FlyerT {
     load_cell_fields();
     return true;
   }
-  // ParticleSurfaceScatter, src/ParSurfaceScatter.cpp:48-61, with the
-  // surface-phonon branches' drand defined (see file note).
-  __device__ void surface_event() {
-    if (Random() * surf_gamma < rough_rate) {
-      idir = I->M.surface_dir[min(max(I->M.nearest_surf[cell_index()], 0), kMaxSurfaces - 1)];
-      request_diffuse();
-      return;
-    }
-    self = false;
-    pick_drand = Random() * (type == 0 ? electron_rate_sum() : hole_rate_sum());
-    pick_pending = true;
-  }
-
   // One particle, one step: particle_fly, src/mcmodel.cpp:1874-2161, split
-  // into begin (the set-up before the event loop), iterate (one pass of the
-  // loop; true when the particle's step is over) and finish (the tallies
-  // after the loop), so a kernel can interleave particles on one lane.
+  // into begin (the set-up before the event loop), one pass of the loop as
+  // advance (to the next event, and the events that are done on the spot),
+  // run_pending and final_states (the work the others left) and settle (the
+  // end of the pass; true when the particle's step is over), and finish (the
+  // tallies after the loop), so a kernel can interleave particles on one
+  // lane and keep a lane's pending work until other lanes have some too.
   // Loop state (particle_fly's locals):
   bool get_tet, get_cell, get_ph, get_imp, get_surf, too_far;
   R ssnl, imprnl, phrnl, TetTf, CellTf;
@@ -1222,8 +1124,8 @@ struct FlyerT {
 
   __device__ void begin() {
     catch_ = false;
-    pick_pending = false;
-    fs_kind = kFsNone;
+    imp_pending = false;
+    draw_kind = kDrawNone;
     loc_mode = kLocNone;
     get_tet = get_cell = get_ph = get_imp = get_surf = true;
     ssnl = imprnl = phrnl = 0;
@@ -1238,33 +1140,67 @@ struct FlyerT {
     imp_gamma = 0;
   }
 
-  __device__ bool iterate() {
+  // The drift pass (no begin(): the cell's fields, band and velocity are
+  // loaded).  no_event: whether the step certainly ends before the first
+  // event, from the same times as advance() compares but without forming
+  // the quotients: an event at num / rate > T, for every rounding of it, is
+  // num > rate T with a margin.  drift: the step's motion as advance() makes
+  // it; false (nothing changed) when the energy would turn negative.
+  __device__ __forceinline__ bool no_event() const;
+  __device__ __forceinline__ bool drift() {
+    const R T = (R)left_time;
+    const double e = energy + (vx * Ex + vy * Ey + vz * Ez) * T;
+    if (e < 0) return false;
+    energy = e;
+    kx += Ex * T;
+    ky += Ey * T;
+    kz += Ez * T;
+    x += vx * T;
+    y += vy * T;
+    z += vz * T;
+    return true;
+  }
+
+  // What is left after an advance().
+  enum : int { kGoOn = 0, kStepOver = 1, kPending = 2, kDraw = 3 };
+  __device__ int advance() {
     GetV();
     if (++loop > kMaxEvents) {
       count(I->Y, kCntTooManyEvents);
       catch_ = true;
-      return true;
+      return kStepOver;
     }
     if (get_tet) { TetTf = TetTime(); get_tet = false; }
     if (get_cell) { CellTf = CellTime(); get_cell = false; }
-    if (get_ph) { phrnl = -m_log(Random()); get_ph = false; }
+    const bool impurities = iband == F.T.bandof[0];
+    const bool surface = I->M.surface_scatter && I->M.in_surf[cell_index()];
+    // the clocks that are to be drawn, in the reference's order (rolled: one
+    // copy of the stream and the logarithm in the loop's code)
+    unsigned clocks = (get_ph ? 1u : 0u) | (impurities && get_imp ? 2u : 0u) | (surface && get_surf ? 4u : 0u);
+    // FP32: a block serves the pass's four draws at most; FP64: its clocks
+    stock(sizeof(R) == 4 ? 4u : (uint32_t)__popc(clocks));
+#pragma unroll 1
+    while (clocks) {
+      const R v = -m_log(Random());
+      if (clocks & 1u) { phrnl = v; get_ph = false; }
+      else if (clocks & 2u) { imprnl = v; get_imp = false; }
+      else { ssnl = v; get_surf = false; }
+      clocks &= clocks - 1u;
+    }
     const R g = tf(itet).gam;
     R PhScTf, ImpScTf, SurfScTf, Tf;
     PhScTf = phrnl / g;
-    if (iband == F.T.bandof[0]) {
-      if (get_imp) { imprnl = -m_log(Random()); get_imp = false; }
+    if (impurities) {
       imp_gamma = GetImpScGamma();
       ImpScTf = imprnl / imp_gamma;
     } else {
       ImpScTf = (R)(2 * I->dt);
-      imp_gamma = (R)(1.0 / F.T.scrt0);
+      imp_gamma = TB::k(F.T).gamma_floor;
     }
-    if (I->M.surface_scatter && I->M.in_surf[cell_index()]) {
-      if (get_surf) { ssnl = -m_log(Random()); get_surf = false; }
+    SurfScTf = (R)(2 * I->dt);
+    if (surface) {
       GetSurfScRate();
-      SurfScTf = (surf_gamma > 0 && ssnl > 0) ? ssnl / surf_gamma : (R)(2 * I->dt);
-    } else {
-      SurfScTf = (R)(2 * I->dt);
+      if (surf_gamma > 0 && ssnl > 0) SurfScTf = ssnl / surf_gamma;
     }
     // Min(..., flag), src/Constant_GlobalVariable_MathFunction.cpp:92-118
     int flag = 1;
@@ -1277,7 +1213,7 @@ struct FlyerT {
     if constexpr (sizeof(R) == 8) {
       if (Tf < kMyZero) {
         catch_ = true;
-        return true;
+        return kStepOver;
       }
     } else {
       // float event times that round to zero (or below) are events now
@@ -1286,7 +1222,7 @@ struct FlyerT {
         if (++zero_run > kMaxZeroTimeEvents) {
           count(I->Y, kCntZeroTime);
           catch_ = true;
-          return true;
+          return kStepOver;
         }
       } else {
         zero_run = 0;
@@ -1313,7 +1249,15 @@ struct FlyerT {
     z += vz * Tf;
     if (energy < 0) {
       catch_ = true;
-      return true;
+      return kStepOver;
+    }
+    ev = flag;
+    int imot = 0;
+    if (flag == 2) imot = I->M.motion[(size_t)cell_index() * 6 + idir];
+    R u = 0;  // the event's draw
+    if ((flag >= 3 && flag <= 5) || (imot == kScattOx && !I->M.surface_scatter)) {
+      if constexpr (sizeof(R) == 8) stock(1);
+      u = Random();
     }
     switch (flag) {
       case 1:
@@ -1322,7 +1266,7 @@ struct FlyerT {
         get_cell = true;
         break;
       case 2:
-        if (HitCell()) {
+        if (HitCell(imot, u)) {
           get_tet = true;
           get_cell = true;
         } else {
@@ -1338,35 +1282,62 @@ struct FlyerT {
           too_far = true;
         }
         break;
-      case 3:
-        phonon_event();
+      case 3: {
+        // ElectronPhononScatter (src/ElectronPhononScatter.cpp:5-95) and
+        // HolePhononScatter (src/HolePhononScatter.cpp:4-83): real or
+        // self-scattering against the variable-gamma majorant
+        const R scasum = CALSCATTSUM((R)energy, iband);
+        pick_drand = u * (scasum > g ? scasum : g);
+        self = scasum < pick_drand;
+        if (!self) draw_kind = kDrawPick;
         break;
+      }
       case 4:
-        if (type == 0) ElectronImpurityScatter();
+        // ElectronImpurityScatter, src/ElectronImpurityScatter.cpp:128-185
+        // (electrons: a hole's impurity time is past the step's end)
+        if (GetImpScRate((R)energy) < u * imp_gamma) self = true;
+        else imp_pending = true;
         break;
       case 5:
-        surface_event();
+        // ParticleSurfaceScatter, src/ParSurfaceScatter.cpp:48-61, with the
+        // surface-phonon branches' drand defined (see file note)
+        if (u * surf_gamma < rough_rate) {
+          idir = I->M.surface_dir[min(max(I->M.nearest_surf[cell_index()], 0), kMaxSurfaces - 1)];
+          draw_kind = kDrawDiffuse;
+        } else {
+          draw_kind = kDrawPickSurface;
+        }
         break;
     }
-    // shared tails: mechanism search, final-state draw, k-point search
-    if (pick_pending) run_pick();
-    if (fs_kind != kFsNone) run_final_state();
+    if (draw_kind != kDrawNone) return kDraw;
+    if (imp_pending || loc_mode != kLocNone) return kPending;
+    return settle() ? kStepOver : kGoOn;
+  }
+
+  __device__ void run_pending() {
+    if (imp_pending) {
+      imp_pending = false;
+      EleImpScUpdateK();
+    }
     if (loc_mode != kLocNone) run_locate();
-    if (flag == 3) {
+  }
+
+  __device__ __forceinline__ bool settle() {
+    if (ev == 3) {
       if (!self) {
         get_tet = true;
         get_cell = true;
-        count(I->Y, kCntPhonon);
+        ++n_ph;
       }
       get_ph = true;
-    } else if (flag == 4) {
+    } else if (ev == 4) {
       if (!self) {
         get_tet = true;
         get_cell = true;
-        count(I->Y, kCntImpurity);
+        ++n_imp;
       }
       get_imp = true;
-    } else if (flag == 5) {
+    } else if (ev == 5) {
       if (!self) {
         get_tet = true;
         get_cell = true;
@@ -1378,11 +1349,16 @@ struct FlyerT {
   }
 
   // Returns 0 done, 1 caught, 2 unfinished (outer-boundary PASS).  A
-  // caller that sums the particles' event counts itself (`loop`, one
+  // caller that sums the particles' events itself (`loop`, n_ph, n_imp: one
   // simulation per launch) passes kCountEvents = false.
   template <bool kCountEvents = true>
   __device__ int finish() {
-    if constexpr (kCountEvents) atomicAdd(&I->Y.counters[kCntEvents], (unsigned long long)loop);
+    if constexpr (kCountEvents) {
+      atomicAdd(&I->Y.counters[kCntEvents], (unsigned long long)loop);
+      if (n_ph) atomicAdd(&I->Y.counters[kCntPhonon], (unsigned long long)n_ph);
+      if (n_imp) atomicAdd(&I->Y.counters[kCntImpurity], (unsigned long long)n_imp);
+      n_ph = n_imp = 0;
+    }
     if (catch_) {
       count(I->Y, kCntCaught);
       return 1;
@@ -1392,14 +1368,6 @@ struct FlyerT {
       return 2;
     }
     return 0;
-  }
-
-  __device__ int fly() {
-    begin();
-    if (left_time > 0)
-      while (!iterate()) {
-      }
-    return finish();
   }
 };
 using Flyer = FlyerT<double>;

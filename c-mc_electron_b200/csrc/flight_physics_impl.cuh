@@ -16,9 +16,9 @@ __device__ __forceinline__ R dfii(R x1, R y1, R z1, R x2, R y2, R z2, R x3, R y3
 
 // Band::SURF, src/Band.cpp:194-332.
 template <typename R>
-__device__ R FlyerT<R>::SURF(R eps, int it) const {
-  const int4 nd = F.T.tnode[it];
-  const V4 *kn = TB::knode(F.T);
+__device__ __noinline__ R FlyerT<R>::SURF(const DevTables &T, R eps, int it) {
+  const int4 nd = T.tnode[it];
+  const V4 *kn = TB::knode(T);
   const V4 k0 = kn[nd.x], k1 = kn[nd.y], k2 = kn[nd.z], k3 = kn[nd.w];
   const R e0 = k0.w, e1 = k1.w, e2 = k2.w, e3 = k3.w;
   if (!(eps > e0 && eps < e3)) return 0;
@@ -63,18 +63,18 @@ __device__ R FlyerT<R>::SURF(R eps, int it) const {
 
 // getK, src/ParticleUtils.cpp:122-284.
 template <typename R>
-__device__ void FlyerT<R>::getK() {
-  const R rv1 = (R)1.0 - m_sqrt(Random());
-  const R rv2 = Random() * ((R)1.0 - rv1);
-  const int4 nd = F.T.tnode[itet];
+template <class Draw>
+__device__ void FlyerT<R>::point_on_surface(int it, double &en, Draw &&draw, R &xkl, R &ykl, R &zkl) const {
+  const R rv1 = (R)1.0 - m_sqrt(draw());
+  const R rv2 = draw() * ((R)1.0 - rv1);
+  const int4 nd = F.T.tnode[it];
   const V4 *kn = TB::knode(F.T);
   const V4 k0 = kn[nd.x], k1 = kn[nd.y], k2 = kn[nd.z], k3 = kn[nd.w];
-  R e = (R)energy;
+  R e = (R)en;
   if ((e < k0.w) || (e > k3.w)) {
-    e = k0.w + (k3.w - k0.w) * Random();
-    energy = e;
+    e = k0.w + (k3.w - k0.w) * draw();
+    en = e;
   }
-  R xkl, ykl, zkl;
   if (e <= k1.w) {
     R r = (e - k0.w) / (k1.w - k0.w);
     const R ax = r * (k1.x - k0.x), ay = r * (k1.y - k0.y), az = r * (k1.z - k0.z);
@@ -98,7 +98,7 @@ __device__ void FlyerT<R>::getK() {
     const R a2 = dfii(dx, dy, dz, bx, by, bz, cx, cy, cz);
     const R a3 = dfii(ax, ay, az, dx, dy, dz, cx, cy, cz);
     const R a4 = dfii(ax, ay, az, bx, by, bz, dx, dy, dz);
-    const R ar = Random() * (a1 + a2 + a3 + a4);
+    const R ar = draw() * (a1 + a2 + a3 + a4);
     if (ar < a1) {
       xkl = rv1 * (bx - ax) + rv2 * (cx - ax) + ax;
       ykl = rv1 * (by - ay) + rv2 * (cy - ay) + ay;
@@ -127,7 +127,6 @@ __device__ void FlyerT<R>::getK() {
     ykl = rv1 * (by - ay) + rv2 * (cy - ay) + ay + k3.y;
     zkl = rv1 * (bz - az) + rv2 * (cz - az) + az + k3.z;
   }
-  out_wedge(kx, ky, kz, xkl, ykl, zkl);
 }
 
 // Interpolation weight of the energy tables (CALSCATTE / CALSCATTH prologue).
@@ -143,10 +142,10 @@ __device__ __forceinline__ TabPosT<R> tab_pos(const DevTables &T, R eed) {
   TabPosT<R> p;
   const R *E = Tab<R>::energy(T);
   if (eed <= (R)0) { p.mode = 0; p.itab = 0; p.intp = 0; }
-  else if (eed >= (R)T.emax) { p.mode = 1; p.itab = kNT - 1; p.intp = 0; }
+  else if (eed >= Tab<R>::k(T).emax) { p.mode = 1; p.itab = kNT - 1; p.intp = 0; }
   else {
     p.mode = 2;
-    p.itab = min((int)(eed / (R)T.dtable), kNT - 2);
+    p.itab = min((int)(eed / Tab<R>::k(T).dtable), kNT - 2);
     p.intp = (eed - E[p.itab]) / (E[p.itab + 1] - E[p.itab]);
   }
   return p;
@@ -163,89 +162,199 @@ __device__ __forceinline__ R tab_at_strided(const R *tab, int stride, const TabP
   return a + p.intp * (b - a);
 }
 
-// Entry idx of Band::CALSCATTE (src/Band.cpp:2165-2231) for initial band ib.
+// Entry idx of Band::CALSCATTE (src/Band.cpp:2165-2231, electrons) or
+// Band::CALSCATTH (:2098-2162, holes) for initial band ini.
 template <typename R>
-__device__ __forceinline__ R electron_rate(const DevTables &T, const TabPosT<R> &p, int ini, int idx) {
-  const int f = idx / T.scpre, is = idx % T.scpre;
-  if (is < T.scpre - 1)
-    return Tab<R>::scatte(T)[(is * 4 + f) * 4 + ini] * tab_at(Tab<R>::dose(T) + (size_t)(is * 4 + f) * kNT, p);
-  return tab_at(Tab<R>::scattiie(T) + (size_t)(f * 4 + ini) * kNT, p);
-}
-// Entry idx of Band::CALSCATTH (src/Band.cpp:2098-2162).
-template <typename R>
-__device__ __forceinline__ R hole_rate(const DevTables &T, const TabPosT<R> &p, int ini, int idx) {
-  const int f = idx / T.scprh, is = idx % T.scprh;
-  if (is < T.scprh - 1)
-    return Tab<R>::scatth(T)[(is * 3 + f) * 3 + ini] * tab_at(Tab<R>::dosh(T) + (size_t)(is * 3 + f) * kNT, p);
-  return tab_at(Tab<R>::scattiih(T) + (size_t)(f * 3 + ini) * kNT, p);
+__device__ __forceinline__ R scatter_rate(const DevTables &T, const TabPosT<R> &p, int carrier, int ini, int idx) {
+  const int per = carrier == 0 ? T.scpre : T.scprh, nb = carrier == 0 ? 4 : 3;
+  const int f = idx / per, is = idx % per;
+  const bool ion = is == per - 1;
+  const R *tab = carrier == 0 ? (ion ? Tab<R>::scattiie(T) : Tab<R>::dose(T))
+                              : (ion ? Tab<R>::scattiih(T) : Tab<R>::dosh(T));
+  const R v = tab_at(tab + (size_t)(ion ? f * nb + ini : is * nb + f) * kNT, p);
+  if (ion) return v;
+  return (carrier == 0 ? Tab<R>::scatte(T) : Tab<R>::scatth(T))[(is * nb + f) * nb + ini] * v;
 }
 
-// Mechanism search of ElectronPhononScatter, src/ElectronPhononScatter.cpp:47-63.
+// The final-state draws of a warp's lanes, one owner at a time.
+//
+// A draw made by its lane alone is a serial chain of dependent loads (the
+// mechanism's running sum over up to 56 tabulated rates, then about 11
+// rejected tetrahedra) that the warp's other lanes wait for.  Here lane l
+// evaluates rates l and l + 32, and, since draw n of a particle's stream is
+// a function of n alone, lane l also holds draw first + l and tests the
+// tetrahedron that draw would pick; the reference's sequence is then read
+// off the lanes' votes, with the same draws used for the same decisions.
 template <typename R>
-__device__ int FlyerT<R>::pick_electron_mechanism(R drand) const {
-  const TabPosT<R> p = tab_pos(F.T, (R)energy);
-  const int ini = iband - F.T.bandof[0], n = F.T.scpre * F.T.nband[0];
-  int iscat = -1;
-  R dscat = 0;
-  while (drand > dscat) {
-    iscat = iscat + 1;
-    if (iscat >= n) return -1;
-    dscat = dscat + electron_rate(F.T, p, ini, iscat);
+__device__ __forceinline__ void FlyerT<R>::final_states(unsigned owners) {
+  const DevTables &T = F.T;
+  const unsigned lane = threadIdx.x & 31u;
+  const unsigned all = 0xffffffffu;
+#pragma unroll 1
+  for (; owners; owners &= owners - 1u) {
+    const int src = __ffs(owners) - 1;
+    const uint32_t o_uid = __shfl_sync(all, uid, src), o_sub = __shfl_sync(all, sub, src);
+    const uint32_t o_step = __shfl_sync(all, step_, src);
+    const unsigned long long o_seed = __shfl_sync(all, (unsigned long long)I->seed, src);
+    // the owner's draws from `at` on; lane l holds draw first + l
+    uint32_t at = __shfl_sync(all, n, src), first = at;
+    R ahead = (R)0;
+    auto look_ahead = [&]() {
+      first = at;
+      if constexpr (sizeof(R) == 8) ahead = mcb200_uniform(o_seed, o_uid, o_step, o_sub, first + lane);
+      else ahead = mcb200_uniform_f32(o_seed, o_uid, o_step, o_sub, first + lane);
+    };
+    auto draw = [&]() -> R {
+      const R v = __shfl_sync(all, ahead, (int)(at - first));
+      ++at;
+      return v;
+    };
+    look_ahead();
+    const int kind = __shfl_sync(all, draw_kind, src);
+    const int carrier = __shfl_sync(all, type, src);
+    const double e_old = __shfl_sync(all, energy, src);
+    const R q_x = __shfl_sync(all, kx, src), q_y = __shfl_sync(all, ky, src), q_z = __shfl_sync(all, kz, src);
+    int ib = __shfl_sync(all, iband, src), is = __shfl_sync(all, isym, src), it = __shfl_sync(all, itet, src);
+    double e_new = e_old;
+    R o_x = (R)0, o_y = (R)0, o_z = (R)0;
+    bool real = true, phonon = false;
+    int tal = 1;  // Diffuse: TALIND(1)
+    if (kind != kDrawDiffuse) {
+      // the mechanism (src/ElectronPhononScatter.cpp:47-63,
+      // src/HolePhononScatter.cpp:49-66): the first whose running sum of
+      // rates reaches drand, added in the reference's order
+      const TabPosT<R> pos = tab_pos(T, (R)e_old);
+      const int count = carrier == 0 ? T.scpre * T.nband[0] : T.scprh * T.nband[1];  // at most 14 x 4
+      const int ini = ib - T.bandof[carrier == 0 ? 0 : 1];
+      R r0 = (R)0, r1 = (R)0;
+      if ((int)lane < count) r0 = scatter_rate<R>(T, pos, carrier, ini, (int)lane);
+      if ((int)lane + 32 < count) r1 = scatter_rate<R>(T, pos, carrier, ini, (int)lane + 32);
+      R drand = __shfl_sync(all, pick_drand, src);
+      if (kind == kDrawPickSurface) {
+        R sum = (R)0;
+        for (int i = 0; i < count; ++i) sum += __shfl_sync(all, i < 32 ? r0 : r1, i & 31);
+        drand = draw() * sum;
+      }
+      int iscat = -1;
+      R dscat = (R)0;
+#pragma unroll 1
+      while (drand > dscat) {
+        if (++iscat >= count) {
+          iscat = -1;
+          break;
+        }
+        dscat = dscat + __shfl_sync(all, iscat < 32 ? r0 : r1, iscat & 31);
+      }
+      real = iscat >= 0;
+      if (real) {
+        const bool quantum = __shfl_sync(all, (int)I->M.quantum, src) != 0;
+        phonon = scatter_setup(iscat, carrier, quantum, e_new, ib, tal, draw);
+      }
+    }
+    if (real) {
+      if (tal == 0) is = ((int)((R)48 * draw()) % 48);
+      else if (tal > 0) {
+        const int valley = final_valley(tal, q_x, q_y, q_z, draw);
+        is = (int)(draw() * (R)8.0) + 8 * (valley - 1);
+      }
+      // get_state, src/ParticleUtils.cpp:48-120
+      real = false;
+      const R e = (R)e_new;
+      int nted = 0;
+      const int *lst = nullptr;
+      if (e_new > 0.0) lst = energy_list(e, ib, nted);
+      if (nted > 0) {
+        const R most = CALDOSTETMAX(e, ib);
+        int tries = 0;
+#pragma unroll 1
+        for (bool open = true; open;) {
+          look_ahead();
+          const int mine = lst[list_pick(ahead, nted)];
+          const TetShapeT<R> &s = ts(mine);
+          const bool holds = (s.e[0] < e) && (s.e[3] > e);
+          const R next = __shfl_down_sync(all, ahead, 1);
+          const bool kept = holds && !(next * most > FASTSURF(e, mine) / s.vgt);
+          const unsigned hold = __ballot_sync(all, holds), keep = __ballot_sync(all, kept);
+          // the sequence of tries: one draw for a tetrahedron off the energy,
+          // two for one that is tested (the last lane's test needs the next
+          // draws: it opens the next round)
+          unsigned q = 0;
+#pragma unroll 1
+          while (q < 31u) {
+            ++tries;
+            const bool last = tries >= kMaxStateTries;
+            if (!last && !((hold >> q) & 1u)) {
+              ++q;
+              continue;
+            }
+            q += 2;
+            if (last || ((keep >> (q - 2u)) & 1u)) {
+              it = __shfl_sync(all, mine, (int)q - 2);
+              open = false;
+              break;
+            }
+          }
+          at = first + q;
+        }
+        real = tries < kMaxStateTries;
+        if (real) {
+          look_ahead();
+          R a, b, c;
+          point_on_surface(it, e_new, draw, a, b, c);
+          out_wedge(S.sym[is], o_x, o_y, o_z, a, b, c);
+        }
+      }
+    }
+    if ((int)lane != src) continue;
+    skip_to(at);
+    draw_kind = kDrawNone;
+    self = !real;
+    if (kind != kDrawDiffuse) {
+      if (!real) continue;
+      kx = o_x; ky = o_y; kz = o_z;
+      energy = e_new;
+      iband = ib; itet = it; isym = is;
+      if (phonon && I->M.heat)
+        heat_to_point((e_new - e_old) * fabs(charge), type == 0 ? I->Y.heat_e : I->Y.heat_h);
+      continue;
+    }
+    // Diffuse, src/CellHit.cpp:243-386: the old state again when the new one
+    // does not move across the face's axis, mirrored when it moves out
+    if (real) energy = e_new;
+    const int axis = idir >> 1;
+    const V4 w = *reinterpret_cast<const V4 *>(tf(real ? it : itet).v);
+    R wx, wy, wz;
+    out_wedge(S.sym[real ? is : isym], wx, wy, wz, w.x, w.y, w.z);
+    const R across = m_pick3((uint32_t)axis, wx, wy, wz);
+    if (real && across != (R)0) {
+      kx = o_x; ky = o_y; kz = o_z;
+      itet = it; isym = is;
+    }
+    if ((idir & 1) ? across > (R)0 : across < (R)0) reflect_axis(axis);
   }
-  return iscat;
-}
-template <typename R>
-__device__ R FlyerT<R>::electron_rate_sum() const {
-  const TabPosT<R> p = tab_pos(F.T, (R)energy);
-  const int ini = iband - F.T.bandof[0], n = F.T.scpre * F.T.nband[0];
-  R s = 0;
-  for (int i = 0; i < n; ++i) s += electron_rate(F.T, p, ini, i);
-  return s;
-}
-// Mechanism search of HolePhononScatter, src/HolePhononScatter.cpp:49-66.
-template <typename R>
-__device__ int FlyerT<R>::pick_hole_mechanism(R drand) const {
-  const TabPosT<R> p = tab_pos(F.T, (R)energy);
-  const int ini = iband - F.T.bandof[1], n = F.T.scprh * F.T.nband[1];
-  int iscat = -1;
-  R dscat = 0;
-  while (drand > dscat) {
-    iscat = iscat + 1;
-    if (iscat >= n) return -1;
-    dscat = dscat + hole_rate(F.T, p, ini, iscat);
-  }
-  return iscat;
-}
-template <typename R>
-__device__ R FlyerT<R>::hole_rate_sum() const {
-  const TabPosT<R> p = tab_pos(F.T, (R)energy);
-  const int ini = iband - F.T.bandof[1], n = F.T.scprh * F.T.nband[1];
-  R s = 0;
-  for (int i = 0; i < n; ++i) s += hole_rate(F.T, p, ini, i);
-  return s;
 }
 
 // EleImpScUpdateK, src/ElectronImpurityScatter.cpp:188-306: Brooks-Herring
-// final state in the ellipsoidal-valley picture, accepted by rejection.
-// FP64 keeps the reference's pow(., -2.0); FP32 writes it as 1 / q^2.
+// final state in the ellipsoidal-valley picture, accepted by rejection (the
+// reference's pow(q, -2.0) as 1 / q^2: half an ulp twice).
 template <typename R>
 __device__ void FlyerT<R>::EleImpScUpdateK() {
-  const DevTables &T = F.T;
+  const FlightConstT<R> &K = TB::k(F.T);
+  stock(3);
+  const R u0 = Random(), u1 = Random(), u2 = Random();
   R xkl, ykl, zkl;
   in_wedge(xkl, ykl, zkl, kx, ky, kz);
-  xkl = xkl - (R)0.85 * (R)T.a0pi;
-  xkl = xkl * m_sqrt((R)(T.meld / T.mell));
-  ykl = ykl * m_sqrt((R)(T.meld / T.melt));
-  zkl = zkl * m_sqrt((R)(T.meld / T.melt));
-  R betaq;
-  if constexpr (sizeof(R) == 4) betaq = imp_beta;
-  else betaq = T.frickel * 4 * kPiD * Rho / T.eps_si;
-  const R eebeta = betaq / (R)(2.0 * T.meld);
-  const R alfa = eebeta * (R)T.meld / ((R)2.0 * (R)energy * (R)T.melt);
-  R pr = Random() / ((R)1.0 + (R)0.5 * alfa);
+  xkl = xkl - K.shift;
+  xkl = xkl * K.in_l;
+  ykl = ykl * K.in_t;
+  zkl = zkl * K.in_t;
+  const R betaq = imp_beta;
+  const R eebeta = betaq / K.two_meld;
+  const R alfa = eebeta * K.meld / ((R)2.0 * (R)energy * K.melt);
+  R pr = u0 / ((R)1.0 + (R)0.5 * alfa);
   const R costr = (R)1.0 - alfa * pr / ((R)1.0 - pr);
   const R sintr = m_sqrt((R)1.0 - costr * costr);
-  pr = (R)(2.0 * kPiD) * Random();
+  pr = (R)(2.0 * kPiD) * u1;
   R cospr, sinpr;
   m_sincos(pr, &sinpr, &cospr);
   const R ca = m_sqrt(xkl * xkl + ykl * ykl);
@@ -256,22 +365,14 @@ __device__ void FlyerT<R>::EleImpScUpdateK() {
   const R yklll = sinphi * costheta * xkll + cosphi * ykll + sinphi * sintheta * zkll;
   const R zklll = -sintheta * xkll + costheta * zkll;
   const R dx = xkl - xklll, dy = ykl - yklll, dz = zkl - zklll;
-  const R ml = (R)(T.mell / T.meld), mt = (R)(T.melt / T.meld);
-  const R q = betaq + ml * dx * dx + mt * (dy * dy + dz * dz);
-  const R qmax = betaq + mt * dx * dx + mt * (dy * dy + dz * dz);
-  R dn, dnmax;
-  if constexpr (sizeof(R) == 4) {
-    dn = (R)1 / (q * q);
-    dnmax = (R)1 / (qmax * qmax);
-  } else {
-    dn = pow(q, -2.0);
-    dnmax = pow(qmax, -2.0);
-  }
-  if (dn > Random() * dnmax) {
-    xkl = xklll * m_sqrt((R)(T.mell / T.meld));
-    ykl = yklll * m_sqrt((R)(T.melt / T.meld));
-    zkl = zklll * m_sqrt((R)(T.melt / T.meld));
-    xkl = xkl + (R)0.85 * (R)T.a0pi;
+  const R q = betaq + K.ml * dx * dx + K.mt * (dy * dy + dz * dz);
+  const R qmax = betaq + K.mt * dx * dx + K.mt * (dy * dy + dz * dz);
+  const R dn = (R)1 / (q * q), dnmax = (R)1 / (qmax * qmax);
+  if (dn > u2 * dnmax) {
+    xkl = xklll * K.out_l;
+    ykl = yklll * K.out_t;
+    zkl = zklll * K.out_t;
+    xkl = xkl + K.shift;
     out_wedge(kx, ky, kz, xkl, ykl, zkl);
     CONFBZ(kx, ky, kz);
     loc_mode = kLocImpurity;  // Getisym + GetEnergy in run_locate
@@ -279,6 +380,79 @@ __device__ void FlyerT<R>::EleImpScUpdateK() {
   } else {
     self = true;
   }
+}
+
+template <typename R>
+__device__ __forceinline__ bool FlyerT<R>::no_event() const {
+  // The margins: the products below are rounded once or twice, the quotients
+  // advance() compares once; the clocks' logarithm is the fast one (absolute
+  // error below 2^-21 near 1, a few ulp elsewhere) and the impurity majorant
+  // and rates are in float, all well inside 2^-16 and 2^-18.
+  const R T = (R)left_time;
+  const R Ts = T * (R)(sizeof(R) == 4 ? 1.0 + 0x1p-18 : 1.0 + 0x1p-40);
+  R xkl, ykl, zkl, xfl, yfl, zfl;
+  in_wedge(xkl, ykl, zkl, kx, ky, kz);
+  in_wedge(xfl, yfl, zfl, Ex, Ey, Ez);
+  const TetFlightT<R> &t = tf(itet);
+  bool stays = true;
+#pragma unroll
+  for (int f = 0; f < 4; ++f) {  // TetTime
+    const R nf = t.n[f][0] * xfl + t.n[f][1] * yfl + t.n[f][2] * zfl;
+    const R num = t.n[f][3] - (t.n[f][0] * xkl + t.n[f][1] * ykl + t.n[f][2] * zkl);
+    stays = stays && (!(nf < 0) || num < nf * Ts);
+  }
+  const DevMesh &M = I->M;
+  auto axis = [&](R v, R up, R down) { return (v > 0 ? up : down) > m_abs(v) * Ts; };  // CellTime
+  if constexpr (Real::kCellRelative) {
+    stays = stays && axis(vx, M.dxf[ic] - x, x) && axis(vy, M.dyf[jc] - y, y) && axis(vz, M.dzf[kc] - z, z);
+  } else {
+    stays = stays && axis(vx, M.lx[ic + 1] - x, x - M.lx[ic]) && axis(vy, M.ly[jc + 1] - y, y - M.ly[jc]) &&
+            axis(vz, M.lz[kc + 1] - z, z - M.lz[kc]);
+  }
+  if (!stays) return false;
+  // the clocks: draws 0, 1 (, 2) as advance() takes them in its first pass
+  const float tf32 = (float)T;
+  uint32_t w[4];
+  philox_rounds(0u, uid, step_, sub, (uint32_t)I->seed, (uint32_t)(I->seed >> 32), w);
+  auto clock = [](float u) { return -__logf(u) * (1.0f - 0x1p-16f) - 0x1p-18f; };
+  float u0, u1;
+  if constexpr (sizeof(R) == 4) {
+    u0 = mcb200_bits_to_unit_f32(w[0]);
+    u1 = mcb200_bits_to_unit_f32(w[1]);
+  } else {
+    u0 = (float)mcb200_bits_to_unit(w[1], w[0]);
+    u1 = (float)mcb200_bits_to_unit(w[3], w[2]);
+  }
+  if (!(clock(u0) > (float)t.gam * tf32)) return false;
+  const bool impurities = iband == F.T.bandof[0];
+  const int c = cell_index();
+  if (impurities) {  // GetImpScGamma
+    float rate = 0.0f;
+    if constexpr (sizeof(R) == 4) {
+      const float e = imp_emax < t.e0 ? t.e0 : (imp_emax > t.e3 ? t.e3 : imp_emax);
+      if (e < imp_ecut) rate = __fdividef(imp_a * sqrtf(e), 1.0f + imp_b * e);
+    } else {
+      const float e = fminf(fmaxf((float)imp_emax, (float)t.e0), (float)t.e3);
+      if (e * (float)F.T.eV0 < 0.120f * (1.0f + 0x1p-16f))
+        rate = __fdividef((float)imp_a * sqrtf(2.0f * F.T.k32.meld * e),
+                          (float)imp_c * (1.0f + __fdividef(4.0f * e * F.T.k32.melt, (float)imp_b)));
+    }
+    if (!(clock(u1) > fmaxf(rate, (float)TB::k(F.T).gamma_floor) * tf32)) return false;
+  }
+  if (M.surface_scatter && M.in_surf[c]) {
+    float u = impurities ? 0.0f : u1;
+    if (impurities) {
+      if constexpr (sizeof(R) == 4) {
+        u = mcb200_bits_to_unit_f32(w[2]);
+      } else {
+        philox_rounds(1u, uid, step_, sub, (uint32_t)I->seed, (uint32_t)(I->seed >> 32), w);
+        u = (float)mcb200_bits_to_unit(w[1], w[0]);
+      }
+    }
+    const float rate = type == 0 ? (float)M.e_rough[c] + (float)M.e_sphon[c] : (float)M.h_rough[c] + (float)M.h_sphon[c];
+    if (!(clock(u) > rate * tf32)) return false;
+  }
+  return true;
 }
 
 }  // namespace mcb200
