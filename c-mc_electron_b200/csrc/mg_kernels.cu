@@ -130,12 +130,16 @@ __device__ __forceinline__ double apply27_part(const MgDevLevel &L, const double
 #pragma unroll
   for (int t = 0; t < (9 + G - 1) / G; ++t) {
     const int row = g + t * G;
-    if (row < 9) {
-      const int i2 = min(max(i + row / 3 - 1, 0), L.px - 1), j2 = min(max(j + row % 3 - 1, 0), L.py - 1);
-      const int base = (j2 * L.px + i2) * L.pz + k;
-      acc += a[row * 3] * x[base + km];
-      acc += a[row * 3 + 1] * x[base];
-      acc += a[row * 3 + 2] * x[base + kp];
+    // (a lane past the ninth row loads the last one's and adds nothing)
+    const int rc = 9 % G == 0 ? row : min(row, 8);
+    const int i2 = min(max(i + rc / 3 - 1, 0), L.px - 1), j2 = min(max(j + rc % 3 - 1, 0), L.py - 1);
+    const int base = (j2 * L.px + i2) * L.pz + k;
+    const double c0 = a[rc * 3], c1 = a[rc * 3 + 1], c2 = a[rc * 3 + 2];
+    const double x0 = x[base + km], x1 = x[base], x2 = x[base + kp];
+    if (rc == row) {
+      acc += c0 * x0;
+      acc += c1 * x1;
+      acc += c2 * x2;
     }
   }
   return acc;
@@ -168,11 +172,14 @@ struct Solve {
     const int g = tid % G;
     double acc = 0.0;
     for (int n = tid / G; n < L.n; n += stride / G) {
+      // (every lane of the group loads these: after the sum they would wait
+      // for it)
+      const double bn = b[n], dn = L.dinv[n], xn0 = xc[n];
+      const bool fixed = L.dir[n] != 0;
       const double ax = l == 0 ? apply7(st7, g0, xc, n) : group_sum<G>(apply27_part<G>(L, xc, n, g));
       if (g != 0) continue;
-      const double bn = b[n], dn = L.dinv[n], xn0 = xc[n];
       double v = xn0 + L.omega * dn * (bn - ax);
-      if (L.dir[n]) v = l == 0 ? dn * bn : 0.0;
+      if (fixed) v = l == 0 ? dn * bn : 0.0;
       xn[n] = v;
       if (dot) acc += bn * v;
     }
@@ -193,10 +200,11 @@ struct Solve {
     const double *x = X(l);
     const int g = tid % G;
     for (int n = tid / G; n < L.n; n += stride / G) {
+      const double bn = (l == 0 ? b0 : L.b)[n];
+      const bool fixed = L.dir[n] != 0;
       const double ax = l == 0 ? apply7(st7, g0, x, n) : group_sum<G>(apply27_part<G>(L, x, n, g));
       if (g != 0) continue;
-      const double v = (l == 0 ? b0 : L.b)[n] - ax;
-      L.r[n] = L.dir[n] ? 0.0 : v;
+      L.r[n] = fixed ? 0.0 : bn - ax;
     }
   }
   __device__ void residual(int l) const {
@@ -221,6 +229,8 @@ struct Solve {
       int ci, cj, ck;
       node_ijk(c, gc, ci, cj, ck);
       const int fi = F.keep[0][ci], fj = F.keep[1][cj], fk = F.keep[2][ck];
+      const bool fixed = C.dir[c] != 0;
+      const double dn = smooth ? C.dinv[c] : 0.0;
       double wz[3];
       int kz[3];
 #pragma unroll
@@ -243,9 +253,9 @@ struct Solve {
       }
       acc = group_sum<G>(acc);
       if (g != 0) continue;
-      if (C.dir[c]) acc = 0.0;
+      if (fixed) acc = 0.0;
       C.b[c] = acc;
-      if (smooth) first(l + 1, c, acc);
+      if (smooth) X(l + 1)[c] = fixed ? 0.0 : C.omega * dn * acc;  // first(l + 1)
     }
   }
   __device__ void restrict_to(int l) const {
@@ -255,39 +265,31 @@ struct Solve {
     else if (G == 2) restrict_level<2>(l);
     else restrict_level<1>(l);
   }
-  // x_l += P x_{l+1} on the free rows.
+  // x_l += P x_{l+1} on the free rows.  The eight loads are unconditional
+  // (an axis that keeps its node has weight 0 and some coarse index for the
+  // second): behind tests of the weights they waited for one another, 8 L2
+  // round trips in a row (FinFET level 1 to 3: 3.5 -> 2.4 us a pass, of
+  // which the grid barrier takes 1.2).
   __device__ void prolong(int l) const {
     const MgDevLevel &F = mg.L[l], &C = mg.L[l + 1];
     const double *xc = X(l + 1);
     double *x = X(l);
     const Grid3 gf{F.px, F.py, F.pz};
     for (int n = tid; n < F.n; n += stride) {
-      if (F.dir[n]) continue;
       int i, j, k;
       node_ijk(n, gf, i, j, k);
       const int2 cx = F.cmap[0][i], cy = F.cmap[1][j], cz = F.cmap[2][k];
       const double2 wx = F.wmap[0][i], wy = F.wmap[1][j], wz = F.wmap[2][k];
+      const bool fixed = F.dir[n] != 0;
+      const double xn = x[n];
+      double v[8];
+#pragma unroll
+      for (int t = 0; t < 8; ++t)
+        v[t] = xc[((t & 4 ? cy.y : cy.x) * C.px + (t & 2 ? cx.y : cx.x)) * C.pz + (t & 1 ? cz.y : cz.x)];
       double acc = 0.0;
 #pragma unroll
-      for (int b = 0; b < 2; ++b) {
-        const double wb = b ? wy.y : wy.x;
-        if (wb == 0.0) continue;
-        const int cj = b ? cy.y : cy.x;
-#pragma unroll
-        for (int a = 0; a < 2; ++a) {
-          const double wa = a ? wx.y : wx.x;
-          if (wa == 0.0) continue;
-          const int ci = a ? cx.y : cx.x;
-#pragma unroll
-          for (int d = 0; d < 2; ++d) {
-            const double wd = d ? wz.y : wz.x;
-            if (wd == 0.0) continue;
-            const int ck = d ? cz.y : cz.x;
-            acc += wa * wb * wd * xc[(cj * C.px + ci) * C.pz + ck];
-          }
-        }
-      }
-      x[n] += acc;
+      for (int t = 0; t < 8; ++t) acc += (t & 2 ? wx.y : wx.x) * (t & 4 ? wy.y : wy.x) * (t & 1 ? wz.y : wz.x) * v[t];
+      if (!fixed) x[n] = xn + acc;
     }
   }
   // x = C^-1 b on the coarsest level, one warp per row; returns sum b.x of
@@ -498,26 +500,31 @@ __device__ __forceinline__ void cg_mg_body(const MgGroup<K> &G) {
     if (work) {
       const int first = it[me] == 0;
       for (int n = S.tid; n < nodes; n += S.stride) {
-        if (dirichlet[n]) {
+        // z and p vanish on Dirichlet nodes, so neighbours need no mask; an
+        // off-grid neighbour has a zero coefficient and is clamped (apply7)
+        int i, j, k;
+        node_ijk(n, g, i, j, k);
+        const CoefRow a{st7 + n, nodes};
+        const int sx = g.pz, sy = g.px * g.pz;
+        const bool fixed = dirichlet[n] != 0;
+        // (pin is not read in the first iteration: it holds no p yet)
+        auto P = [&](int m) { return first ? z[m] : z[m] + beta * pin[m]; };
+        const double pn = P(n), p0 = P(i > 0 ? n - sx : n), p1 = P(i + 1 < g.px ? n + sx : n);
+        const double p2 = P(j > 0 ? n - sy : n), p3 = P(j + 1 < g.py ? n + sy : n);
+        const double p4 = P(k > 0 ? n - 1 : n), p5 = P(k + 1 < g.pz ? n + 1 : n);
+        double acc = a[6] * pn;
+        acc += a[0] * p0;
+        acc += a[1] * p1;
+        acc += a[2] * p2;
+        acc += a[3] * p3;
+        acc += a[4] * p4;
+        acc += a[5] * p5;
+        if (fixed) {
           q[n] = 0.0;
           pout[n] = 0.0;
           continue;
         }
-        // z and p vanish on Dirichlet nodes, so neighbours need no mask
-        int i, j, k;
-        node_ijk(n, g, i, j, k);
-        const CoefRow a{st7 + n, nodes};
-        // (pin is not read in the first iteration: it holds no p yet)
-        auto P = [&](int m) { return first ? z[m] : z[m] + beta * pin[m]; };
-        const double pn = P(n);
         pout[n] = pn;
-        double acc = a[6] * pn;
-        if (i > 0) acc += a[0] * P(n - g.pz);
-        if (i + 1 < g.px) acc += a[1] * P(n + g.pz);
-        if (j > 0) acc += a[2] * P(n - g.px * g.pz);
-        if (j + 1 < g.py) acc += a[3] * P(n + g.px * g.pz);
-        if (k > 0) acc += a[4] * P(n - 1);
-        if (k + 1 < g.pz) acc += a[5] * P(n + 1);
         q[n] = acc;
         v += pn * acc;
       }
@@ -533,32 +540,37 @@ __device__ __forceinline__ void cg_mg_body(const MgGroup<K> &G) {
       double *rout = rin == r ? Y.r1 : r;
       double *x0 = S.X(0);
       // first-sweep value of node m from its updated residual, as first(0)
-      auto first0 = [&](int m) { return dirichlet[m] ? 0.0 : L0.fscale[m] * (rin[m] - alpha * q[m]); };
+      // (a Dirichlet row's factor is zero)
+      auto first0 = [&](int m) { return L0.fscale[m] * (rin[m] - alpha * q[m]); };
       const int sx = g.pz, sy = g.px * g.pz;
       for (int n = S.tid; n < nodes; n += S.stride) {
-        double rn = rin[n];
-        if (!dirichlet[n]) {
-          x[n] += alpha * pout[n];
-          rn = rin[n] - alpha * q[n];
-          a2 += rn * rn;
-        }
-        rout[n] = rn;
-        const double f = dirichlet[n] ? 0.0 : L0.fscale[n] * rn;
-        x0[n] = f;
+        const double ri = rin[n], qn = q[n], pn = pout[n], xn = x[n], fs = L0.fscale[n];
+        const bool fixed = dirichlet[n] != 0, alone = L0.dir[n] != 0;
         // level 0's residual of the first sweep (apply7's terms and order;
         // an off-grid neighbour has a zero coefficient and is clamped)
         int i, j, k;
         node_ijk(n, g, i, j, k);
         const CoefRow a{st7 + n, nodes};
+        const double f0 = first0(i > 0 ? n - sx : n), f1 = first0(i + 1 < g.px ? n + sx : n);
+        const double f2 = first0(j > 0 ? n - sy : n), f3 = first0(j + 1 < g.py ? n + sy : n);
+        const double f4 = first0(k > 0 ? n - 1 : n), f5 = first0(k + 1 < g.pz ? n + 1 : n);
+        double rn = ri;
+        if (!fixed) {
+          x[n] = xn + alpha * pn;
+          rn = ri - alpha * qn;
+          a2 += rn * rn;
+        }
+        rout[n] = rn;
+        const double f = fixed ? 0.0 : fs * rn;
+        x0[n] = f;
         double acc = a[6] * f;
-        acc += a[0] * first0(i > 0 ? n - sx : n);
-        acc += a[1] * first0(i + 1 < g.px ? n + sx : n);
-        acc += a[2] * first0(j > 0 ? n - sy : n);
-        acc += a[3] * first0(j + 1 < g.py ? n + sy : n);
-        acc += a[4] * first0(k > 0 ? n - 1 : n);
-        acc += a[5] * first0(k + 1 < g.pz ? n + 1 : n);
-        const double v = rn - acc;
-        L0.r[n] = L0.dir[n] ? 0.0 : v;
+        acc += a[0] * f0;
+        acc += a[1] * f1;
+        acc += a[2] * f2;
+        acc += a[3] * f3;
+        acc += a[4] * f4;
+        acc += a[5] * f5;
+        L0.r[n] = alone ? 0.0 : rn - acc;
       }
       S.b0 = rout;
     } else if (work) {
