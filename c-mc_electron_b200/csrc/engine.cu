@@ -1699,11 +1699,21 @@ int mcb200_set_quantum_correction(mcb200_ctx *c, const mcb200_quantum_params *p,
       d.list = h.list.empty() ? nullptr : dupload(h.list, c->mesh_owned);
       d.inside = dupload(h.inside, c->mesh_owned);
       d.eb = dupload(h.eb, c->mesh_owned);
-      d.range = dupload(h.range, c->mesh_owned);
-      d.qcl = dupload(h.qcl, c->mesh_owned);
       std::vector<int2> win(h.lower.size());
       for (size_t i = 0; i < win.size(); ++i) win[i] = make_int2(h.lower[i], h.upper[i]);
       d.window = dupload(win, c->mesh_owned);
+      const double *qcl = dupload(h.qcl, c->mesh_owned);
+      const int count[3] = {d.px, d.py, d.pz};
+      for (int a = 0, at = 0; a < 3; at += count[a], ++a) {
+        for (int i = 0; i < count[a]; ++i) d.width[a] = std::max(d.width[a], h.upper[at + i] - h.lower[at + i] + 1);
+        std::vector<double2> e(h.edge[a].size() / 2);
+        for (size_t i = 0; i < e.size(); ++i) e[i] = make_double2(h.edge[a][2 * i], h.edge[a][2 * i + 1]);
+        double *diff = dalloc<double>((size_t)count[a] * d.width[a] * kBoxKinds, c->mesh_owned);
+        launch_erf_differences(dupload(e, c->mesh_owned), qcl + at, d.window + at, count[a], d.width[a], diff,
+                               c->stream);
+        d.erf_diff[a] = diff;
+      }
+      ck(cudaGetLastError(), "quantum set-up");
       c->qc = d;
       if (!c->qc_pot) c->qc_pot = dalloc<double>((size_t)d.px * d.py * d.pz, c->mesh_owned);
       c->qc_set = true;

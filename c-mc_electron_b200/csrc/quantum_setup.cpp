@@ -85,7 +85,6 @@ QuantumHost quantum_setup(int nx, int ny, int nz, const double *lx, const double
   QuantumHost q;
   q.inside.assign(nodes, 0);
   q.eb.assign(nodes, 0.0);
-  q.range.assign(6 * nodes, 0.0);
   // init_ep_range (src/mcmodel.cpp:2406-2492)
   const double sx = kSqrt2 * p.theta[0], sy = kSqrt2 * p.theta[1], sz = kSqrt2 * p.theta[2];
   for (int j = 0; j < py; ++j)
@@ -93,22 +92,29 @@ QuantumHost quantum_setup(int nx, int ny, int nz, const double *lx, const double
       for (int k = 0; k < pz; ++k) {
         const size_t n = node(i, j, k);
         const unsigned m = mat[n], b = bc[n];
-        q.inside[n] = (m & (kNodeOxide | kNodeSilicon)) ? 1 : 0;
+        if (m & (kNodeOxide | kNodeSilicon)) {
+          const int kx = (b & kNodeUp ? 1 : 0) | (b & kNodeDown ? 2 : 0);
+          const int ky = (b & kNodeLeft ? 1 : 0) | (b & kNodeRight ? 2 : 0);
+          const int kz = (b & kNodeFront ? 1 : 0) | (b & kNodeBack ? 2 : 0);
+          q.inside[n] = (uint8_t)(1 + kx + 4 * ky + 16 * kz);
+        }
         if ((m & kNodeOxide) && !(m & kNodeSilicon)) q.eb[n] = -p.eb;
-        const double x11 = (b & kNodeUp) ? lx[i] - p.ratio[0] * p.theta[0] : lx[i] - 0.5 * dx[i - 1];
-        const double x22 = (b & kNodeDown) ? lx[i] + p.ratio[0] * p.theta[0] : lx[i] + 0.5 * dx[i];
-        const double y11 = (b & kNodeLeft) ? ly[j] - p.ratio[1] * p.theta[1] : ly[j] - 0.5 * dy[j - 1];
-        const double y22 = (b & kNodeRight) ? ly[j] + p.ratio[1] * p.theta[1] : ly[j] + 0.5 * dy[j];
-        const double z11 = (b & kNodeFront) ? lz[k] - p.ratio[2] * p.theta[2] : lz[k] - 0.5 * dz[k - 1];
-        const double z22 = (b & kNodeBack) ? lz[k] + p.ratio[2] * p.theta[2] : lz[k] + 0.5 * dz[k];
-        q.range[0 * nodes + n] = x11 / sx;
-        q.range[1 * nodes + n] = x22 / sx;
-        q.range[2 * nodes + n] = y11 / sy;
-        q.range[3 * nodes + n] = y22 / sy;
-        q.range[4 * nodes + n] = z11 / sz;
-        q.range[5 * nodes + n] = z22 / sz;
         if (m & kNodeQuantum) q.list.push_back((int)n);
       }
+  // the box edges by index and kind (an end of the axis is always outside)
+  auto edges = [](const double *l, const double *d, int n, double w, double scale, std::vector<double> &out) {
+    out.assign((size_t)n * kBoxKinds * 2, 0.0);
+    for (int i = 0; i < n; ++i)
+      for (int kind = 0; kind < kBoxKinds; ++kind) {
+        const double a = (kind & 1) || i == 0 ? l[i] - w : l[i] - 0.5 * d[i - 1];
+        const double b = (kind & 2) || i == n - 1 ? l[i] + w : l[i] + 0.5 * d[i];
+        out[((size_t)i * kBoxKinds + kind) * 2] = a / scale;
+        out[((size_t)i * kBoxKinds + kind) * 2 + 1] = b / scale;
+      }
+  };
+  edges(lx, dx, px, p.ratio[0] * p.theta[0], sx, q.edge[0]);
+  edges(ly, dy, py, p.ratio[1] * p.theta[1], sy, q.edge[1]);
+  edges(lz, dz, pz, p.ratio[2] * p.theta[2], sz, q.edge[2]);
   // init_effective_potential (src/mcmodel.cpp:2584-2630) and the scaled
   // node coordinates (:2483-2492)
   q.qcl.resize(px + py + pz);

@@ -37,9 +37,9 @@ struct QuantumParams {
 // Per-node data of the correction for a px x py x pz node grid (node (i, j, k)
 // at (j * px + i) * pz + k).
 struct QuantumHost {
-  std::vector<uint8_t> inside;   // node of an oxide or silicon cell
+  std::vector<uint8_t> inside;   // 0, or 1 + the box kinds of a node of an oxide or silicon cell (QuantumDevice)
   std::vector<double> eb;        // -Eb on oxide nodes that are not silicon, else 0
-  std::vector<double> range;     // [6][nodes]: x1, x2, y1, y2, z1, z2
+  std::vector<double> edge[3];   // per axis [index][kind][2]: the box edges of a node, scaled
   std::vector<double> qcl;       // [px + py + pz]: node coordinate / (sqrt 2 theta), per axis
   std::vector<int> lower, upper; // [px + py + pz]: window of each node index, per axis
   std::vector<int> list;         // the quantum nodes
@@ -56,13 +56,22 @@ QuantumHost quantum_setup(int nx, int ny, int nz, const double *lx, const double
 struct QuantumDevice {
   int px = 0, py = 0, pz = 0, n_list = 0;
   const int *list = nullptr;
-  const uint8_t *inside = nullptr;
+  const uint8_t *inside = nullptr;  // per node: 0, or 1 + its kind of box on each axis (kBoxKinds), x + 4 y + 16 z
   const double *eb = nullptr;
-  const double *range = nullptr;
-  const double *qcl = nullptr;
   const int2 *window = nullptr;  // (lower, upper) per axis index
+  // The erf differences of the sum, per axis.  A node's box on an axis
+  // depends on its index and on which of its two neighbours are inside
+  // (four kinds), so the difference for target index t, source index
+  // window[t].x + w and kind is erf_diff[axis][((t * width + w) * 4 + kind].
+  const double *erf_diff[3] = {nullptr, nullptr, nullptr};
+  int width[3] = {0, 0, 0};      // the widest window of the axis
 };
+constexpr int kBoxKinds = 4;  // 1: the lower neighbour is outside, 2: the upper one
 
+// erf_diff of one axis from its box edges, edge[index * 4 + kind] = {lower,
+// upper} and the targets' coordinates (all scaled); out: n * width * 4.
+void launch_erf_differences(const double2 *edge, const double *target, const int2 *window, int n, int width,
+                            double *out, cudaStream_t s);
 // out = pot, with the effective potential at every quantum node (computed
 // from pot, not from out).
 void launch_effective_potential(const QuantumDevice &q, const double *pot, double *out, cudaStream_t s);
