@@ -115,12 +115,11 @@ void build_tables(mcb200_batch *b) {
     base.seed = b->cfg[k].seed;
     base.step = b->member_step[k];  // advanced with b->steps after every step
     base.n = c->dev_counts;
-    base.listed = c->tickets + 1 + mcb200_ctx::kGenerations;
     base.capacity = (int)c->capacity;
     for (int par = 0; par < 2; ++par) {
       BatchInstT<R> e = base;
       e.P = store<R>(c, par == 0 ? c->cur : 1 - c->cur);
-      e.list = store<R>(c, par == 0 ? 1 - c->cur : c->cur).uid;  // free until the step's sort
+      e.lists = flight_lists(store<R>(c, par == 0 ? 1 - c->cur : c->cur), c->tickets + kFlightTickets);
       e.C = children<R>(c, 0);
       t[(size_t)par * n + k] = e;
     }
@@ -217,36 +216,44 @@ void batch_transport(mcb200_batch *b, uint64_t early = 0) {
   const int flip = (int)((b->steps_done - b->built_at) & 1);
   const BatchInstT<R> *tab = static_cast<const BatchInstT<R> *>(b->tables);
   const int sms = b->m[0]->sm_count;
-  unsigned int *side_ticket = b->tickets + 1 + mcb200_ctx::kGenerations;
+  unsigned int *side_ticket = b->tickets + kFlightTickets;
+  long long expected = 0;  // the members' counts as the host last knew them
+  for (int k = 0; k < n; ++k)
+    if ((batched >> k) & 1) expected += (long long)b->m[k]->n;
+  const bool apart = draws_apart(sizeof(R) == 4, expected);
+  const BatchPart flight = apart ? BatchPart::kFlightFirst : BatchPart::kFlight;
   if (batched) {
     if (early) {
       ck(cudaMemsetAsync(side_ticket, 0, sizeof(unsigned int), b->side), "memset");
       if (launch_batch_drift<R>(F, tab + (size_t)flip * n, n, early, sms, b->side))
         throw std::runtime_error("batched drift launch failed");
       ck(cudaEventRecord(b->ev_side0, b->side), "event");  // the side counter is reset, the lists are made
-      if (launch_batch_flight<R>(F, tab + (size_t)flip * n, n, early, b->steps, false, side_ticket, 1, sms, b->side,
+      if (launch_batch_flight<R>(F, tab + (size_t)flip * n, n, early, b->steps, flight, side_ticket, 1, sms, b->side,
                                  b->smem_table))
         throw std::runtime_error("batched flight launch failed");
       ck(cudaEventRecord(b->ev_side, b->side), "event");
     }
-    ck(cudaMemsetAsync(b->tickets, 0, sizeof(unsigned int) * (1 + mcb200_ctx::kGenerations), b->stream), "memset");
+    ck(cudaMemsetAsync(b->tickets, 0, sizeof(unsigned int) * kFlightTickets, b->stream), "memset");
     if (launch_batch_drift<R>(F, tab + (size_t)flip * n, n, batched & ~early, sms, b->stream))
       throw std::runtime_error("batched drift launch failed");
-    if (launch_batch_flight<R>(F, tab + (size_t)flip * n, n, batched & ~early, b->steps, false, b->tickets,
+    if (launch_batch_flight<R>(F, tab + (size_t)flip * n, n, batched & ~early, b->steps, flight, b->tickets,
                                b->blocks_per_sm, sms, b->stream, b->smem_table))
       throw std::runtime_error("batched flight launch failed");
     if (early) {  // the helper, then the side launch's end
       ck(cudaStreamWaitEvent(b->stream, b->ev_side0, 0), "wait");
-      if (launch_batch_flight<R>(F, tab + (size_t)flip * n, n, early, b->steps, false, side_ticket, b->blocks_per_sm,
+      if (launch_batch_flight<R>(F, tab + (size_t)flip * n, n, early, b->steps, flight, side_ticket, b->blocks_per_sm,
                                  sms, b->stream, b->smem_table))
         throw std::runtime_error("batched flight launch failed");
       ck(cudaStreamWaitEvent(b->stream, b->ev_side, 0), "wait");
     }
+    if (apart && launch_batch_flight<R>(F, tab + (size_t)flip * n, n, batched, b->steps, BatchPart::kDraws,
+                                        b->tickets + 1, b->blocks_per_sm, sms, b->stream, b->smem_table))
+      throw std::runtime_error("batched flight launch failed");
     for (int g = 0; g < mcb200_ctx::kGenerations; ++g)
-      if (launch_batch_flight<R>(F, tab + (size_t)(2 + g) * n, n, batched, b->steps, true, b->tickets + 1 + g,
+      if (launch_batch_flight<R>(F, tab + (size_t)(2 + g) * n, n, batched, b->steps, BatchPart::kChildren, b->tickets + 2 + g,
                                  b->blocks_per_sm, sms, b->stream, b->smem_table))
         throw std::runtime_error("batched copy flight launch failed");
-    // (a drift pass and its flight count as one)
+    // (a drift pass, its flight and the draws' count as one)
     b->launches += 2 + mcb200_ctx::kGenerations + (early ? 2 : 0);
   }
   ck(cudaEventRecord(b->ev_flight, b->stream), "event");
@@ -464,7 +471,7 @@ int mcb200_batch_create(mcb200_ctx *const *ctxs, const mcb200_batch_member *memb
     const size_t entry = b->precision == MCB200_FLIGHT_FP32 ? sizeof(BatchInstT<float>) : sizeof(BatchInstT<double>);
     ck(cudaMalloc(&b->tables, 6 * (size_t)n * entry), "cudaMalloc");
     ck(cudaMalloc(&b->steps, (size_t)n * sizeof(uint32_t)), "cudaMalloc");
-    ck(cudaMalloc(&b->tickets, (2 + mcb200_ctx::kGenerations) * sizeof(unsigned int)), "cudaMalloc");
+    ck(cudaMalloc(&b->tickets, (kFlightTickets + 1) * sizeof(unsigned int)), "cudaMalloc");
     std::vector<uint32_t> first_steps(n);
     for (int k = 0; k < n; ++k) first_steps[k] = members[k].first_step;
     b->member_step = first_steps;

@@ -180,6 +180,22 @@ struct DevParticlesT {
 using DevParticles = DevParticlesT<double>;
 using DevParticles32 = DevParticlesT<float>;
 
+// A step's flight works in the step's other particle buffer (free until the
+// sort writes it): the list of the particles the drift pass left, the list
+// of those that wait for a final-state draw, and, entry p for particle p,
+// what the store does not hold of the latter's flight (FlyerT::save).
+template <typename R>
+struct FlightListsT {
+  uint32_t *list, *draws;
+  unsigned int *count;          // [2] entries of the two lists, zeroed by the step reset
+  R *phrnl, *imprnl, *ssnl;     // the clocks' remainders
+  R *tet_time, *cell_time;      // times to the faces
+  R *pick_drand;                // the mechanism search's draw
+  double *left_time;
+  uint2 *progress;              // {draws made, events | zero_run << 20}
+  uint32_t *info;               // packed flags
+};
+
 // Bytes of one particle in the store.
 template <typename R>
 constexpr int particle_bytes() { return 6 * (int)sizeof(R) + 2 * 8 + 4 * 4; }

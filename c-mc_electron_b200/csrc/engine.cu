@@ -544,7 +544,7 @@ void init_device_context(mcb200_ctx *c, size_t max_particles) {
   c->append_count = dalloc<unsigned int>(1, c->owned);
   c->bounds = dalloc<unsigned long long>(4, c->owned);
   ck(cudaMemsetAsync(c->bounds, 0, 4 * sizeof(unsigned long long), c->stream), "memset");
-  c->tickets = dalloc<unsigned int>(2 + mcb200_ctx::kGenerations, c->owned);
+  c->tickets = dalloc<unsigned int>(kFlightTickets + 2, c->owned);  // and the flight lists' counts
   c->y.counters = dalloc<unsigned long long>(kCntNumCounters, c->owned);
   c->y.contact = dalloc<long long>(kMaxContacts * 6, c->owned);
   c->total = dalloc<unsigned int>(1, c->owned);
@@ -2054,7 +2054,7 @@ void step_prepare(mcb200_ctx *c) {
                            c->ts->dt, c->ib, grid_for(c, c->capacity, 256), s);
     c->launches += 2;
   }
-  StepCounters z{c->tickets, {}, c->append_count, c->tickets + 1 + mcb200_ctx::kGenerations};
+  StepCounters z{c->tickets, {}, c->append_count, c->tickets + kFlightTickets};
   for (int g = 0; g < mcb200_ctx::kGenerations; ++g) z.count[g] = children<R>(c, g).count;
   z.count[mcb200_ctx::kGenerations] = c->sink_count;
   if constexpr (sizeof(R) == 4)  // the per-cell records the flight reads
@@ -2107,13 +2107,14 @@ void enqueue_flights(mcb200_ctx *c, FlightCtxT<R> F, cudaEvent_t *ev) {
   cudaStream_t s = c->stream;
   F.C = children<R>(c, 0);
   if (ev) ck(cudaEventRecord(ev[1], s), "event");
-  // (the list of the particles with events lies in the other buffer, which
-  // the step's sort writes after the flights)
-  launch_flight(F, store<R>(c, c->cur), DevCount{c->dev_counts, nullptr, (int)c->capacity},
-                store<R>(c, 1 - c->cur).uid, c->tickets + 1 + mcb200_ctx::kGenerations, c->tickets, c->sm_count, s);
+  // (the flight's lists lie in the other buffer, which the step's sort
+  // writes after the flights)
+  c->launches += launch_flight(F, store<R>(c, c->cur),
+                               flight_lists(store<R>(c, 1 - c->cur), c->tickets + kFlightTickets),
+                               DevCount{c->dev_counts, nullptr, (int)c->capacity}, (long long)c->n, c->tickets,
+                               c->sm_count, s);
   ck(cudaGetLastError(), "flight kernel");
   if (ev) ck(cudaEventRecord(ev[2], s), "event");
-  c->launches += 2;
   for (int g = 0; g < mcb200_ctx::kGenerations; ++g) {
     if (g + 1 < mcb200_ctx::kGenerations) {
       F.C = children<R>(c, g + 1);
@@ -2122,7 +2123,7 @@ void enqueue_flights(mcb200_ctx *c, FlightCtxT<R> F, cudaEvent_t *ev) {
       F.C.count = c->sink_count;
       F.C.capacity = 0;
     }
-    launch_child_flight(F, children<R>(c, g), c->child_cap, c->tickets + 1 + g, c->sm_count, s);
+    launch_child_flight(F, children<R>(c, g), c->child_cap, c->tickets + 2 + g, c->sm_count, s);
     ck(cudaGetLastError(), "child flight kernel");
     c->launches += 1;
   }

@@ -97,6 +97,13 @@ void alloc_particles(DevParticlesT<R> &d, size_t cap, std::vector<void *> &owned
   k.commit(owned);
 }
 
+// A step's flight lists in its free particle buffer.
+template <typename R>
+FlightListsT<R> flight_lists(const DevParticlesT<R> &b, unsigned int *count) {
+  return FlightListsT<R>{b.uid, b.meta, count, b.x, b.y, b.z, b.kx, b.ky, b.kz, b.energy,
+                         reinterpret_cast<uint2 *>(b.charge), b.cell};
+}
+
 template <typename R>
 void alloc_children(DevChildrenT<R> &d, int cap, std::vector<void *> &owned) {
   Carve k;

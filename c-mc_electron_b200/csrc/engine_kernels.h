@@ -15,13 +15,19 @@ using FlightCtx = FlightCtxT<double>;
 
 // Flight launches: the drift pass over the store's n particles (device
 // count; n.max sizes the grids), which flies those without an event and
-// lists the others (list: room for n.max indices, *listed zeroed), then the
-// persistent flight of the listed ones.  `ticket` is a zeroed device counter
-// the persistent blocks take indices from; a child generation reads its own
-// count; n_hint bounds the copies a generation holds.
+// lists the others, and the persistent flight of the listed ones; with
+// draws_apart (by `expected`, the host's idea of the count: it changes the
+// launches, not the result) that one leaves the particles that come to a
+// final-state draw, and a third launch flies these.  `lists` has room for
+// n.max particles; returns the kernels launched.  tickets: zeroed device counters the
+// persistent blocks take indices from, one a launch (kFlightTickets: these
+// two, then the child generations); a child generation reads its own count;
+// n_hint bounds the copies a generation holds.
+constexpr int kFlightTickets = 2 + kChildGenerations;
+bool draws_apart(bool fp32, long long particles);
 template <typename R>
-void launch_flight(const FlightCtxT<R> &F, const DevParticlesT<R> &P, DevCount n, uint32_t *list,
-                   unsigned int *listed, unsigned int *ticket, int sm_count, cudaStream_t s);
+int launch_flight(const FlightCtxT<R> &F, const DevParticlesT<R> &P, const FlightListsT<R> &lists, DevCount n,
+                  long long expected, unsigned int *tickets, int sm_count, cudaStream_t s);
 template <typename R>
 void launch_child_flight(const FlightCtxT<R> &F, const DevChildrenT<R> &in, int n_hint, unsigned int *ticket,
                          int sm_count, cudaStream_t s);
@@ -32,13 +38,16 @@ struct BatchInstT;
 template <typename R>
 int launch_batch_drift(const FlightCtxT<R> &F, const BatchInstT<R> *inst, int ninst, uint64_t members, int sm_count,
                        cudaStream_t s);
-// One persistent launch flying the listed particles (child == false) or the copies
-// of one generation (child == true) of the simulations k < ninst with bit k
+// One persistent launch flying the listed particles, those left to the draws,
+// or the copies of one generation, of the simulations k < ninst with bit k
 // of `members` set (inst: device table of BatchInstT, steps: their step
 // numbers); blocks_per_sm <= 0: as many as fit.  Returns 0 on success.
+// kFlight: the listed particles, draws included; kFlightFirst and kDraws: the
+// same in two launches.
+enum class BatchPart : int { kFlight = 0, kFlightFirst = 1, kDraws = 2, kChildren = 3 };
 template <typename R>
 int launch_batch_flight(const FlightCtxT<R> &F, const BatchInstT<R> *inst, int ninst, uint64_t members,
-                        const uint32_t *steps, bool child, unsigned int *ticket, int blocks_per_sm, int sm_count,
+                        const uint32_t *steps, BatchPart part, unsigned int *ticket, int blocks_per_sm, int sm_count,
                         cudaStream_t s, bool smem_table);
 // steps[k] += 1 and the step field of simulation k in `ntab` consecutive
 // tables of n simulations (the tables the batched flights read in place).
@@ -56,10 +65,10 @@ void launch_append_children(const ChildSetT<R> &set, unsigned int *next_uid, con
 // The counters a step starts from, zeroed in one launch: the flight tickets,
 // the copy count of every generation and of the sink, and the appended count.
 struct StepCounters {
-  unsigned int *tickets;  // [1 + kChildGenerations]
+  unsigned int *tickets;  // [kFlightTickets]
   unsigned int *count[kChildGenerations + 1];
   unsigned int *appended;  // copies appended to the store this step
-  unsigned int *listed;    // particles the drift pass left to the flight
+  unsigned int *listed;    // [2] the flight's list counts (FlightListsT::count)
 };
 // The flight's per-cell records (DevMesh::cell32, [cells][3] float4, or
 // cell64, [cells][3] double2) and the step reset of z, in one launch.

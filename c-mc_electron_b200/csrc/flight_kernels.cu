@@ -16,6 +16,7 @@
 //      counting-sorted by cell into the second particle buffer; the
 //      scatter's last block makes the sorted count the particle count.
 #include <algorithm>
+#include <type_traits>
 
 #include "engine_kernels.h"
 #include "flight_physics.cuh"
@@ -34,11 +35,29 @@ namespace mcb200 {
 #endif
 template <typename R>
 constexpr int kFlightBlocks = sizeof(R) == 4 ? MCB200_FLIGHT_BLOCKS_F32 : MCB200_FLIGHT_BLOCKS_F64;
+// The flight without draws fits FP32 in 80 registers (2M electrons: 610 us at
+// two blocks per SM, 560 at three).
+template <typename R>
+constexpr int kNoDrawBlocks = sizeof(R) == 4 ? 3 : MCB200_FLIGHT_BLOCKS_F64;
 // Threads per block of the flight kernels (a tuning define like the above).
 #ifndef MCB200_FLIGHT_THREADS
 #define MCB200_FLIGHT_THREADS 256
 #endif
 constexpr int kFlightThreads = MCB200_FLIGHT_THREADS;
+
+// The expected particle count from which a step's final-state draws are left
+// to a launch of their own (draws_apart; tuning defines).  Without the draws
+// the flight's loop has two thirds of the code and no register spills (FP64),
+// or fits three blocks per SM (FP32); the second launch costs the latency of
+// a draw and the rest of its particles' steps, 30-40 us.  Measured, one
+// launch against two: FP64 2M electrons 1326 -> 972 us, 100k 196 -> 173, bar of
+// 4800 worse; FP32 2M 756 -> 666, FinFET of 530k 112 -> 118, 76k 73 -> 83.
+#ifndef MCB200_DRAWS_APART_F32
+#define MCB200_DRAWS_APART_F32 1000000
+#endif
+#ifndef MCB200_DRAWS_APART_F64
+#define MCB200_DRAWS_APART_F64 65536
+#endif
 
 constexpr uint32_t kMetaDead = 1u << 16;
 constexpr uint32_t kMetaUnfinished = 1u << 17;
@@ -52,13 +71,15 @@ __device__ void load_sym(SymSmemT<R> &S, const DevTables &T) {
   __syncthreads();
 }
 
-// Loading and storing the flown particles of the main store (StoreIO: the
-// particles drift_kernel listed) and of a child generation (ChildIO).  load
-// takes the q-th particle to fly and returns where store puts it (-1: none).
-template <typename R>
+// Loading and storing the flown particles of the main store (StoreIO: those
+// that drift_kernel listed or, kResume, those a launch without draws left to
+// them) and of a child generation (ChildIO).  load takes the q-th particle
+// to fly, with the state its flight is in, and returns where store puts it
+// (-1: none); defer leaves a particle to the draws.
+template <typename R, bool kResume>
 struct StoreIO {
   DevParticlesT<R> P;
-  const uint32_t *list;  // the particles to fly
+  FlightListsT<R> lists;
   double dt;
   uint32_t step;  // the particles' step number (their random streams)
   // particle p of the store; false: not to be flown
@@ -80,9 +101,22 @@ struct StoreIO {
     f.left_time = dt;
     return true;
   }
-  __device__ int load(int q, FlyerT<R> &f) const {
-    const int p = (int)list[q];
-    return read(p, f) ? p : -1;
+  __device__ int load(int q, FlyerT<R> &f, int &state) const {
+    const int p = (int)(kResume ? lists.draws : lists.list)[q];
+    if (!read(p, f)) return -1;
+    if constexpr (kResume) {
+      f.resume(lists, p);
+      state = FlyerT<R>::kDraw;
+    } else {
+      f.begin();
+      state = FlyerT<R>::kGoOn;
+    }
+    return p;
+  }
+  __device__ void defer(int p, const FlyerT<R> &f) const {
+    f.save(lists, p);
+    store(p, f, 0);
+    lists.draws[atomicAdd(lists.count + 1, 1u)] = (uint32_t)p;
   }
   __device__ void store(int p, const FlyerT<R> &f, int r) const {
     P.x[p] = f.x; P.y[p] = f.y; P.z[p] = f.z;
@@ -100,7 +134,7 @@ template <typename R>
 struct ChildIO {
   DevChildrenT<R> C;
   uint32_t step;
-  __device__ int load(int p, FlyerT<R> &f) const {
+  __device__ int load(int p, FlyerT<R> &f, int &state) const {
     f.step_ = step;
     f.x = C.x[p]; f.y = C.y[p]; f.z = C.z[p];
     f.kx = C.kx[p]; f.ky = C.ky[p]; f.kz = C.kz[p];
@@ -114,6 +148,8 @@ struct ChildIO {
     f.start_stream(C.parent_uid[p], C.sub[p]);
     f.nchild = 0;
     f.left_time = C.left_time[p];
+    f.begin();
+    state = FlyerT<R>::kGoOn;
     return p;
   }
   __device__ void store(int p, const FlyerT<R> &f, int r) const {
@@ -156,7 +192,7 @@ struct ChildIO {
 #ifndef MCB200_FLIGHT_CHUNK
 #define MCB200_FLIGHT_CHUNK 64
 #endif
-template <typename R, bool kLaneEvents, class IO>
+template <typename R, bool kLaneEvents, bool kDraws, class IO>
 __device__ __forceinline__ void fly_interleaved(const FlightCtxT<R> &F, const SymSmemT<R> &S, const IO &io, int n,
                                                 unsigned int *ticket) {
   static_assert(kFlightThreads == FlyerT<R>::kRingStride, "one ring column a thread");
@@ -186,13 +222,17 @@ __device__ __forceinline__ void fly_interleaved(const FlightCtxT<R> &F, const Sy
     atomicAdd(&F.Y.counters[kCntImpurity], (unsigned long long)f.n_imp);
     events = f.n_ph = f.n_imp = 0;
   };
-  auto done = [&]() {
-    const int r = f.template finish<!kLaneEvents>();
+  auto count_events = [&]() {
     if constexpr (kLaneEvents) {
-      events += (uint32_t)f.loop;
+      events += (uint32_t)(f.loop - f.counted);
       if (events >= 0x80000000u) flush();
+    } else {
+      f.count_events();
     }
-    return r;
+  };
+  auto done = [&]() {
+    count_events();
+    return f.finish();
   };
   for (;;) {
     if (!exhausted) {
@@ -218,13 +258,10 @@ __device__ __forceinline__ void fly_interleaved(const FlightCtxT<R> &F, const Sy
           next += give;
         }
         if (q >= 0) {
-          p = io.load(q, f);
-          if (p >= 0) {
-            f.begin();
-            if (!(f.left_time > 0)) {
-              io.store(p, f, done());
-              p = -1;
-            }
+          p = io.load(q, f, state);
+          if (p >= 0 && !(f.left_time > 0)) {
+            io.store(p, f, done());
+            p = -1;
           }
         }
       }
@@ -234,9 +271,15 @@ __device__ __forceinline__ void fly_interleaved(const FlightCtxT<R> &F, const Sy
       if (exhausted) break;
       continue;
     }
-    if (p >= 0) state = f.advance();
-    const unsigned draws = __ballot_sync(0xffffffffu, p >= 0 && state == FlyerT<R>::kDraw);
-    if (draws) f.final_states(draws);
+    if (p >= 0 && state == FlyerT<R>::kGoOn) state = f.advance();
+    if constexpr (kDraws) {
+      const unsigned draws = __ballot_sync(0xffffffffu, p >= 0 && state == FlyerT<R>::kDraw);
+      if (draws) f.final_states(draws);
+    } else if (p >= 0 && state == FlyerT<R>::kDraw) {
+      io.defer(p, f);
+      count_events();
+      p = -1;
+    }
     if (p >= 0 && state >= FlyerT<R>::kPending) {
       if (state == FlyerT<R>::kPending) f.run_pending();
       state = f.settle() ? FlyerT<R>::kStepOver : FlyerT<R>::kGoOn;
@@ -326,7 +369,7 @@ __global__ void __launch_bounds__(kFlightThreads) drift_kernel(const __grid_cons
   pdl_wait();
   const int count = n.get();
   const uint32_t step = F.step_dev ? *F.step_dev : F.step;
-  const StoreIO<R> io{P, nullptr, F.dt, step};
+  const StoreIO<R, false> io{P, FlightListsT<R>{}, F.dt, step};
   unsigned int done = 0;
   for (int base = blockIdx.x * kFlightThreads; base < count; base += gridDim.x * kFlightThreads) {
     const int p = base + (int)threadIdx.x;
@@ -340,17 +383,17 @@ __global__ void __launch_bounds__(kFlightThreads) drift_kernel(const __grid_cons
   if ((threadIdx.x & 31u) == 0 && done) atomicAdd(&F.Y.counters[kCntEvents], (unsigned long long)done);
 }
 
-template <typename R>
-__global__ void __launch_bounds__(kFlightThreads, kFlightBlocks<R>) flight_kernel(FlightCtxT<R> F, DevParticlesT<R> P,
-                                                                       const uint32_t *list, DevCount n,
-                                                                       unsigned int *ticket) {
+template <typename R, bool kDraws, bool kResume>
+__global__ void __launch_bounds__(kFlightThreads, kDraws ? kFlightBlocks<R> : kNoDrawBlocks<R>)
+    flight_kernel(FlightCtxT<R> F, DevParticlesT<R> P, FlightListsT<R> lists, unsigned int *ticket) {
   __shared__ SymSmemT<R> S;
-  load_sym(S, F.T);  // the band tables: nothing the kernel ahead writes
+  if constexpr (!kResume) load_sym(S, F.T);  // the band tables: nothing the kernel ahead writes
   pdl_wait();
-  const int count = n.get();
+  const int count = (int)lists.count[kResume ? 1 : 0];
   if (count == 0) return;
+  if constexpr (kResume) load_sym(S, F.T);
   const uint32_t step = F.step_dev ? *F.step_dev : F.step;
-  fly_interleaved<R, true>(F, S, StoreIO<R>{P, list, F.dt, step}, count, ticket);
+  fly_interleaved<R, true, kDraws>(F, S, StoreIO<R, kResume>{P, lists, F.dt, step}, count, ticket);
 }
 
 // Copies made during the previous pass (buffer `in`) fly the rest of their
@@ -364,7 +407,7 @@ __global__ void __launch_bounds__(kFlightThreads, kFlightBlocks<R>) child_flight
   __shared__ SymSmemT<R> S;
   load_sym(S, F.T);
   const uint32_t step = F.step_dev ? *F.step_dev : F.step;
-  fly_interleaved<R, true>(F, S, ChildIO<R>{in, step}, count, ticket);
+  fly_interleaved<R, true, true>(F, S, ChildIO<R>{in, step}, count, ticket);
 }
 
 // ---- batched flight ------------------------------------------------------
@@ -376,7 +419,7 @@ __global__ void __launch_bounds__(kFlightThreads, kFlightBlocks<R>) child_flight
 // tallies, copy buffer, dt, seed and step (FlyerT::I).  A particle's draws
 // still come from its own stream (seed, uid, step), so it flies exactly as
 // in a launch of its simulation alone.
-template <typename R, bool kChild>
+template <typename R, bool kChild, bool kResume>
 struct BatchIO {
   const BatchInstT<R> *I;  // shared memory
   const int *prefix;       // [ninst + 1], shared memory
@@ -390,18 +433,22 @@ struct BatchIO {
     }
     return lo;
   }
-  __device__ int load(int q, FlyerT<R> &f) const {
+  __device__ int load(int q, FlyerT<R> &f, int &state) const {
     const int k = find(q);
     const BatchInstT<R> &b = I[k];
     f.I = &b;
     const int p = q - prefix[k];
-    if constexpr (kChild) return ChildIO<R>{b.in, b.step}.load(p, f);
-    else return StoreIO<R>{b.P, b.list, b.dt, b.step}.load(p, f);
+    if constexpr (kChild) return ChildIO<R>{b.in, b.step}.load(p, f, state);
+    else return StoreIO<R, kResume>{b.P, b.lists, b.dt, b.step}.load(p, f, state);
+  }
+  __device__ void defer(int p, const FlyerT<R> &f) const {
+    const BatchInstT<R> *b = static_cast<const BatchInstT<R> *>(f.I);
+    StoreIO<R, false>{b->P, b->lists, b->dt, b->step}.defer(p, f);
   }
   __device__ void store(int p, const FlyerT<R> &f, int r) const {
     const BatchInstT<R> *b = static_cast<const BatchInstT<R> *>(f.I);
     if constexpr (kChild) ChildIO<R>{b->in, b->step}.store(p, f, r);
-    else StoreIO<R>{b->P, b->list, b->dt, b->step}.store(p, f, r);
+    else StoreIO<R, kResume>{b->P, b->lists, b->dt, b->step}.store(p, f, r);
   }
 };
 
@@ -420,7 +467,7 @@ constexpr size_t batch_smem_bytes(int ninst, bool table) {
 // per simulation, taken from the SM's L1 share) and takes the step numbers
 // from `steps`; otherwise lanes read the table where it lies (global memory,
 // through L1), whose step fields advance_batch_steps keeps current.
-template <typename R, bool kChild, bool kSmemTable>
+template <typename R, bool kChild, bool kDraws, bool kResume, bool kSmemTable>
 __global__ void __launch_bounds__(kFlightThreads, kFlightBlocks<R>) batch_flight_kernel(const __grid_constant__ FlightCtxT<R> F,
                                                                              const BatchInstT<R> *inst,
                                                                              int ninst, uint64_t members,
@@ -451,14 +498,14 @@ __global__ void __launch_bounds__(kFlightThreads, kFlightBlocks<R>) batch_flight
     for (int k = 0; k < ninst; ++k) {
       prefix[k] = run;
       if ((members >> k) & 1ull)
-        run += kChild ? min((int)*I[k].in.count, I[k].in.capacity) : (int)*I[k].listed;
+        run += kChild ? min((int)*I[k].in.count, I[k].in.capacity) : (int)I[k].lists.count[kResume ? 1 : 0];
     }
     prefix[ninst] = run;
   }
   load_sym(S, F.T);  // ends with a barrier: the table and prefix are visible
   const int total = prefix[ninst];
   if (total == 0) return;
-  fly_interleaved<R, false>(F, S, BatchIO<R, kChild>{I, prefix, ninst}, total, ticket);
+  fly_interleaved<R, false, kDraws>(F, S, BatchIO<R, kChild, kResume>{I, prefix, ninst}, total, ticket);
 }
 
 // The drift pass of many simulations in one launch: the blocks take 256
@@ -494,11 +541,11 @@ __global__ void __launch_bounds__(kFlightThreads) batch_drift_kernel(const __gri
     FlyerT<R> f(F, S, nullptr);
     f.I = &b;
     bool unfinished;
-    const StoreIO<R> io{b.P, nullptr, b.dt, b.step};
+    const StoreIO<R, false> io{b.P, FlightListsT<R>{}, b.dt, b.step};
     const unsigned done = __reduce_add_sync(0xffffffffu, drift_block(F, f, io, p, p < count, unfinished));
     if ((threadIdx.x & 31u) == 0 && done) atomicAdd(&b.Y.counters[kCntEvents], (unsigned long long)done);
-    const unsigned at = place_in_list(unfinished, b.listed);
-    if (unfinished) b.list[at] = (uint32_t)p;
+    const unsigned at = place_in_list(unfinished, b.lists.count);
+    if (unfinished) b.lists.list[at] = (uint32_t)p;
   }
 }
 
@@ -525,14 +572,10 @@ void launch_advance_batch_steps(uint32_t *steps, BatchInstT<R> *tab, int n, int 
 // The step's counters are reset in the same launch (block 0: zeroed work
 // tickets, copy counts and appended count), which the flight then reads.
 __device__ __forceinline__ void reset_step_counters(const StepCounters &z, int t) {
-  if (t < 1 + kChildGenerations) {
-    z.tickets[t] = 0u;
-    *z.count[t] = 0u;
-  }
-  if (t == 0) {
-    *z.appended = 0u;
-    *z.listed = 0u;
-  }
+  if (t < kFlightTickets) z.tickets[t] = 0u;
+  if (t < 1 + kChildGenerations) *z.count[t] = 0u;
+  if (t == 0) *z.appended = 0u;
+  if (t < 2) z.listed[t] = 0u;
 }
 // FP64 flight's records (DevMesh::cell64): the factors of the reference's
 // expressions that hold no particle value, each rounded as there.
@@ -943,7 +986,7 @@ int flight_grid(int n, int block, int sm_count) {
   int &per_sm = per_sm_of[current_device()];
   if (per_sm == 0) {
     int b = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, flight_kernel<R>, block, 0) != cudaSuccess || b < 1) b = 1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, flight_kernel<R, true, false>, block, 0) != cudaSuccess || b < 1) b = 1;
     per_sm = b;
   }
   const long long want = ((long long)n + block / 32 - 1) / (block / 32);
@@ -962,13 +1005,24 @@ int drift_grid(long long tiles, int sm_count) {
   }
   return (int)std::max<long long>(1, std::min<long long>(tiles, (long long)per_sm * sm_count));
 }
+bool draws_apart(bool fp32, long long particles) {
+  return particles >= (fp32 ? MCB200_DRAWS_APART_F32 : MCB200_DRAWS_APART_F64);
+}
 template <typename R>
-void launch_flight(const FlightCtxT<R> &F, const DevParticlesT<R> &P, DevCount n, uint32_t *list,
-                   unsigned int *listed, unsigned int *ticket, int sm_count, cudaStream_t s) {
+int launch_flight(const FlightCtxT<R> &F, const DevParticlesT<R> &P, const FlightListsT<R> &lists, DevCount n,
+                  long long expected, unsigned int *tickets, int sm_count, cudaStream_t s) {
   launch_pdl(drift_kernel<R>, drift_grid<R>(((long long)n.max + kFlightThreads - 1) / kFlightThreads, sm_count),
-             kFlightThreads, 0, s, F, P, n, list, listed);
-  launch_pdl(flight_kernel<R>, flight_grid<R>(n.max, kFlightThreads, sm_count), kFlightThreads, 0, s, F, P,
-             (const uint32_t *)list, DevCount{listed, nullptr, n.max}, ticket);
+             kFlightThreads, 0, s, F, P, n, lists.list, lists.count);
+  const int grid = flight_grid<R>(n.max, kFlightThreads, sm_count);
+  if (!draws_apart(sizeof(R) == 4, expected)) {
+    launch_pdl(flight_kernel<R, true, false>, grid, kFlightThreads, 0, s, F, P, lists, tickets);
+    return 2;
+  }
+  const int first = (int)std::min<long long>(((long long)n.max + kFlightThreads / 32 - 1) / (kFlightThreads / 32),
+                                             (long long)kNoDrawBlocks<R> * sm_count);
+  launch_pdl(flight_kernel<R, false, false>, std::max(first, 1), kFlightThreads, 0, s, F, P, lists, tickets);
+  launch_pdl(flight_kernel<R, true, true>, grid, kFlightThreads, 0, s, F, P, lists, tickets + 1);
+  return 3;
 }
 template <typename R>
 int launch_batch_drift(const FlightCtxT<R> &F, const BatchInstT<R> *inst, int ninst, uint64_t members, int sm_count,
@@ -987,16 +1041,22 @@ void launch_child_flight(const FlightCtxT<R> &F, const DevChildrenT<R> &in, int 
 }
 template <typename R>
 int launch_batch_flight(const FlightCtxT<R> &F, const BatchInstT<R> *inst, int ninst, uint64_t members,
-                        const uint32_t *steps, bool child, unsigned int *ticket, int blocks_per_sm, int sm_count,
+                        const uint32_t *steps, BatchPart part, unsigned int *ticket, int blocks_per_sm, int sm_count,
                         cudaStream_t s, bool smem_table) {
   if (ninst < 1 || ninst > kMaxBatch) return 1;
   const size_t smem = batch_smem_bytes<R>(ninst, smem_table);
-  auto kernel = smem_table ? (child ? batch_flight_kernel<R, true, true> : batch_flight_kernel<R, false, true>)
-                           : (child ? batch_flight_kernel<R, true, false> : batch_flight_kernel<R, false, false>);
+  auto pick = [&](auto table) {
+    constexpr bool T = decltype(table)::value;
+    return part == BatchPart::kFlight        ? batch_flight_kernel<R, false, true, false, T>
+           : part == BatchPart::kFlightFirst ? batch_flight_kernel<R, false, false, false, T>
+           : part == BatchPart::kDraws       ? batch_flight_kernel<R, false, true, true, T>
+                                             : batch_flight_kernel<R, true, true, false, T>;
+  };
+  auto kernel = smem_table ? pick(std::true_type{}) : pick(std::false_type{});
   if (smem_table) {
     // the opt-in to more than 48 KB of dynamic shared memory holds per device
-    static bool opted[kMaxDevices][2] = {};
-    bool &done = opted[current_device()][child ? 1 : 0];
+    static bool opted[kMaxDevices][4] = {};
+    bool &done = opted[current_device()][(int)part];
     if (!done) {
       if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)batch_smem_bytes<R>(kMaxBatch, true)) != cudaSuccess)
@@ -1061,8 +1121,8 @@ void launch_cell_sort(const DevParticlesT<R> &src, DevCount n, const DevParticle
 #define MCB200_INSTANTIATE(R)                                                                                   \
   template void launch_seed<R>(const FlightCtx &, const DevParticlesT<R> &, int, int, const int *,            \
                                const double *, int, uint32_t, int, cudaStream_t);                             \
-  template void launch_flight<R>(const FlightCtxT<R> &, const DevParticlesT<R> &, DevCount, uint32_t *,         \
-                                 unsigned int *, unsigned int *, int, cudaStream_t);                            \
+  template int launch_flight<R>(const FlightCtxT<R> &, const DevParticlesT<R> &, const FlightListsT<R> &,        \
+                                DevCount, long long, unsigned int *, int, cudaStream_t);                        \
   template int launch_batch_drift<R>(const FlightCtxT<R> &, const BatchInstT<R> *, int, uint64_t, int,          \
                                      cudaStream_t);                                                             \
   template void launch_child_flight<R>(const FlightCtxT<R> &, const DevChildrenT<R> &, int, unsigned int *, int, \
@@ -1071,7 +1131,7 @@ void launch_cell_sort(const DevParticlesT<R> &src, DevCount n, const DevParticle
                                           const unsigned int *, int, unsigned int *, unsigned int *, int,       \
                                           cudaStream_t);                                                        \
   template int launch_batch_flight<R>(const FlightCtxT<R> &, const BatchInstT<R> *, int, uint64_t,             \
-                                      const uint32_t *, bool, unsigned int *, int, int, cudaStream_t, bool);    \
+                                      const uint32_t *, BatchPart, unsigned int *, int, int, cudaStream_t, bool); \
   template void launch_advance_batch_steps<R>(uint32_t *, BatchInstT<R> *, int, int, cudaStream_t);           \
   template void launch_cell_sort<R>(const DevParticlesT<R> &, DevCount, const DevParticlesT<R> &, int, int, int, \
                                     unsigned int *, unsigned int *, unsigned int *, unsigned int *, int,        \

@@ -40,7 +40,7 @@ namespace mcb200 {
 
 constexpr double kMyZero = 1e-13;          // MY_ZERO, include/defs.h
 constexpr double kPiD = 3.141592653589793238462643e0;
-constexpr int kMaxEvents = 1000000;
+constexpr int kMaxEvents = 1000000;  // fits in 20 bits (FlyerT::save)
 constexpr int kMaxStateTries = 10000;
 // FP32 flight: consecutive zero-length events after which a particle is
 // taken as stuck (counted in kCntZeroTime and caught).
@@ -186,8 +186,7 @@ struct BatchInstT : FlightInstT<R> {
   DevParticlesT<R> P;
   DevChildrenT<R> in;
   const unsigned int *n;
-  uint32_t *list;        // the particles the drift pass leaves to the flight, and their count
-  unsigned int *listed;
+  FlightListsT<R> lists;
   int capacity;
   int pad_;
 };
@@ -1121,6 +1120,7 @@ struct FlyerT {
   bool get_tet, get_cell, get_ph, get_imp, get_surf, too_far;
   R ssnl, imprnl, phrnl, TetTf, CellTf;
   int loop, zero_run;
+  int counted;  // of `loop`, the events already added to the counters
 
   __device__ void begin() {
     catch_ = false;
@@ -1135,7 +1135,7 @@ struct FlyerT {
     load_cell_fields();
     iband = tf(itet).band;
     GetV();
-    loop = 0;
+    loop = counted = 0;
     surf_gamma = 0;
     imp_gamma = 0;
   }
@@ -1159,6 +1159,54 @@ struct FlyerT {
     y += vy * T;
     z += vz * T;
     return true;
+  }
+
+  // The flight's state while it waits for a final-state draw.
+  __device__ __forceinline__ void save(const FlightListsT<R> &m, int p) const {
+    m.phrnl[p] = phrnl;
+    m.imprnl[p] = imprnl;
+    m.ssnl[p] = ssnl;
+    m.tet_time[p] = TetTf;
+    m.cell_time[p] = CellTf;
+    m.pick_drand[p] = pick_drand;
+    m.left_time[p] = left_time;
+    m.progress[p] = make_uint2(n, (uint32_t)loop | (uint32_t)zero_run << 20);
+    m.info[p] = (get_tet ? 1u : 0u) | (get_ph ? 2u : 0u) | (get_imp ? 4u : 0u) | (get_surf ? 8u : 0u) |
+                (self ? 16u : 0u) | (imp_pending ? 32u : 0u) | (uint32_t)loc_mode << 6 | (uint32_t)draw_kind << 8 |
+                (uint32_t)idir << 10 | (uint32_t)itetdir << 13 | (uint32_t)ev << 15 |
+                (uint32_t)nchild << 20;
+  }
+  // After the store's part is loaded.
+  __device__ __forceinline__ void resume(const FlightListsT<R> &m, int p) {
+    phrnl = m.phrnl[p];
+    imprnl = m.imprnl[p];
+    ssnl = m.ssnl[p];
+    TetTf = m.tet_time[p];
+    CellTf = m.cell_time[p];
+    pick_drand = m.pick_drand[p];
+    left_time = m.left_time[p];
+    const uint2 c = m.progress[p];
+    n = c.x;
+    stocked = n & ~(kBlockDraws - 1u);
+    loop = counted = (int)(c.y & 0xfffffu);
+    zero_run = (int)(c.y >> 20);
+    const uint32_t w = m.info[p];
+    get_tet = get_cell = w & 1u;
+    get_ph = w & 2u;
+    get_imp = w & 4u;
+    get_surf = w & 8u;
+    self = w & 16u;
+    imp_pending = w & 32u;
+    loc_mode = (int)(w >> 6 & 3u);
+    draw_kind = (int)(w >> 8 & 3u);
+    idir = (int)(w >> 10 & 7u);
+    itetdir = (int)(w >> 13 & 3u);
+    ev = (int)(w >> 15 & 7u);
+    nchild = (int)(w >> 20);
+    catch_ = too_far = false;
+    surf_gamma = imp_gamma = 0;
+    load_cell_fields();
+    iband = tf(itet).band;
   }
 
   // What is left after an advance().
@@ -1348,17 +1396,16 @@ struct FlyerT {
     return !(left_time > 0);
   }
 
-  // Returns 0 done, 1 caught, 2 unfinished (outer-boundary PASS).  A
-  // caller that sums the particles' events itself (`loop`, n_ph, n_imp: one
-  // simulation per launch) passes kCountEvents = false.
-  template <bool kCountEvents = true>
+  // The particle's events into the simulation's counters (a caller that sums
+  // them itself, one simulation per launch, does not call it).
+  __device__ void count_events() {
+    atomicAdd(&I->Y.counters[kCntEvents], (unsigned long long)(loop - counted));
+    if (n_ph) atomicAdd(&I->Y.counters[kCntPhonon], (unsigned long long)n_ph);
+    if (n_imp) atomicAdd(&I->Y.counters[kCntImpurity], (unsigned long long)n_imp);
+    n_ph = n_imp = 0;
+  }
+  // Returns 0 done, 1 caught, 2 unfinished (outer-boundary PASS).
   __device__ int finish() {
-    if constexpr (kCountEvents) {
-      atomicAdd(&I->Y.counters[kCntEvents], (unsigned long long)loop);
-      if (n_ph) atomicAdd(&I->Y.counters[kCntPhonon], (unsigned long long)n_ph);
-      if (n_imp) atomicAdd(&I->Y.counters[kCntImpurity], (unsigned long long)n_imp);
-      n_ph = n_imp = 0;
-    }
     if (catch_) {
       count(I->Y, kCntCaught);
       return 1;
