@@ -45,6 +45,17 @@ constexpr int kNoDrawBlocks = sizeof(R) == 4 ? 3 : MCB200_FLIGHT_BLOCKS_F64;
 #endif
 constexpr int kFlightThreads = MCB200_FLIGHT_THREADS;
 
+// Resident blocks per SM of the drift pass (measured best: FP32 of 4 to 6, 80 us
+// for 2M electrons; FP64 of 2 to 4, 155 us).
+#ifndef MCB200_DRIFT_BLOCKS_F32
+#define MCB200_DRIFT_BLOCKS_F32 4
+#endif
+#ifndef MCB200_DRIFT_BLOCKS_F64
+#define MCB200_DRIFT_BLOCKS_F64 3
+#endif
+template <typename R>
+constexpr int kDriftBlocks = sizeof(R) == 4 ? MCB200_DRIFT_BLOCKS_F32 : MCB200_DRIFT_BLOCKS_F64;
+
 // The expected particle count from which a step's final-state draws are left
 // to a launch of their own (draws_apart; tuning defines).  Without the draws
 // the flight's loop has two thirds of the code and no register spills (FP64),
@@ -360,7 +371,7 @@ __device__ __forceinline__ unsigned place_in_list(bool mine, unsigned int *count
 }
 
 template <typename R>
-__global__ void __launch_bounds__(kFlightThreads) drift_kernel(const __grid_constant__ FlightCtxT<R> F,
+__global__ void __launch_bounds__(kFlightThreads, kDriftBlocks<R>) drift_kernel(const __grid_constant__ FlightCtxT<R> F,
                                                                const __grid_constant__ DevParticlesT<R> P, DevCount n,
                                                                uint32_t *list, unsigned int *listed) {
   __shared__ SymSmemT<R> S;  // its operations only
@@ -511,7 +522,7 @@ __global__ void __launch_bounds__(kFlightThreads, kFlightBlocks<R>) batch_flight
 // The drift pass of many simulations in one launch: the blocks take 256
 // particles of one simulation at a time.
 template <typename R>
-__global__ void __launch_bounds__(kFlightThreads) batch_drift_kernel(const __grid_constant__ FlightCtxT<R> F,
+__global__ void __launch_bounds__(kFlightThreads, kDriftBlocks<R>) batch_drift_kernel(const __grid_constant__ FlightCtxT<R> F,
                                                                      const BatchInstT<R> *inst, int ninst,
                                                                      uint64_t members) {
   __shared__ SymSmemT<R> S;

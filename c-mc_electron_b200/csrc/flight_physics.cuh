@@ -794,23 +794,28 @@ struct FlyerT {
     const int rows = phon == 0 ? 201 : 51;
     const double *tab = T.disp + T.disp_off[which] + (ei - 1);
     const double ran = (double)draw();
-    int i = 0;
+    // The walk down the column, by the whole warp (its lanes all call this
+    // with the same arguments): 32 rows are loaded at once and added in
+    // order.  FEKLOEM wraps before the last row is added, the others after.
+    const int lane = (int)(threadIdx.x & 31u);
+    const int last_row = which == 0 ? rows - 1 : rows;
+    int i = 1;
     double ksum = 0.0;
-    if (which == 0) {  // FEKLOEM wraps before adding: rows 0..199
+    bool open = true;
 #pragma unroll 1
-      while (ksum < ran) {
-        ++i;
-        if (i == rows) { ksum = 1.1; i = 1; }
-        ksum += tab[(size_t)(i - 1) * cols];
-      }
-    } else {
+    for (int base = 0; open && base < last_row; base += 32) {
+      const double mine = base + lane < last_row ? tab[(size_t)(base + lane) * cols] : 0.0;
 #pragma unroll 1
-      while (ksum < ran) {
-        ++i;
-        ksum += tab[(size_t)(i - 1) * cols];
-        if (i == rows) { ksum = 1.1; i = 1; }
+      for (int t = 0; t < 32 && base + t < last_row; ++t) {
+        ksum += __shfl_sync(0xffffffffu, mine, t);
+        if (!(ksum < ran)) {
+          i = base + t + 1;
+          open = false;
+          break;
+        }
       }
     }
+    if (open || i == rows) i = 1;
     const int j = i % 2, k = i / 2;
     const double c = phon == 0 ? 0.01 : 0.04;
     double ef;
