@@ -66,6 +66,18 @@ void push_counts(mcb200_ctx *c) {
   c->n_stale = false;
 }
 
+// n fixed-point sums of the device as doubles, converted where they land
+// (a buffer of their own would be another array's worth of page faults).
+void read_fixed(double *out, const void *src, size_t n, double scale) {
+  static_assert(sizeof(long long) == sizeof(double), "converted in place");
+  ck(cudaMemcpy(out, src, n * sizeof(long long), cudaMemcpyDeviceToHost), "copy");
+  for (size_t i = 0; i < n; ++i) {
+    long long v;
+    std::memcpy(&v, out + i, sizeof(v));
+    out[i] = (double)v / scale;
+  }
+}
+
 // Reads back the timing of ring slot q (its events are complete or the call waits for them).
 void harvest_timing(mcb200_ctx *c, int q) {
   if (!c->ev_pending[q]) return;
@@ -556,7 +568,7 @@ void init_device_context(mcb200_ctx *c, size_t max_particles) {
   ck(cudaMemsetAsync(c->dev_counts, 0, 4 * sizeof(unsigned int), c->stream), "memset");
   ck(cudaMemsetAsync(c->dev_psteps, 0, sizeof(unsigned long long), c->stream), "memset");
   ck(cudaMallocHost(&c->h_pinned, 64 * sizeof(unsigned int)), "cudaMallocHost");
-  ck(cudaMallocHost(&c->h_scratch, 16 * sizeof(double)), "cudaMallocHost");
+  ck(cudaMallocHost(&c->h_scratch, (16 + kCntNumCounters + kMaxContacts * 6) * sizeof(double)), "cudaMallocHost");
   ck(cudaMemsetAsync(c->y.counters, 0, sizeof(unsigned long long) * kCntNumCounters, c->stream), "memset");
   ck(cudaMemsetAsync(c->y.contact, 0, sizeof(long long) * kMaxContacts * 6, c->stream), "memset");
   ck(cudaStreamSynchronize(c->stream), "sync");
@@ -831,6 +843,7 @@ int mcb200_set_cells(mcb200_ctx *c, const int32_t *motion_rule, const int32_t *a
     m.surface_scatter = (flags & MCB200_FLAG_SURFACE_SCATTER) ? 1 : 0;
     m.surface_impurity = (flags & MCB200_FLAG_SURFACE_IMPURITY) ? 1 : 0;
     m.heat = (flags & MCB200_FLAG_HEAT) ? 1 : 0;
+    if (m.heat) c->heat_tallied = true;
     m.quantum = (flags & MCB200_FLAG_QUANTUM) ? 1 : 0;
     if (m.quantum && !c->ts->dt.disp)
       return fail(c, MCB200_ERR_STATE, "quantum correction needs the phonon dispersion tables (kloem.txt, kloab.txt, "
@@ -1212,12 +1225,18 @@ int mcb200_get_tallies(mcb200_ctx *c, uint64_t *counters, double *contact, doubl
   if (!c->mesh_set) return fail(c, MCB200_ERR_STATE, "mcb200_get_tallies before mcb200_set_mesh");
   try {
     ck(cudaSetDevice(c->device), "cudaSetDevice");
-    ck(cudaStreamSynchronize(c->stream), "sync");
-    pull_counts(c);
-    if (counters) ck(cudaMemcpy(counters, c->y.counters, sizeof(uint64_t) * kCntNumCounters, cudaMemcpyDeviceToHost), "copy");
+    // the small tallies to pinned memory, ahead of the wait
+    long long *small = reinterpret_cast<long long *>(c->h_scratch + 16);
+    ck(cudaMemcpyAsync(small, c->y.counters, sizeof(long long) * kCntNumCounters, cudaMemcpyDeviceToHost, c->stream),
+       "copy");
+    ck(cudaMemcpyAsync(small + kCntNumCounters, c->y.contact, sizeof(long long) * kMaxContacts * 6,
+                       cudaMemcpyDeviceToHost, c->stream),
+       "copy");
+    if (!c->n_stale) ck(cudaStreamSynchronize(c->stream), "sync");
+    pull_counts(c);  // (waits for the stream when the counts are stale)
+    if (counters) std::memcpy(counters, small, sizeof(uint64_t) * kCntNumCounters);
     if (contact) {
-      std::vector<long long> v(kMaxContacts * 6);
-      ck(cudaMemcpy(v.data(), c->y.contact, sizeof(long long) * v.size(), cudaMemcpyDeviceToHost), "copy");
+      const long long *v = small + kCntNumCounters;
       for (int i = 0; i < kMaxContacts; ++i) {
         contact[i * 6 + 0] = (double)v[i * 6 + 0];
         contact[i * 6 + 1] = (double)v[i * 6 + 1] / kChargeScale;
@@ -1227,17 +1246,14 @@ int mcb200_get_tallies(mcb200_ctx *c, uint64_t *counters, double *contact, doubl
         contact[i * 6 + 5] = (double)v[i * 6 + 5] / kEnergyScale;
       }
     }
-    auto get = [&](double *dst, const long long *src, size_t n, double scale) {
-      if (!dst) return;
-      std::vector<long long> v(n);
-      ck(cudaMemcpy(v.data(), src, sizeof(long long) * n, cudaMemcpyDeviceToHost), "copy");
-      for (size_t i = 0; i < n; ++i) dst[i] = (double)v[i] / scale;
-    };
     const size_t nodes = (size_t)(c->mesh.nx + 1) * (c->mesh.ny + 1) * (c->mesh.nz + 1);
-    get(lcurrent, c->y.lcurrent, c->mesh.ny + 1, kChargeScale);
-    get(rcurrent, c->y.rcurrent, c->mesh.ny + 1, kChargeScale);
-    get(heat_e, c->y.heat_e, nodes, kEnergyScale);
-    get(heat_h, c->y.heat_h, nodes, kEnergyScale);
+    if (lcurrent) read_fixed(lcurrent, c->y.lcurrent, c->mesh.ny + 1, kChargeScale);
+    if (rcurrent) read_fixed(rcurrent, c->y.rcurrent, c->mesh.ny + 1, kChargeScale);
+    // (a heat tally that was off since the last reset holds zeros)
+    if (heat_e && c->heat_tallied) read_fixed(heat_e, c->y.heat_e, nodes, kEnergyScale);
+    else if (heat_e) std::fill(heat_e, heat_e + nodes, 0.0);
+    if (heat_h && c->heat_tallied) read_fixed(heat_h, c->y.heat_h, nodes, kEnergyScale);
+    else if (heat_h) std::fill(heat_h, heat_h + nodes, 0.0);
     return MCB200_OK;
   } catch (const CapacityError &e) {
     return fail(c, MCB200_ERR_CAPACITY, e.what());
@@ -1311,6 +1327,7 @@ int mcb200_reset_tallies(mcb200_ctx *c) {
       ck(cudaMemsetAsync(c->y.rcurrent, 0, sizeof(long long) * (c->mesh.ny + 1), s), "memset");
       ck(cudaMemsetAsync(c->y.heat_e, 0, sizeof(long long) * nodes, s), "memset");
       ck(cudaMemsetAsync(c->y.heat_h, 0, sizeof(long long) * nodes, s), "memset");
+      c->heat_tallied = c->mesh.heat != 0;
     }
     if (c->ib.sum) ck(cudaMemsetAsync(c->ib.sum, 0, 2 * sizeof(double), s), "memset");
     ck(cudaStreamSynchronize(s), "sync");
@@ -1812,6 +1829,7 @@ int mcb200_set_heat_tally(mcb200_ctx *c, int enable) {
   if (!c) return MCB200_ERR_ARG;
   if (!c->cells_set) return fail(c, MCB200_ERR_STATE, "mcb200_set_heat_tally before mcb200_set_cells");
   c->mesh.heat = enable ? 1 : 0;
+  if (enable) c->heat_tallied = true;
   return MCB200_OK;
 }
 
@@ -1907,9 +1925,7 @@ int mcb200_stat_get(mcb200_ctx *c, const char *name, double *out, size_t n) {
     }
     if (nm == "cell_count") {
       if (n < cells) return fail(c, MCB200_ERR_CAPACITY, "output too small");
-      std::vector<unsigned long long> h(cells);
-      ck(cudaMemcpy(h.data(), c->sb.cell_count, cells * 8, cudaMemcpyDeviceToHost), "copy");
-      for (size_t q = 0; q < cells; ++q) out[q] = (double)h[q];
+      read_fixed(out, c->sb.cell_count, cells, 1.0);
       return MCB200_OK;
     }
     if (nm == "pot_sum" || nm == "qc_pot_sum") {
@@ -1924,11 +1940,8 @@ int mcb200_stat_get(mcb200_ctx *c, const char *name, double *out, size_t n) {
       for (int f = 0; f < 5; ++f)
         if (nm == std::string(t == 0 ? "electron_" : "hole_") + fields[f]) {
           if (n < nodes) return fail(c, MCB200_ERR_CAPACITY, "output too small");
-          std::vector<long long> h(nodes);
-          ck(cudaMemcpy(h.data(), c->sb.node + ((size_t)t * 5 + f) * nodes, nodes * 8, cudaMemcpyDeviceToHost),
-             "copy");
           const double scale = f < 3 ? c->ss.v[t] : (f == 3 ? c->ss.q[t] : c->ss.e[t]);
-          for (size_t q = 0; q < nodes; ++q) out[q] = (double)h[q] / scale;
+          read_fixed(out, c->sb.node + ((size_t)t * 5 + f) * nodes, nodes, scale);
           return MCB200_OK;
         }
     return fail(c, MCB200_ERR_ARG, "unknown statistic " + nm);

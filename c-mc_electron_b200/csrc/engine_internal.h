@@ -209,6 +209,7 @@ struct mcb200_ctx {
   // sort scratch
   unsigned int *hist = nullptr, *offsets = nullptr, *tile_sums = nullptr, *total = nullptr;
   int ncells = 0;
+  bool heat_tallied = false;         // heat may have been tallied since the last reset
   unsigned int *h_pinned = nullptr;  // small pinned readback area
   MrScratch mr;                      // in mesh_owned
   // effective-potential quantum correction (mcb200_set_quantum_correction);
