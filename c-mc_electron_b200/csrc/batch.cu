@@ -40,6 +40,9 @@ struct mcb200_batch {
   uint64_t graph_replays = 0, graph_captures = 0;
   cudaEvent_t marks[8] = {};
   void *tables = nullptr;          // device: [6][n] BatchInstT (main flight x 2 parities, 4 copy generations)
+  void *tails = nullptr;           // device: [2][n] BatchTailT, by store parity
+  int *tile_first = nullptr;       // device: [n + 1]
+  int record_tiles = 0, scan_tiles = 0;  // of all members
   uint32_t *steps = nullptr;       // device: step number of each member
   unsigned int *tickets = nullptr;  // device: work counters of the batched launches (main, 4 copy generations, side)
   bool overlap = true;              // fly the members not solving Poisson beside the solves
@@ -50,7 +53,7 @@ struct mcb200_batch {
   uint64_t solo = 0;
   size_t solo_min = 0;  // their smallest particle count (0: none solo)
   cudaEvent_t ev_steps = nullptr;  // after the step numbers advanced
-  std::vector<unsigned char> snap;  // per member: DevMesh, DevTallies and store parity the tables were built for
+  std::vector<unsigned char> snap;  // per member: what the tables were built for (MemberSnap)
   uint64_t steps_done = 0, built_at = 0;
   int blocks_per_sm = 0;  // batched flight grid (0: as many as fit); mcb200_batch_autotune
   uint64_t launches = 0;
@@ -72,6 +75,8 @@ struct mcb200_batch {
     if (tables) cudaFree(tables);
     if (steps) cudaFree(steps);
     if (tickets) cudaFree(tickets);
+    if (tails) cudaFree(tails);
+    if (tile_first) cudaFree(tile_first);
     if (ev_flight) cudaEventDestroy(ev_flight);
     for (cudaEvent_t e : ev_member)
       if (e) cudaEventDestroy(e);
@@ -90,22 +95,36 @@ int bfail(mcb200_batch *b, int code, const std::string &msg) {
   return code;
 }
 
-constexpr size_t kSnapBytes = sizeof(DevMesh) + sizeof(DevTallies) + sizeof(int);
+// What the tables hold of a member that can change between its steps.
+struct MemberSnap {
+  DevMesh mesh;
+  DevTallies tallies;
+  const void *hist, *offsets, *tile_sums;
+  int shift, parity;
+};
+constexpr size_t kSnapBytes = sizeof(MemberSnap);
 
 void snapshot(const mcb200_ctx *c, int parity, unsigned char *out) {
-  std::memcpy(out, &c->mesh, sizeof(DevMesh));
-  std::memcpy(out + sizeof(DevMesh), &c->y, sizeof(DevTallies));
-  std::memcpy(out + sizeof(DevMesh) + sizeof(DevTallies), &parity, sizeof(int));
+  std::memset(out, 0, kSnapBytes);
+  std::memcpy(out + offsetof(MemberSnap, mesh), &c->mesh, sizeof(DevMesh));
+  std::memcpy(out + offsetof(MemberSnap, tallies), &c->y, sizeof(DevTallies));
+  const void *sort[3] = {c->hist, c->offsets, c->tile_sums};
+  std::memcpy(out + offsetof(MemberSnap, hist), sort, sizeof(sort));
+  std::memcpy(out + offsetof(MemberSnap, shift), &c->sort_shift, sizeof(int));
+  std::memcpy(out + offsetof(MemberSnap, parity), &parity, sizeof(int));
 }
 
 // The six tables of the batch, for the members' current stores and meshes:
 // main flight at this step's store parity and at the next, then the four
 // copy generations (copies of generation g go to g + 1; the last
-// generation's copies are counted in the member's sink).
+// generation's copies are counted in the member's sink); and the members'
+// part of the step's records and tail, by store parity.
 template <typename R>
 void build_tables(mcb200_batch *b) {
   const int n = (int)b->m.size();
   std::vector<BatchInstT<R>> t(6 * (size_t)n);
+  std::vector<BatchTailT<R>> tail(2 * (size_t)n);
+  b->record_tiles = b->scan_tiles = 0;
   for (int k = 0; k < n; ++k) {
     mcb200_ctx *c = b->m[k];
     BatchInstT<R> base{};
@@ -135,19 +154,48 @@ void build_tables(mcb200_batch *b) {
       }
       t[(size_t)(2 + g) * n + k] = e;
     }
+    for (int par = 0; par < 2; ++par) {
+      BatchTailT<R> e{};
+      e.M = c->mesh;
+      e.records = sizeof(R) == 4 ? (void *)c->cell32 : (void *)c->cell64;
+      e.counters = step_counters<R>(c);
+      e.src = store<R>(c, par == 0 ? c->cur : 1 - c->cur);
+      e.dst = store<R>(c, par == 0 ? 1 - c->cur : c->cur);
+      for (int g = 0; g < mcb200_ctx::kGenerations; ++g) e.set.g[g] = children<R>(c, g);
+      e.finish = step_finish(c);
+      e.overflow = c->dev_counts + 2;
+      e.hist = c->hist;
+      e.offsets = c->offsets;
+      e.tile_sums = c->tile_sums;
+      e.total = c->total;
+      e.bounds = c->bounds;
+      e.cells = c->ncells;
+      e.shift = c->sort_shift;
+      e.buckets = (c->ncells + (1 << c->sort_shift) - 1) >> c->sort_shift;
+      e.capacity = (int)c->capacity;
+      e.nx = c->mesh.nx;
+      e.nz = c->mesh.nz;
+      tail[(size_t)par * n + k] = e;
+      if (par == 0) {
+        b->record_tiles += (e.cells + 255) / 256;
+        b->scan_tiles += (e.buckets + 1023) / 1024;
+      }
+    }
     snapshot(c, c->cur, &b->snap[(size_t)k * kSnapBytes]);
   }
   // the previous launches may still read the tables: replace them in order on the batch stream
   ck(cudaStreamSynchronize(b->stream), "sync");
   ck(cudaMemcpyAsync(b->tables, t.data(), t.size() * sizeof(BatchInstT<R>), cudaMemcpyHostToDevice, b->stream),
      "upload batch tables");
+  ck(cudaMemcpyAsync(b->tails, tail.data(), tail.size() * sizeof(BatchTailT<R>), cudaMemcpyHostToDevice, b->stream),
+     "upload batch tables");
   ck(cudaStreamSynchronize(b->stream), "sync");
   b->built_at = b->steps_done;
   b->drop_graphs();  // they hold the old tables' layout assumptions
 }
 
-// True when every member still has the mesh, tallies and store parity the
-// tables assume for this step.
+// True when every member still has the mesh, tallies, sort buffers and store
+// parity the tables assume for this step.
 bool tables_current(const mcb200_batch *b) {
   const int flip = (int)((b->steps_done - b->built_at) & 1);
   unsigned char now[kSnapBytes];
@@ -155,7 +203,7 @@ bool tables_current(const mcb200_batch *b) {
     const mcb200_ctx *c = b->m[k];
     const unsigned char *was = &b->snap[k * kSnapBytes];
     int built_cur = 0;
-    std::memcpy(&built_cur, was + sizeof(DevMesh) + sizeof(DevTallies), sizeof(int));
+    std::memcpy(&built_cur, was + offsetof(MemberSnap, parity), sizeof(int));
     if (c->cur != (flip ? 1 - built_cur : built_cur)) return false;
     snapshot(c, built_cur, now);
     if (std::memcmp(now, was, kSnapBytes) != 0) return false;
@@ -195,7 +243,7 @@ void batch_transport(mcb200_batch *b, uint64_t early = 0) {
   F.T = b->m[0]->ts->dt;
   for (int k = 0; k < n; ++k) {
     mcb200_ctx *c = b->m[k];
-    step_prepare<R>(c);
+    step_prepare<R>(c, ((solo >> k) & 1) != 0);
     if ((solo >> k) & 1) {
       FlightCtxT<R> Fk;
       Fk.T = F.T;
@@ -215,6 +263,7 @@ void batch_transport(mcb200_batch *b, uint64_t early = 0) {
   // 2. the batched flights
   const int flip = (int)((b->steps_done - b->built_at) & 1);
   const BatchInstT<R> *tab = static_cast<const BatchInstT<R> *>(b->tables);
+  const BatchTailT<R> *tails = static_cast<const BatchTailT<R> *>(b->tails) + (size_t)flip * n;
   const int sms = b->m[0]->sm_count;
   unsigned int *side_ticket = b->tickets + kFlightTickets;
   long long expected = 0;  // the members' counts as the host last knew them
@@ -225,7 +274,8 @@ void batch_transport(mcb200_batch *b, uint64_t early = 0) {
   if (batched) {
     if (early) {
       ck(cudaMemsetAsync(side_ticket, 0, sizeof(unsigned int), b->side), "memset");
-      if (launch_batch_drift<R>(F, tab + (size_t)flip * n, n, early, sms, b->side))
+      if (launch_batch_records<R>(F.T, tails, n, early, b->record_tiles, b->side) ||
+          launch_batch_drift<R>(F, tab + (size_t)flip * n, n, early, sms, b->side))
         throw std::runtime_error("batched drift launch failed");
       ck(cudaEventRecord(b->ev_side0, b->side), "event");  // the side counter is reset, the lists are made
       if (launch_batch_flight<R>(F, tab + (size_t)flip * n, n, early, b->steps, flight, side_ticket, 1, sms, b->side,
@@ -234,7 +284,8 @@ void batch_transport(mcb200_batch *b, uint64_t early = 0) {
       ck(cudaEventRecord(b->ev_side, b->side), "event");
     }
     ck(cudaMemsetAsync(b->tickets, 0, sizeof(unsigned int) * kFlightTickets, b->stream), "memset");
-    if (launch_batch_drift<R>(F, tab + (size_t)flip * n, n, batched & ~early, sms, b->stream))
+    if (launch_batch_records<R>(F.T, tails, n, batched & ~early, b->record_tiles, b->stream) ||
+        launch_batch_drift<R>(F, tab + (size_t)flip * n, n, batched & ~early, sms, b->stream))
       throw std::runtime_error("batched drift launch failed");
     if (launch_batch_flight<R>(F, tab + (size_t)flip * n, n, batched & ~early, b->steps, flight, b->tickets,
                                b->blocks_per_sm, sms, b->stream, b->smem_table))
@@ -253,15 +304,24 @@ void batch_transport(mcb200_batch *b, uint64_t early = 0) {
       if (launch_batch_flight<R>(F, tab + (size_t)(2 + g) * n, n, batched, b->steps, BatchPart::kChildren, b->tickets + 2 + g,
                                  b->blocks_per_sm, sms, b->stream, b->smem_table))
         throw std::runtime_error("batched copy flight launch failed");
-    // (a drift pass, its flight and the draws' count as one)
+    // the members' tails
+    if (launch_batch_tails<R>(tails, n, batched, b->scan_tiles, b->tile_first, sms, b->stream))
+      throw std::runtime_error("batched sort launch failed");
+    // (counted: the flights; a drift pass, its flight and the draws' as one)
     b->launches += 2 + mcb200_ctx::kGenerations + (early ? 2 : 0);
   }
   ck(cudaEventRecord(b->ev_flight, b->stream), "event");
-  // 3. every member: its tail after its flights, on its own stream
+  // 3. every solo member: its tail after its flights, on its own stream; the
+  //    others' streams wait for theirs
   for (int k = 0; k < n; ++k) {
     mcb200_ctx *c = b->m[k];
-    if (!((solo >> k) & 1)) ck(cudaStreamWaitEvent(c->stream, b->ev_flight, 0), "wait");
-    step_tail<R>(c);
+    if ((solo >> k) & 1) {
+      step_tail<R>(c);
+      continue;
+    }
+    ck(cudaStreamWaitEvent(c->stream, b->ev_flight, 0), "wait");
+    c->cur = 1 - c->cur;
+    c->n_stale = true;
   }
   // 4. the step numbers advance once every flight has read them; the solo
   //    members' next flights wait for that
@@ -472,6 +532,10 @@ int mcb200_batch_create(mcb200_ctx *const *ctxs, const mcb200_batch_member *memb
     ck(cudaMalloc(&b->tables, 6 * (size_t)n * entry), "cudaMalloc");
     ck(cudaMalloc(&b->steps, (size_t)n * sizeof(uint32_t)), "cudaMalloc");
     ck(cudaMalloc(&b->tickets, (kFlightTickets + 1) * sizeof(unsigned int)), "cudaMalloc");
+    ck(cudaMalloc(&b->tails, 2 * (size_t)n * (b->precision == MCB200_FLIGHT_FP32 ? sizeof(BatchTailT<float>)
+                                                                                 : sizeof(BatchTailT<double>))),
+       "cudaMalloc");
+    ck(cudaMalloc(&b->tile_first, (n + 1) * sizeof(int)), "cudaMalloc");
     std::vector<uint32_t> first_steps(n);
     for (int k = 0; k < n; ++k) first_steps[k] = members[k].first_step;
     b->member_step = first_steps;

@@ -2056,20 +2056,43 @@ void surface_rates_enqueue(mcb200_ctx *c, cudaStream_t s) {
   c->launches += 1;
 }
 
+template <typename R>
+StepCounters step_counters(mcb200_ctx *c) {
+  StepCounters z{c->tickets, {}, c->append_count, c->tickets + kFlightTickets};
+  for (int g = 0; g < mcb200_ctx::kGenerations; ++g) z.count[g] = children<R>(c, g).count;
+  z.count[mcb200_ctx::kGenerations] = c->sink_count;
+  return z;
+}
+StepFinish step_finish(mcb200_ctx *c) {
+  StepFinish fin;
+  fin.n = c->dev_counts;
+  fin.sorted_total = c->total;
+  fin.next_uid = c->dev_counts + 1;
+  fin.appended = c->append_count;
+  fin.particle_steps = c->dev_psteps;
+  fin.blocks = c->finish_blocks;
+  fin.scan_blocks = c->finish_blocks + 1;
+  return fin;
+}
+template StepCounters step_counters<float>(mcb200_ctx *);
+template StepCounters step_counters<double>(mcb200_ctx *);
+
 // Before the flights of a step: the induced-current tally (when on), work
 // counters, the FP32 per-cell records, and zeroed copy counters of every
 // generation and of the sink.
 template <typename R>
-void step_prepare(mcb200_ctx *c) {
+void step_prepare(mcb200_ctx *c, bool records) {
   cudaStream_t s = c->stream;
   if (c->induced_contact >= 0) {  // the induced current of the store the step starts from
     launch_induced_current(store<R>(c, c->cur), DevCount{c->dev_counts, nullptr, (int)c->capacity}, c->mesh,
                            c->ts->dt, c->ib, grid_for(c, c->capacity, 256), s);
     c->launches += 2;
   }
-  StepCounters z{c->tickets, {}, c->append_count, c->tickets + kFlightTickets};
-  for (int g = 0; g < mcb200_ctx::kGenerations; ++g) z.count[g] = children<R>(c, g).count;
-  z.count[mcb200_ctx::kGenerations] = c->sink_count;
+  const StepCounters z = step_counters<R>(c);
+  if (!records) {  // (a batch makes them in one launch for its members)
+    join_stat(c);
+    return;
+  }
   if constexpr (sizeof(R) == 4)  // the per-cell records the flight reads
     launch_records_and_reset(c->ts->dt, c->mesh, c->cell32, c->ncells, z, s);
   else
@@ -2093,14 +2116,7 @@ void step_tail(mcb200_ctx *c) {
   ck(cudaGetLastError(), "append children");
   c->launches += 1;
   const int other = 1 - c->cur;
-  StepFinish fin;  // by the scatter's last block
-  fin.n = c->dev_counts;
-  fin.sorted_total = c->total;
-  fin.next_uid = c->dev_counts + 1;
-  fin.appended = c->append_count;
-  fin.particle_steps = c->dev_psteps;
-  fin.blocks = c->finish_blocks;
-  fin.scan_blocks = c->finish_blocks + 1;
+  const StepFinish fin = step_finish(c);  // by the scatter's last block
   launch_cell_sort(store<R>(c, c->cur), DevCount{c->dev_counts, c->append_count, cap}, store<R>(c, other), c->ncells,
                    c->mesh.nx, c->mesh.nz, c->hist, c->offsets, c->tile_sums, c->total, c->sort_shift, c->bounds,
                    grid_for(c, c->capacity, 256), s, fin);
@@ -2166,7 +2182,7 @@ void step_impl(mcb200_ctx *c, uint32_t step, uint64_t seed, double dt) {
     c->ev_pending[q] = true;
     ck(cudaEventRecord(ev[0], s), "event");
   }
-  step_prepare<R>(c);
+  step_prepare<R>(c, true);
   enqueue_flights<R>(c, F, ev);
   // 3.-4. append the copies, sort by cell
   step_tail<R>(c);
@@ -2177,8 +2193,8 @@ void step_impl(mcb200_ctx *c, uint32_t step, uint64_t seed, double dt) {
   }
 }
 
-template void step_prepare<float>(mcb200_ctx *);
-template void step_prepare<double>(mcb200_ctx *);
+template void step_prepare<float>(mcb200_ctx *, bool);
+template void step_prepare<double>(mcb200_ctx *, bool);
 template void step_tail<float>(mcb200_ctx *);
 template void step_tail<double>(mcb200_ctx *);
 template void enqueue_flights<float>(mcb200_ctx *, FlightCtxT<float>, cudaEvent_t *);

@@ -338,7 +338,10 @@ void surface_rates_enqueue(mcb200_ctx *c, cudaStream_t s);
 void deposit_enqueue(mcb200_ctx *c, cudaStream_t s);
 // The parts of a transport step around its flights (engine.cu).
 template <typename R>
-void step_prepare(mcb200_ctx *c);
+void step_prepare(mcb200_ctx *c, bool records);
+template <typename R>
+StepCounters step_counters(mcb200_ctx *c);
+StepFinish step_finish(mcb200_ctx *c);
 template <typename R>
 void step_tail(mcb200_ctx *c);
 // The main and copy flights of a step on the context's stream (after

@@ -92,6 +92,31 @@ struct StepFinish {
   unsigned int *blocks = nullptr;
   unsigned int *scan_blocks = nullptr;
 };
+// One member's part of a batch's step kernels (device table): its cell
+// records and step counters, and its step's tail (the copies of `set` join
+// `src`, which is sorted into `dst`).
+template <typename R>
+struct BatchTailT {
+  DevMesh M;
+  void *records;  // float4 or double2 [cells][3]
+  StepCounters counters;
+  DevParticlesT<R> src, dst;
+  ChildSetT<R> set;
+  StepFinish finish;
+  unsigned int *overflow, *hist, *offsets, *tile_sums, *total;
+  unsigned long long *bounds;
+  int cells, buckets, capacity, nx, nz, shift;
+};
+// The records of the members in `members` (tiles: of 256 cells, of all
+// members); their tails in four launches (scan_tiles: of 1024 buckets, of
+// all members; tile_first: device scratch of n + 1 ints).  Return 0 on
+// success.
+template <typename R>
+int launch_batch_records(const DevTables &T, const BatchTailT<R> *tails, int n, uint64_t members, int tiles,
+                         cudaStream_t s);
+template <typename R>
+int launch_batch_tails(const BatchTailT<R> *tails, int n, uint64_t members, int scan_tiles, int *tile_first,
+                       int sm_count, cudaStream_t s);
 template <typename R>
 void launch_seed(const FlightCtx &F, const DevParticlesT<R> &P, int offset, int n, const int *cell_of,
                  const double *charge, int type, uint32_t uid0, int grid, cudaStream_t s);

@@ -590,11 +590,7 @@ __device__ __forceinline__ void reset_step_counters(const StepCounters &z, int t
 }
 // FP64 flight's records (DevMesh::cell64): the factors of the reference's
 // expressions that hold no particle value, each rounded as there.
-__global__ void cell_records64_kernel(DevTables T, DevMesh M, double2 *out, int cells, StepCounters z) {
-  pdl_wait();
-  if (blockIdx.x == 0) reset_step_counters(z, threadIdx.x);
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= cells) return;
+__device__ __forceinline__ void cell_record(const DevTables &T, const DevMesh &M, double2 *out, int c) {
   const double rho = M.rho[c], da = M.da[c];
   // a surface-impurity cell: the reference's formula is commented out there
   // and leaves the rate unset; the engine treats it as zero
@@ -606,11 +602,7 @@ __global__ void cell_records64_kernel(DevTables T, DevMesh M, double2 *out, int 
       make_double2(kPiD * (fr * fr), T.frickel * 4 * kPiD * rho / (8.0 * T.melt * T.eps_si));
   out[3 * (size_t)c + 2] = make_double2(T.frickel * 4 * kPiD * rho / T.eps_si, 0.0);
 }
-__global__ void cell_records32_kernel(DevTables T, DevMesh M, float4 *out, int cells, StepCounters z) {
-  pdl_wait();
-  if (blockIdx.x == 0) reset_step_counters(z, threadIdx.x);
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= cells) return;
+__device__ __forceinline__ void cell_record(const DevTables &T, const DevMesh &M, float4 *out, int c) {
   const double rho = M.rho[c], da = M.da[c];
   const bool on = (da * T.conc0 >= 1e22) && !(M.surface_scatter && M.surface_impurity && M.in_surf[c]);
   const double eebeta = T.frickel * 4 * kPiD * rho / (2.0 * T.meld * T.eps_si);
@@ -624,6 +616,14 @@ __global__ void cell_records32_kernel(DevTables T, DevMesh M, float4 *out, int c
                                        (float)(T.frickel * 4 * kPiD * rho / T.eps_si), (float)(0.120 / T.eV0), 0.0f);
 }
 
+template <typename Rec>
+__global__ void cell_records_kernel(DevTables T, DevMesh M, Rec *out, int cells, StepCounters z) {
+  pdl_wait();
+  if (blockIdx.x == 0) reset_step_counters(z, threadIdx.x);
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c < cells) cell_record(T, M, out, c);
+}
+
 // ---- counting sort by cell ------------------------------------------------
 __device__ __forceinline__ int cell_linear(uint32_t c, int nx, int nz) {
   return (int)((((c >> 10) & 1023) * nx + (c & 1023)) * nz + ((c >> 20) & 1023));
@@ -634,21 +634,24 @@ __device__ __forceinline__ int cell_linear(uint32_t c, int nx, int nz) {
 // shorter and leave the particles of a bucket in arrival order.  When the
 // scatter will compute the sorted store's charge bounds, they start from
 // zero here.
+__device__ __forceinline__ void histogram_warp(const uint32_t *cell, const uint32_t *meta, int n, int nx, int nz,
+                                               unsigned int *hist, int shift, int p) {
+  // a warp takes 32 consecutive particles; lanes of the same bucket (a
+  // cell-sorted store holds runs of them) add their count with one atomic
+  const unsigned lane = threadIdx.x & 31u;
+  unsigned int key = 0xffffffffu;
+  if (p < n && !(meta[p] & kMetaDead)) key = (unsigned int)(cell_linear(cell[p], nx, nz) >> shift);
+  const unsigned int peers = __match_any_sync(0xffffffffu, key);
+  if (key != 0xffffffffu && (int)lane == __ffs(peers) - 1) atomicAdd(&hist[key], (unsigned int)__popc(peers));
+}
 __global__ void cell_histogram(const uint32_t *cell, const uint32_t *meta, DevCount count, int nx, int nz,
                                unsigned int *hist, int shift, unsigned long long *bounds) {
   pdl_wait();
   const int n = count.get();
   if (bounds && blockIdx.x == 0 && threadIdx.x < 4) bounds[threadIdx.x] = 0ull;
-  // a warp walks 32 consecutive particles; lanes of the same bucket (a
-  // cell-sorted store holds runs of them) add their count with one atomic
-  const unsigned lane = threadIdx.x & 31u;
-  for (int base = blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < n; base += gridDim.x * blockDim.x) {
-    const int p = base + (int)lane;
-    unsigned int key = 0xffffffffu;
-    if (p < n && !(meta[p] & kMetaDead)) key = (unsigned int)(cell_linear(cell[p], nx, nz) >> shift);
-    const unsigned int peers = __match_any_sync(0xffffffffu, key);
-    if (key != 0xffffffffu && (int)lane == __ffs(peers) - 1) atomicAdd(&hist[key], (unsigned int)__popc(peers));
-  }
+  const int lane = (int)(threadIdx.x & 31u);
+  for (int base = blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < n; base += gridDim.x * blockDim.x)
+    histogram_warp(cell, meta, n, nx, nz, hist, shift, base + lane);
 }
 
 // Exclusive scan of `count` values, single pass per 1024-wide tile plus a
@@ -681,12 +684,11 @@ __device__ void scan_tile_sums_block(unsigned int *tile_sums, int ntiles, unsign
 // finish then scans the tile sums too (scan_tile_sums' work, one launch
 // fewer).  clear (or null): the input, zeroed once read (the step's sort
 // keeps its histogram zero between sorts, so no memset precedes it).
-__global__ void scan_tiles(const unsigned int *in, unsigned int *out, unsigned int *tile_sums, int n,
-                           unsigned int *blocks, unsigned int *total, unsigned int *clear) {
+__device__ void scan_tile(const unsigned int *in, unsigned int *out, unsigned int *tile_sums, int n,
+                          unsigned int *blocks, unsigned int *total, unsigned int *clear, int tile, int ntiles) {
   __shared__ unsigned int s[1024];
   __shared__ bool last;
-  pdl_wait();
-  const int i = blockIdx.x * 1024 + threadIdx.x;
+  const int i = tile * 1024 + threadIdx.x;
   const unsigned int v = i < n ? in[i] : 0u;
   if (clear && i < n) clear[i] = 0u;
   s[threadIdx.x] = v;
@@ -698,17 +700,22 @@ __global__ void scan_tiles(const unsigned int *in, unsigned int *out, unsigned i
     __syncthreads();
   }
   if (i < n) out[i] = s[threadIdx.x] - v;
-  if (threadIdx.x == 1023) tile_sums[blockIdx.x] = s[1023];
+  if (threadIdx.x == 1023) tile_sums[tile] = s[1023];
   if (blocks == nullptr) return;  // uniform over the grid
   if (threadIdx.x == 1023) {
     __threadfence();
-    last = atomicAdd(blocks, 1u) == gridDim.x - 1;
+    last = atomicAdd(blocks, 1u) == (unsigned)ntiles - 1u;
   }
   __syncthreads();
   if (!last) return;  // uniform over the block
   __threadfence();
-  scan_tile_sums_block(tile_sums, (int)gridDim.x, total);
+  scan_tile_sums_block(tile_sums, ntiles, total);
   if (threadIdx.x == 0) *blocks = 0u;
+}
+__global__ void scan_tiles(const unsigned int *in, unsigned int *out, unsigned int *tile_sums, int n,
+                           unsigned int *blocks, unsigned int *total, unsigned int *clear) {
+  pdl_wait();
+  scan_tile(in, out, tile_sums, n, blocks, total, clear, (int)blockIdx.x, (int)gridDim.x);
 }
 __global__ void scan_tile_sums(unsigned int *tile_sums, int ntiles, unsigned int *total) {
   scan_tile_sums_block(tile_sums, ntiles, total);
@@ -726,6 +733,79 @@ __global__ void scan_add(unsigned int *out, const unsigned int *tile_sums, int n
 // tile_base (optional): cursor holds tile-local offsets and the tile's
 // exclusive prefix is added (scan_add's work, one launch fewer; the cursor
 // then ends as tile-local cell ends).
+// One warp's 32 particles, p this lane's; mx and cnt collect the bounds.
+template <typename R>
+__device__ __forceinline__ void scatter_warp(const DevParticlesT<R> &src, const DevParticlesT<R> &dst, int n,
+                                             unsigned int *cursor, int nx, int nz, int shift,
+                                             const unsigned int *tile_base, int p, unsigned long long *mx,
+                                             unsigned long long *cnt) {
+  // lanes of the same bucket take consecutive slots with one atomic
+  const unsigned lane = threadIdx.x & 31u;
+  const uint32_t m = p < n ? src.meta[p] : kMetaDead;
+  const bool live = !(m & kMetaDead);
+  const unsigned int key = live ? (unsigned int)(cell_linear(src.cell[p], nx, nz) >> shift) : 0xffffffffu;
+  const unsigned int peers = __match_any_sync(0xffffffffu, key);
+  const int leader = __ffs(peers) - 1;
+  unsigned int first = 0;
+  if (live && (int)lane == leader) first = atomicAdd(&cursor[key], (unsigned int)__popc(peers));
+  first = __shfl_sync(0xffffffffu, first, leader);
+  if (!live) return;
+  const unsigned int q = first + (unsigned int)__popc(peers & ((1u << lane) - 1u)) +
+                         (tile_base ? tile_base[key >> 10] : 0u);
+  const double charge = src.charge[p];
+  dst.x[q] = src.x[p]; dst.y[q] = src.y[p]; dst.z[q] = src.z[p];
+  dst.kx[q] = src.kx[p]; dst.ky[q] = src.ky[p]; dst.kz[q] = src.kz[p];
+  dst.energy[q] = src.energy[p]; dst.charge[q] = charge;
+  dst.cell[q] = src.cell[p];
+  dst.itet[q] = src.itet[p];
+  dst.meta[q] = m & 0xffffu;
+  dst.uid[q] = src.uid[p];
+  const int t = ((m >> 8) & 255) == 0 ? 0 : 1;
+  const unsigned long long b = (unsigned long long)__double_as_longlong(fabs(charge));
+  mx[t] = b > mx[t] ? b : mx[t];
+  cnt[t] += 1;
+}
+// The block's bounds into the store's (every thread of a block of up to 256 calls it).
+__device__ __forceinline__ void scatter_bounds(unsigned long long *mx, unsigned long long *cnt,
+                                               unsigned long long *bounds) {
+  __shared__ unsigned long long red[4][8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int t = 0; t < 2; ++t) {
+    for (int o = 16; o > 0; o >>= 1) {
+      const unsigned long long om = __shfl_down_sync(0xffffffffu, mx[t], o);
+      mx[t] = om > mx[t] ? om : mx[t];
+      cnt[t] += __shfl_down_sync(0xffffffffu, cnt[t], o);
+    }
+    if (lane == 0) {
+      red[t][warp] = mx[t];
+      red[2 + t][warp] = cnt[t];
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x < 4) {
+    const int v = threadIdx.x;
+    unsigned long long a = 0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) a = v < 2 ? (red[v][w] > a ? red[v][w] : a) : a + red[v][w];
+    if (v < 2) {
+      if (a) atomicMax(bounds + v, a);
+    } else if (a) {
+      atomicAdd(bounds + v, a);
+    }
+  }
+}
+// The end of the step, by the last of `parts` (thread 0 of each calls it
+// once its block is done with the count).
+__device__ __forceinline__ void finish_step(const StepFinish &finish, unsigned int parts) {
+  __threadfence();
+  const unsigned int done = atomicAdd(finish.blocks, 1u);
+  if (done == parts - 1u) {  // every part has read the count
+    __threadfence();
+    *finish.particle_steps += *finish.n;
+    *finish.n = *finish.sorted_total;
+    *finish.next_uid += *finish.appended;
+    *finish.blocks = 0u;
+  }
+}
 template <typename R>
 __global__ void __launch_bounds__(256) cell_scatter(DevParticlesT<R> src, DevCount count, DevParticlesT<R> dst,
                                                     unsigned int *cursor, int nx, int nz, int shift,
@@ -734,73 +814,13 @@ __global__ void __launch_bounds__(256) cell_scatter(DevParticlesT<R> src, DevCou
   pdl_wait();
   const int n = count.get();
   unsigned long long mx[2] = {0, 0}, cnt[2] = {0, 0};
-  // lanes of the same bucket take consecutive slots with one atomic
-  const unsigned lane = threadIdx.x & 31u;
-  for (int base = blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < n; base += gridDim.x * blockDim.x) {
-    const int p = base + (int)lane;
-    const uint32_t m = p < n ? src.meta[p] : kMetaDead;
-    const bool live = !(m & kMetaDead);
-    const unsigned int key = live ? (unsigned int)(cell_linear(src.cell[p], nx, nz) >> shift) : 0xffffffffu;
-    const unsigned int peers = __match_any_sync(0xffffffffu, key);
-    const int leader = __ffs(peers) - 1;
-    unsigned int first = 0;
-    if (live && (int)lane == leader) first = atomicAdd(&cursor[key], (unsigned int)__popc(peers));
-    first = __shfl_sync(0xffffffffu, first, leader);
-    if (!live) continue;
-    const unsigned int q = first + (unsigned int)__popc(peers & ((1u << lane) - 1u)) +
-                           (tile_base ? tile_base[key >> 10] : 0u);
-    const double charge = src.charge[p];
-    dst.x[q] = src.x[p]; dst.y[q] = src.y[p]; dst.z[q] = src.z[p];
-    dst.kx[q] = src.kx[p]; dst.ky[q] = src.ky[p]; dst.kz[q] = src.kz[p];
-    dst.energy[q] = src.energy[p]; dst.charge[q] = charge;
-    dst.cell[q] = src.cell[p];
-    dst.itet[q] = src.itet[p];
-    dst.meta[q] = m & 0xffffu;
-    dst.uid[q] = src.uid[p];
-    const int t = ((m >> 8) & 255) == 0 ? 0 : 1;
-    const unsigned long long b = (unsigned long long)__double_as_longlong(fabs(charge));
-    mx[t] = b > mx[t] ? b : mx[t];
-    cnt[t] += 1;
-  }
-  if (bounds != nullptr) {  // uniform over the grid
-    __shared__ unsigned long long red[4][8];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int t = 0; t < 2; ++t) {
-      for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long om = __shfl_down_sync(0xffffffffu, mx[t], o);
-        mx[t] = om > mx[t] ? om : mx[t];
-        cnt[t] += __shfl_down_sync(0xffffffffu, cnt[t], o);
-      }
-      if (lane == 0) {
-        red[t][warp] = mx[t];
-        red[2 + t][warp] = cnt[t];
-      }
-    }
-    __syncthreads();
-    if (threadIdx.x < 4) {
-      const int v = threadIdx.x;
-      unsigned long long a = 0;
-      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) a = v < 2 ? (red[v][w] > a ? red[v][w] : a) : a + red[v][w];
-      if (v < 2) {
-        if (a) atomicMax(bounds + v, a);
-      } else if (a) {
-        atomicAdd(bounds + v, a);
-      }
-    }
-  }
-  if (finish.n != nullptr) {  // uniform over the grid
+  const int lane = (int)(threadIdx.x & 31u);
+  for (int base = blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < n; base += gridDim.x * blockDim.x)
+    scatter_warp(src, dst, n, cursor, nx, nz, shift, tile_base, base + lane, mx, cnt);
+  if (bounds != nullptr) scatter_bounds(mx, cnt, bounds);  // uniform over the grid
+  if (finish.n != nullptr) {                               // uniform over the grid
     __syncthreads();  // every thread of the block has read the count
-    if (threadIdx.x == 0) {
-      __threadfence();
-      const unsigned int done = atomicAdd(finish.blocks, 1u);
-      if (done == gridDim.x - 1) {  // the last block: every block has read the count
-        __threadfence();
-        *finish.particle_steps += *finish.n;
-        *finish.n = *finish.sorted_total;
-        *finish.next_uid += *finish.appended;
-        *finish.blocks = 0u;
-      }
-    }
+    if (threadIdx.x == 0) finish_step(finish, gridDim.x);
   }
 }
 
@@ -843,15 +863,14 @@ struct CopyRef {
   }
 };
 
+// Block `block` of `blocks` (256 threads).
 template <typename R>
-__global__ void __launch_bounds__(256) append_children_kernel(ChildSetT<R> set, const unsigned int *next_uid,
-                                                              DevParticlesT<R> dst, const unsigned int *n,
-                                                              int capacity, unsigned int *appended,
-                                                              unsigned int *overflow) {
+__device__ __forceinline__ void append_block(const ChildSetT<R> &set, const unsigned int *next_uid,
+                                             const DevParticlesT<R> &dst, const unsigned int *n, int capacity,
+                                             unsigned int *appended, unsigned int *overflow, int block, int blocks) {
   constexpr int kChunk = 2048;
   __shared__ uint64_t keys[kChunk];
   __shared__ uint32_t part[8][32];
-  pdl_wait();
   const CopyRef<R> ref(set);
   int total = 0;
 #pragma unroll
@@ -860,7 +879,7 @@ __global__ void __launch_bounds__(256) append_children_kernel(ChildSetT<R> set, 
   const uint32_t uid0 = *next_uid;
   const unsigned int n0 = *n;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int base_i = blockIdx.x * 32; base_i < total; base_i += gridDim.x * 32) {
+  for (int base_i = block * 32; base_i < total; base_i += blocks * 32) {
     const int i = base_i + lane;
     uint64_t my = ~0ull;
     bool my_alive = false;
@@ -900,6 +919,130 @@ __global__ void __launch_bounds__(256) append_children_kernel(ChildSetT<R> set, 
         dst.uid[q] = uid0 + r;
       }
     }
+  }
+}
+
+template <typename R>
+__global__ void __launch_bounds__(256) append_children_kernel(ChildSetT<R> set, const unsigned int *next_uid,
+                                                              DevParticlesT<R> dst, const unsigned int *n,
+                                                              int capacity, unsigned int *appended,
+                                                              unsigned int *overflow) {
+  pdl_wait();
+  append_block(set, next_uid, dst, n, capacity, appended, overflow, (int)blockIdx.x, (int)gridDim.x);
+}
+
+// ---- the members' step kernels of a batch ------------------------------------
+// The cell records, the copies' append and the sort of every batched member
+// in one launch each, in place of five launches per member: 32 members of
+// 5k-50k particles took 160 launches a step, most of them shorter than their
+// launch.  32 members of FP32 stores of up to 45k particles: 104 us a step
+// (records 28, append 2, histogram 9, scan 25, scatter 37) where the 160
+// launches took some 220; the step of 853 us fell to 745.  `tails` is the
+// batch's table (BatchTailT), `members` the members taken (bit k).
+//
+// Tiles: a block finds the simulation of a tile in the prefix of the
+// members' tile counts (shared memory).
+struct TilePrefix {
+  int *first;  // [n + 1]
+  int n;
+  // tiles(k) for k < n, by every thread of the block
+  template <class Tiles>
+  __device__ __forceinline__ void fill(Tiles &&tiles) {
+    for (int k = threadIdx.x; k < n; k += blockDim.x) first[k] = tiles(k);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      int run = 0;
+      for (int k = 0; k < n; ++k) {
+        const int c = first[k];
+        first[k] = run;
+        run += c;
+      }
+      first[n] = run;
+    }
+    __syncthreads();
+  }
+  __device__ __forceinline__ int find(int t) const {
+    int lo = 0, hi = n - 1;
+    while (lo < hi) {  // the last k with first[k] <= t (members without tiles are passed over)
+      const int mid = (lo + hi + 1) >> 1;
+      if (first[mid] <= t) lo = mid;
+      else hi = mid - 1;
+    }
+    return lo;
+  }
+};
+template <typename R, typename Rec>
+__global__ void __launch_bounds__(256) batch_records_kernel(const __grid_constant__ DevTables T,
+                                                            const BatchTailT<R> *tails, int n, uint64_t members) {
+  __shared__ int first[kMaxBatch + 1];
+  TilePrefix tp{first, n};
+  tp.fill([&](int k) { return (members >> k) & 1ull ? (tails[k].cells + 255) / 256 : 0; });
+  for (int t = blockIdx.x; t < first[n]; t += gridDim.x) {
+    const int k = tp.find(t), tile = t - first[k];
+    const BatchTailT<R> &b = tails[k];
+    if (tile == 0) reset_step_counters(b.counters, threadIdx.x);
+    const int c = tile * 256 + (int)threadIdx.x;
+    if (c < b.cells) cell_record(T, b.M, static_cast<Rec *>(b.records), c);
+  }
+}
+constexpr int kAppendBlocks = 8;  // per member: 32 copies a block, a step of 50k particles makes a few
+template <typename R>
+__global__ void __launch_bounds__(256) batch_append_kernel(const BatchTailT<R> *tails, uint64_t members) {
+  const int k = (int)blockIdx.x / kAppendBlocks;
+  if (!((members >> k) & 1ull)) return;
+  const BatchTailT<R> &b = tails[k];
+  append_block(b.set, b.finish.next_uid, b.src, b.finish.n, b.capacity, b.counters.appended, b.overflow,
+               (int)blockIdx.x % kAppendBlocks, kAppendBlocks);
+}
+template <typename R>
+__device__ __forceinline__ int tail_count(const BatchTailT<R> &b) {
+  const unsigned long long v = (unsigned long long)*b.finish.n + *b.counters.appended;
+  return (int)(v < (unsigned long long)b.capacity ? v : (unsigned long long)b.capacity);
+}
+// Also leaves the prefix of the members' tiles for the scatter, which ends
+// the members' steps while it runs (their counts change under it).
+template <typename R>
+__global__ void __launch_bounds__(256) batch_histogram_kernel(const BatchTailT<R> *tails, int n, uint64_t members,
+                                                              int *tile_first) {
+  __shared__ int first[kMaxBatch + 1];
+  TilePrefix tp{first, n};
+  tp.fill([&](int k) { return (members >> k) & 1ull ? max(1, (tail_count(tails[k]) + 255) / 256) : 0; });
+  if (blockIdx.x == 0)
+    for (int k = threadIdx.x; k <= n; k += blockDim.x) tile_first[k] = first[k];
+  for (int t = blockIdx.x; t < first[n]; t += gridDim.x) {
+    const int k = tp.find(t), tile = t - first[k];
+    const BatchTailT<R> &b = tails[k];
+    if (tile == 0 && threadIdx.x < 4) b.bounds[threadIdx.x] = 0ull;
+    histogram_warp(b.src.cell, b.src.meta, tail_count(b), b.nx, b.nz, b.hist, b.shift, tile * 256 + (int)threadIdx.x);
+  }
+}
+template <typename R>
+__global__ void __launch_bounds__(1024) batch_scan_kernel(const BatchTailT<R> *tails, int n, uint64_t members) {
+  __shared__ int first[kMaxBatch + 1];
+  TilePrefix tp{first, n};
+  tp.fill([&](int k) { return (members >> k) & 1ull ? (tails[k].buckets + 1023) / 1024 : 0; });
+  if ((int)blockIdx.x >= first[n]) return;
+  const int k = tp.find((int)blockIdx.x);
+  const BatchTailT<R> &b = tails[k];
+  scan_tile(b.hist, b.offsets, b.tile_sums, b.buckets, b.finish.scan_blocks, b.total, b.hist,
+            (int)blockIdx.x - first[k], first[k + 1] - first[k]);
+}
+template <typename R>
+__global__ void __launch_bounds__(256) batch_scatter_kernel(const BatchTailT<R> *tails, int n, const int *tile_first) {
+  __shared__ int first[kMaxBatch + 1];
+  for (int k = threadIdx.x; k <= n; k += blockDim.x) first[k] = tile_first[k];
+  __syncthreads();
+  const TilePrefix tp{first, n};
+  for (int t = blockIdx.x; t < first[n]; t += gridDim.x) {
+    const int k = tp.find(t), tile = t - first[k];
+    const BatchTailT<R> &b = tails[k];
+    const int count = tail_count(b);  // (this tile is not done: the member's count still stands)
+    unsigned long long mx[2] = {0, 0}, cnt[2] = {0, 0};
+    scatter_warp(b.src, b.dst, count, b.offsets, b.nx, b.nz, b.shift, b.tile_sums, tile * 256 + (int)threadIdx.x, mx,
+                 cnt);
+    scatter_bounds(mx, cnt, b.bounds);
+    __syncthreads();  // every thread has read the count, and the bounds are read from shared memory
+    if (threadIdx.x == 0) finish_step(b.finish, (unsigned)(first[k + 1] - first[k]));
   }
 }
 
@@ -1085,11 +1228,27 @@ int launch_batch_flight(const FlightCtxT<R> &F, const BatchInstT<R> *inst, int n
 }
 void launch_records_and_reset(const DevTables &T, const DevMesh &M, float4 *out, int cells, const StepCounters &z,
                               cudaStream_t s) {
-  launch_pdl(cell_records32_kernel, std::max((cells + 255) / 256, 1), 256, 0, s, T, M, out, cells, z);
+  launch_pdl(cell_records_kernel<float4>, std::max((cells + 255) / 256, 1), 256, 0, s, T, M, out, cells, z);
 }
 void launch_records_and_reset(const DevTables &T, const DevMesh &M, double2 *out, int cells, const StepCounters &z,
                               cudaStream_t s) {
-  launch_pdl(cell_records64_kernel, std::max((cells + 255) / 256, 1), 256, 0, s, T, M, out, cells, z);
+  launch_pdl(cell_records_kernel<double2>, std::max((cells + 255) / 256, 1), 256, 0, s, T, M, out, cells, z);
+}
+template <typename R>
+int launch_batch_records(const DevTables &T, const BatchTailT<R> *tails, int n, uint64_t members, int tiles,
+                         cudaStream_t s) {
+  using Rec = std::conditional_t<sizeof(R) == 4, float4, double2>;
+  batch_records_kernel<R, Rec><<<std::max(tiles, 1), 256, 0, s>>>(T, tails, n, members);
+  return cudaGetLastError() == cudaSuccess ? 0 : 1;
+}
+template <typename R>
+int launch_batch_tails(const BatchTailT<R> *tails, int n, uint64_t members, int scan_tiles, int *tile_first,
+                       int sm_count, cudaStream_t s) {
+  batch_append_kernel<R><<<n * kAppendBlocks, 256, 0, s>>>(tails, members);
+  batch_histogram_kernel<R><<<8 * sm_count, 256, 0, s>>>(tails, n, members, tile_first);
+  batch_scan_kernel<R><<<std::max(scan_tiles, 1), 1024, 0, s>>>(tails, n, members);
+  batch_scatter_kernel<R><<<8 * sm_count, 256, 0, s>>>(tails, n, tile_first);
+  return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
 template <typename R>
 void launch_append_children(const ChildSetT<R> &set, unsigned int *next_uid, const DevParticlesT<R> &dst,
@@ -1143,6 +1302,8 @@ void launch_cell_sort(const DevParticlesT<R> &src, DevCount n, const DevParticle
                                           cudaStream_t);                                                        \
   template int launch_batch_flight<R>(const FlightCtxT<R> &, const BatchInstT<R> *, int, uint64_t,             \
                                       const uint32_t *, BatchPart, unsigned int *, int, int, cudaStream_t, bool); \
+  template int launch_batch_records<R>(const DevTables &, const BatchTailT<R> *, int, uint64_t, int, cudaStream_t); \
+  template int launch_batch_tails<R>(const BatchTailT<R> *, int, uint64_t, int, int *, int, cudaStream_t);       \
   template void launch_advance_batch_steps<R>(uint32_t *, BatchInstT<R> *, int, int, cudaStream_t);           \
   template void launch_cell_sort<R>(const DevParticlesT<R> &, DevCount, const DevParticlesT<R> &, int, int, int, \
                                     unsigned int *, unsigned int *, unsigned int *, unsigned int *, int,        \

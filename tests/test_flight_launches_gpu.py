@@ -105,6 +105,42 @@ def test_holes_and_electrons_as_parts_in_a_hot_field(root, carrier):
         assert np.array_equal(engines[0][k].view(np.uint8), both.view(np.uint8)), k
 
 
+@pytest.mark.parametrize("graphs", [False, True])
+@pytest.mark.parametrize("precision", [mcb200.FLIGHT_FP64, mcb200.FLIGHT_FP32])
+def test_batch_tails_at_tile_edges(root, precision, graphs):
+    """A batch's records, appends and sorts take its members' tiles of 256
+    particles together: members of none, one, and a tile more or less one end
+    as alone, also when a member's sort buckets change between steps."""
+    counts = [257, 0, 1, 255, 256, 513]
+    engines = []
+    for m in counts:
+        pair = [box(root, m + 64, precision) for _ in range(2)]
+        if m:
+            for eng in pair:
+                eng.upload(ensemble(root, m, precision))
+        engines.append(pair)
+    dt = 1e-15 / engines[0][0].units()["time0"]
+    batch = mcb200.Batch([(pair[1], dict(dt=dt, seed=9 + k, first_step=k, self_consistent=0, poisson_every=1))
+                          for k, pair in enumerate(engines)])
+    batch.use_graphs(graphs)
+    for at, steps, bucket in ((0, 3, 1), (3, 2, 8), (5, 2, 1)):
+        for k, pair in enumerate(engines):
+            for eng in pair if k % 2 == 0 else ():
+                eng.set_sort_bucket(bucket)
+            for step in range(at, at + steps):
+                pair[0].step(k + step, 9 + k, dt)
+        batch.run(steps)
+    batch.sync()
+    for m, (alone, member) in zip(counts, engines):
+        a, b = by_uid(alone), by_uid(member)
+        assert a["uid"].size == m
+        for key in a:
+            np.testing.assert_array_equal(a[key], b[key], err_msg=f"{m} {key}")
+        ta, tb = alone.tallies(), member.tallies()
+        assert [ta[key] for key in ("events", "phonon", "impurity")] == [tb[key] for key in ("events", "phonon", "impurity")]
+    batch.close()
+
+
 def philox_block0(uid, step, seed):
     """The stream's first Philox4x32-10 block per uid (include/mcb200_rng.h), words [4, n]."""
     c = [np.zeros(len(uid), np.uint64), uid.astype(np.uint64), np.full(len(uid), step, np.uint64),
