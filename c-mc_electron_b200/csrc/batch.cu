@@ -273,8 +273,7 @@ void batch_transport(mcb200_batch *b, uint64_t early = 0) {
   const BatchPart flight = apart ? BatchPart::kFlightFirst : BatchPart::kFlight;
   if (batched) {
     if (early) {
-      ck(cudaMemsetAsync(side_ticket, 0, sizeof(unsigned int), b->side), "memset");
-      if (launch_batch_records<R>(F.T, tails, n, early, b->record_tiles, b->side) ||
+      if (launch_batch_records<R>(F.T, tails, n, early, b->record_tiles, side_ticket, 1, b->side) ||
           launch_batch_drift<R>(F, tab + (size_t)flip * n, n, early, sms, b->side))
         throw std::runtime_error("batched drift launch failed");
       ck(cudaEventRecord(b->ev_side0, b->side), "event");  // the side counter is reset, the lists are made
@@ -283,8 +282,8 @@ void batch_transport(mcb200_batch *b, uint64_t early = 0) {
         throw std::runtime_error("batched flight launch failed");
       ck(cudaEventRecord(b->ev_side, b->side), "event");
     }
-    ck(cudaMemsetAsync(b->tickets, 0, sizeof(unsigned int) * kFlightTickets, b->stream), "memset");
-    if (launch_batch_records<R>(F.T, tails, n, batched & ~early, b->record_tiles, b->stream) ||
+    if (launch_batch_records<R>(F.T, tails, n, batched & ~early, b->record_tiles, b->tickets, kFlightTickets,
+                                b->stream) ||
         launch_batch_drift<R>(F, tab + (size_t)flip * n, n, batched & ~early, sms, b->stream))
       throw std::runtime_error("batched drift launch failed");
     if (launch_batch_flight<R>(F, tab + (size_t)flip * n, n, batched & ~early, b->steps, flight, b->tickets,

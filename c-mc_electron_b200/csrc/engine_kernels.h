@@ -108,12 +108,12 @@ struct BatchTailT {
   int cells, buckets, capacity, nx, nz, shift;
 };
 // The records of the members in `members` (tiles: of 256 cells, of all
-// members); their tails in four launches (scan_tiles: of 1024 buckets, of
+// members), which also zeroes the batch's `ntickets` work tickets; their tails in four launches (scan_tiles: of 1024 buckets, of
 // all members; tile_first: device scratch of n + 1 ints).  Return 0 on
 // success.
 template <typename R>
 int launch_batch_records(const DevTables &T, const BatchTailT<R> *tails, int n, uint64_t members, int tiles,
-                         cudaStream_t s);
+                         unsigned int *tickets, int ntickets, cudaStream_t s);
 template <typename R>
 int launch_batch_tails(const BatchTailT<R> *tails, int n, uint64_t members, int scan_tiles, int *tile_first,
                        int sm_count, cudaStream_t s);

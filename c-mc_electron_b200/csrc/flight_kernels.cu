@@ -430,25 +430,58 @@ __global__ void __launch_bounds__(kFlightThreads, kFlightBlocks<R>) child_flight
 // tallies, copy buffer, dt, seed and step (FlyerT::I).  A particle's draws
 // still come from its own stream (seed, uid, step), so it flies exactly as
 // in a launch of its simulation alone.
-template <typename R, bool kChild, bool kResume>
-struct BatchIO {
-  const BatchInstT<R> *I;  // shared memory
-  const int *prefix;       // [ninst + 1], shared memory
-  int ninst;
-  __device__ __forceinline__ int find(int q) const {
-    int lo = 0, hi = ninst - 1;
+
+// The simulation of a batch's ticket or tile: the prefix of the members'
+// counts, in shared memory.  One warp reads the counts, a lane or two per
+// member: read one after another by one thread they cost 16 us a launch for
+// 32 members (a copy flight without copies took 17.3 us and takes 2.5 this way).
+struct MemberPrefix {
+  int *first;  // [n + 1]
+  int n;
+  // count(k) for k < n; by every thread of the block
+  template <class Count>
+  __device__ __forceinline__ void fill(Count &&count) {
+    static_assert(kMaxBatch <= 64, "two members a lane");
+    if (threadIdx.x < 32) {
+      const int k = (int)threadIdx.x;
+      const int a = k < n ? count(k) : 0, b = k + 32 < n ? count(k + 32) : 0;
+      int upto_a = a, upto_b = b;
+      for (int off = 1; off < 32; off <<= 1) {
+        const int ta = __shfl_up_sync(0xffffffffu, upto_a, off), tb = __shfl_up_sync(0xffffffffu, upto_b, off);
+        if (k >= off) {
+          upto_a += ta;
+          upto_b += tb;
+        }
+      }
+      upto_b += __shfl_sync(0xffffffffu, upto_a, 31);
+      if (k < n) first[k] = upto_a - a;
+      if (k + 32 < n) first[k + 32] = upto_b - b;
+      if (k == 31) first[n] = upto_b;
+    }
+    __syncthreads();
+  }
+  __device__ __forceinline__ int total() const { return first[n]; }
+  // the last k with first[k] <= t (members without a count are passed over)
+  __device__ __forceinline__ int find(int t) const {
+    int lo = 0, hi = n - 1;
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
-      if (prefix[mid] <= q) lo = mid;
+      if (first[mid] <= t) lo = mid;
       else hi = mid - 1;
     }
     return lo;
   }
+};
+
+template <typename R, bool kChild, bool kResume>
+struct BatchIO {
+  const BatchInstT<R> *I;  // shared memory
+  MemberPrefix members;
   __device__ int load(int q, FlyerT<R> &f, int &state) const {
-    const int k = find(q);
+    const int k = members.find(q);
     const BatchInstT<R> &b = I[k];
     f.I = &b;
-    const int p = q - prefix[k];
+    const int p = q - members.first[k];
     if constexpr (kChild) return ChildIO<R>{b.in, b.step}.load(p, f, state);
     else return StoreIO<R, kResume>{b.P, b.lists, b.dt, b.step}.load(p, f, state);
   }
@@ -486,37 +519,27 @@ __global__ void __launch_bounds__(kFlightThreads, kFlightBlocks<R>) batch_flight
                                                                              unsigned int *ticket) {
   extern __shared__ __align__(16) unsigned char batch_smem[];
   __shared__ SymSmemT<R> S;
-  const BatchInstT<R> *I;
-  int *prefix;
+  MemberPrefix prefix{reinterpret_cast<int *>(batch_smem + (kSmemTable ? ninst * sizeof(BatchInstT<R>) : 0)), ninst};
+  prefix.fill([&](int k) {
+    if (!((members >> k) & 1ull)) return 0;
+    return kChild ? min((int)*inst[k].in.count, inst[k].in.capacity) : (int)inst[k].lists.count[kResume ? 1 : 0];
+  });
+  const int total = prefix.total();
+  if (total == 0) return;
+  const BatchInstT<R> *I = inst;
   if constexpr (kSmemTable) {
     BatchInstT<R> *T = reinterpret_cast<BatchInstT<R> *>(batch_smem);
-    prefix = reinterpret_cast<int *>(T + ninst);
     static_assert(sizeof(BatchInstT<R>) % 8 == 0, "the table is copied in 8-byte words");
     const unsigned long long *src = reinterpret_cast<const unsigned long long *>(inst);
     unsigned long long *dst = reinterpret_cast<unsigned long long *>(T);
     const int words = ninst * (int)(sizeof(BatchInstT<R>) / 8);
     for (int w = threadIdx.x; w < words; w += blockDim.x) dst[w] = src[w];
     __syncthreads();
-    if (threadIdx.x == 0)
-      for (int k = 0; k < ninst; ++k) T[k].step = steps[k];
+    for (int k = threadIdx.x; k < ninst; k += blockDim.x) T[k].step = steps[k];
     I = T;
-  } else {
-    prefix = reinterpret_cast<int *>(batch_smem);
-    I = inst;
   }
-  if (threadIdx.x == 0) {
-    int run = 0;
-    for (int k = 0; k < ninst; ++k) {
-      prefix[k] = run;
-      if ((members >> k) & 1ull)
-        run += kChild ? min((int)*I[k].in.count, I[k].in.capacity) : (int)I[k].lists.count[kResume ? 1 : 0];
-    }
-    prefix[ninst] = run;
-  }
-  load_sym(S, F.T);  // ends with a barrier: the table and prefix are visible
-  const int total = prefix[ninst];
-  if (total == 0) return;
-  fly_interleaved<R, false, kDraws>(F, S, BatchIO<R, kChild, kResume>{I, prefix, ninst}, total, ticket);
+  load_sym(S, F.T);  // ends with a barrier: the table is visible
+  fly_interleaved<R, false, kDraws>(F, S, BatchIO<R, kChild, kResume>{I, prefix}, total, ticket);
 }
 
 // The drift pass of many simulations in one launch: the blocks take 256
@@ -528,24 +551,13 @@ __global__ void __launch_bounds__(kFlightThreads, kDriftBlocks<R>) batch_drift_k
   __shared__ SymSmemT<R> S;
   __shared__ int first[kMaxBatch + 1];  // the tiles before each simulation's
   for (int i = threadIdx.x; i < 48; i += blockDim.x) S.sym[i] = F.T.sym_packed[i];
-  for (int k = threadIdx.x; k < ninst; k += blockDim.x)
-    first[k] = (members >> k) & 1ull
-                   ? (min((int)*inst[k].n, inst[k].capacity) + kFlightThreads - 1) / kFlightThreads : 0;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int run = 0;
-    for (int k = 0; k < ninst; ++k) {
-      const int c = first[k];
-      first[k] = run;
-      run += c;
-    }
-    first[ninst] = run;
-  }
-  __syncthreads();
-  const int tiles = first[ninst];
+  MemberPrefix prefix{first, ninst};
+  prefix.fill([&](int k) {
+    return (members >> k) & 1ull ? (min((int)*inst[k].n, inst[k].capacity) + kFlightThreads - 1) / kFlightThreads : 0;
+  });
+  const int tiles = prefix.total();
   for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
-    int k = 0;  // uniform over the block
-    while (first[k + 1] <= t) ++k;
+    const int k = prefix.find(t);  // uniform over the block
     const BatchInstT<R> &b = inst[k];
     const int count = min((int)*b.n, b.capacity);
     const int p = (t - first[k]) * kFlightThreads + (int)threadIdx.x;
@@ -939,43 +951,13 @@ __global__ void __launch_bounds__(256) append_children_kernel(ChildSetT<R> set, 
 // (records 28, append 2, histogram 9, scan 25, scatter 37) where the 160
 // launches took some 220; the step of 853 us fell to 745.  `tails` is the
 // batch's table (BatchTailT), `members` the members taken (bit k).
-//
-// Tiles: a block finds the simulation of a tile in the prefix of the
-// members' tile counts (shared memory).
-struct TilePrefix {
-  int *first;  // [n + 1]
-  int n;
-  // tiles(k) for k < n, by every thread of the block
-  template <class Tiles>
-  __device__ __forceinline__ void fill(Tiles &&tiles) {
-    for (int k = threadIdx.x; k < n; k += blockDim.x) first[k] = tiles(k);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int run = 0;
-      for (int k = 0; k < n; ++k) {
-        const int c = first[k];
-        first[k] = run;
-        run += c;
-      }
-      first[n] = run;
-    }
-    __syncthreads();
-  }
-  __device__ __forceinline__ int find(int t) const {
-    int lo = 0, hi = n - 1;
-    while (lo < hi) {  // the last k with first[k] <= t (members without tiles are passed over)
-      const int mid = (lo + hi + 1) >> 1;
-      if (first[mid] <= t) lo = mid;
-      else hi = mid - 1;
-    }
-    return lo;
-  }
-};
 template <typename R, typename Rec>
 __global__ void __launch_bounds__(256) batch_records_kernel(const __grid_constant__ DevTables T,
-                                                            const BatchTailT<R> *tails, int n, uint64_t members) {
+                                                            const BatchTailT<R> *tails, int n, uint64_t members,
+                                                            unsigned int *tickets, int ntickets) {
   __shared__ int first[kMaxBatch + 1];
-  TilePrefix tp{first, n};
+  if (blockIdx.x == 0 && (int)threadIdx.x < ntickets) tickets[threadIdx.x] = 0u;
+  MemberPrefix tp{first, n};
   tp.fill([&](int k) { return (members >> k) & 1ull ? (tails[k].cells + 255) / 256 : 0; });
   for (int t = blockIdx.x; t < first[n]; t += gridDim.x) {
     const int k = tp.find(t), tile = t - first[k];
@@ -1005,7 +987,7 @@ template <typename R>
 __global__ void __launch_bounds__(256) batch_histogram_kernel(const BatchTailT<R> *tails, int n, uint64_t members,
                                                               int *tile_first) {
   __shared__ int first[kMaxBatch + 1];
-  TilePrefix tp{first, n};
+  MemberPrefix tp{first, n};
   tp.fill([&](int k) { return (members >> k) & 1ull ? max(1, (tail_count(tails[k]) + 255) / 256) : 0; });
   if (blockIdx.x == 0)
     for (int k = threadIdx.x; k <= n; k += blockDim.x) tile_first[k] = first[k];
@@ -1019,7 +1001,7 @@ __global__ void __launch_bounds__(256) batch_histogram_kernel(const BatchTailT<R
 template <typename R>
 __global__ void __launch_bounds__(1024) batch_scan_kernel(const BatchTailT<R> *tails, int n, uint64_t members) {
   __shared__ int first[kMaxBatch + 1];
-  TilePrefix tp{first, n};
+  MemberPrefix tp{first, n};
   tp.fill([&](int k) { return (members >> k) & 1ull ? (tails[k].buckets + 1023) / 1024 : 0; });
   if ((int)blockIdx.x >= first[n]) return;
   const int k = tp.find((int)blockIdx.x);
@@ -1032,7 +1014,7 @@ __global__ void __launch_bounds__(256) batch_scatter_kernel(const BatchTailT<R> 
   __shared__ int first[kMaxBatch + 1];
   for (int k = threadIdx.x; k <= n; k += blockDim.x) first[k] = tile_first[k];
   __syncthreads();
-  const TilePrefix tp{first, n};
+  const MemberPrefix tp{first, n};
   for (int t = blockIdx.x; t < first[n]; t += gridDim.x) {
     const int k = tp.find(t), tile = t - first[k];
     const BatchTailT<R> &b = tails[k];
@@ -1236,9 +1218,9 @@ void launch_records_and_reset(const DevTables &T, const DevMesh &M, double2 *out
 }
 template <typename R>
 int launch_batch_records(const DevTables &T, const BatchTailT<R> *tails, int n, uint64_t members, int tiles,
-                         cudaStream_t s) {
+                         unsigned int *tickets, int ntickets, cudaStream_t s) {
   using Rec = std::conditional_t<sizeof(R) == 4, float4, double2>;
-  batch_records_kernel<R, Rec><<<std::max(tiles, 1), 256, 0, s>>>(T, tails, n, members);
+  batch_records_kernel<R, Rec><<<std::max(tiles, 1), 256, 0, s>>>(T, tails, n, members, tickets, ntickets);
   return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
 template <typename R>
@@ -1302,7 +1284,8 @@ void launch_cell_sort(const DevParticlesT<R> &src, DevCount n, const DevParticle
                                           cudaStream_t);                                                        \
   template int launch_batch_flight<R>(const FlightCtxT<R> &, const BatchInstT<R> *, int, uint64_t,             \
                                       const uint32_t *, BatchPart, unsigned int *, int, int, cudaStream_t, bool); \
-  template int launch_batch_records<R>(const DevTables &, const BatchTailT<R> *, int, uint64_t, int, cudaStream_t); \
+  template int launch_batch_records<R>(const DevTables &, const BatchTailT<R> *, int, uint64_t, int,            \
+                                       unsigned int *, int, cudaStream_t);                                      \
   template int launch_batch_tails<R>(const BatchTailT<R> *, int, uint64_t, int, int *, int, cudaStream_t);       \
   template void launch_advance_batch_steps<R>(uint32_t *, BatchInstT<R> *, int, int, cudaStream_t);           \
   template void launch_cell_sort<R>(const DevParticlesT<R> &, DevCount, const DevParticlesT<R> &, int, int, int, \
