@@ -668,25 +668,51 @@ __global__ void cell_histogram(const uint32_t *cell, const uint32_t *meta, DevCo
 
 // Exclusive scan of `count` values, single pass per 1024-wide tile plus a
 // tile-sum pass (cells are at most ~10^6, so three small launches suffice).
-// Exclusive scan of the tile sums in place by one block of 1024 threads,
-// 1024 tiles per pass with the running total carried between passes.
+// Blocks of 256 threads, four consecutive values a thread: shuffles within
+// the warps and one exchange of the warps' sums (a block of 1024 threads that
+// doubled its reach in shared memory met 20 barriers a tile: 1M buckets 25.5
+// us, here 13.1; 16k buckets 5.6, here 3.1).
+constexpr int kScanThreads = 256;
+constexpr int kScanTile = 4 * kScanThreads;
+// The sum of the values of the threads before this one; all: of the block's.
+__device__ __forceinline__ unsigned int scan_block(unsigned int mine, unsigned int *all) {
+  __shared__ unsigned int sums[kScanThreads / 32];
+  const int lane = (int)(threadIdx.x & 31u), warp = (int)(threadIdx.x >> 5);
+  unsigned int upto = mine;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const unsigned int t = __shfl_up_sync(0xffffffffu, upto, off);
+    if (lane >= off) upto += t;
+  }
+  if (lane == 31) sums[warp] = upto;
+  __syncthreads();
+  unsigned int before = 0, run = 0;
+#pragma unroll
+  for (int w = 0; w < kScanThreads / 32; ++w) {
+    if (w == warp) before = run;
+    run += sums[w];
+  }
+  __syncthreads();  // the sums are reused by the next call
+  *all = run;
+  return before + upto - mine;
+}
+// Exclusive scan of the tile sums in place by one block, 1024 tiles per pass
+// with the running total carried between passes.
 __device__ void scan_tile_sums_block(unsigned int *tile_sums, int ntiles, unsigned int *total) {
-  __shared__ unsigned int s[1024];
   unsigned int carry = 0;
-  for (int base = 0; base < ntiles; base += 1024) {
-    const int t = base + threadIdx.x;
-    const unsigned int v = t < ntiles ? __ldcg(tile_sums + t) : 0u;  // written by other blocks: read at L2
-    s[threadIdx.x] = v;
-    __syncthreads();
-    for (int off = 1; off < 1024; off <<= 1) {
-      const unsigned int a = threadIdx.x >= (unsigned)off ? s[threadIdx.x - off] : 0u;
-      __syncthreads();
-      s[threadIdx.x] += a;
-      __syncthreads();
+  for (int base = 0; base < ntiles; base += kScanTile) {
+    const int t = base + 4 * (int)threadIdx.x;
+    unsigned int v[4], all;
+#pragma unroll
+    for (int e = 0; e < 4; ++e)  // other blocks' writes: read at L2
+      v[e] = t + e < ntiles ? __ldcg(tile_sums + t + e) : 0u;
+    unsigned int at = carry + scan_block(v[0] + v[1] + v[2] + v[3], &all);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      if (t + e < ntiles) tile_sums[t + e] = at;
+      at += v[e];
     }
-    if (t < ntiles) tile_sums[t] = carry + s[threadIdx.x] - v;
-    carry += s[1023];
-    __syncthreads();
+    carry += all;
   }
   if (threadIdx.x == 0) *total = carry;
 }
@@ -698,23 +724,37 @@ __device__ void scan_tile_sums_block(unsigned int *tile_sums, int ntiles, unsign
 // keeps its histogram zero between sorts, so no memset precedes it).
 __device__ void scan_tile(const unsigned int *in, unsigned int *out, unsigned int *tile_sums, int n,
                           unsigned int *blocks, unsigned int *total, unsigned int *clear, int tile, int ntiles) {
-  __shared__ unsigned int s[1024];
   __shared__ bool last;
-  const int i = tile * 1024 + threadIdx.x;
-  const unsigned int v = i < n ? in[i] : 0u;
-  if (clear && i < n) clear[i] = 0u;
-  s[threadIdx.x] = v;
-  __syncthreads();
-  for (int off = 1; off < 1024; off <<= 1) {
-    unsigned int t = threadIdx.x >= (unsigned)off ? s[threadIdx.x - off] : 0u;
-    __syncthreads();
-    s[threadIdx.x] += t;
-    __syncthreads();
+  const int i = tile * kScanTile + 4 * (int)threadIdx.x;
+  // 16-byte accesses where the arrays start on 16 bytes and all four values exist
+  const bool whole =
+      i + 3 < n && (((uintptr_t)in | (uintptr_t)out | (uintptr_t)clear) & 15) == 0;
+  unsigned int v[4] = {0u, 0u, 0u, 0u}, all;
+  if (whole) {
+    const uint4 q = *reinterpret_cast<const uint4 *>(in + i);
+    v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+    if (clear) *reinterpret_cast<uint4 *>(clear + i) = make_uint4(0u, 0u, 0u, 0u);
+  } else {
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (i + e < n) {
+        v[e] = in[i + e];
+        if (clear) clear[i + e] = 0u;
+      }
   }
-  if (i < n) out[i] = s[threadIdx.x] - v;
-  if (threadIdx.x == 1023) tile_sums[tile] = s[1023];
+  const unsigned int at = scan_block(v[0] + v[1] + v[2] + v[3], &all);
+  const uint4 o = make_uint4(at, at + v[0], at + v[0] + v[1], at + v[0] + v[1] + v[2]);
+  if (whole) {
+    *reinterpret_cast<uint4 *>(out + i) = o;
+  } else {
+    if (i < n) out[i] = o.x;
+    if (i + 1 < n) out[i + 1] = o.y;
+    if (i + 2 < n) out[i + 2] = o.z;
+    if (i + 3 < n) out[i + 3] = o.w;
+  }
+  if (threadIdx.x == 0) tile_sums[tile] = all;
   if (blocks == nullptr) return;  // uniform over the grid
-  if (threadIdx.x == 1023) {
+  if (threadIdx.x == 0) {
     __threadfence();
     last = atomicAdd(blocks, 1u) == (unsigned)ntiles - 1u;
   }
@@ -724,12 +764,12 @@ __device__ void scan_tile(const unsigned int *in, unsigned int *out, unsigned in
   scan_tile_sums_block(tile_sums, ntiles, total);
   if (threadIdx.x == 0) *blocks = 0u;
 }
-__global__ void scan_tiles(const unsigned int *in, unsigned int *out, unsigned int *tile_sums, int n,
+__global__ void __launch_bounds__(kScanThreads) scan_tiles(const unsigned int *in, unsigned int *out, unsigned int *tile_sums, int n,
                            unsigned int *blocks, unsigned int *total, unsigned int *clear) {
   pdl_wait();
   scan_tile(in, out, tile_sums, n, blocks, total, clear, (int)blockIdx.x, (int)gridDim.x);
 }
-__global__ void scan_tile_sums(unsigned int *tile_sums, int ntiles, unsigned int *total) {
+__global__ void __launch_bounds__(kScanThreads) scan_tile_sums(unsigned int *tile_sums, int ntiles, unsigned int *total) {
   scan_tile_sums_block(tile_sums, ntiles, total);
 }
 __global__ void scan_add(unsigned int *out, const unsigned int *tile_sums, int n) {
@@ -947,9 +987,9 @@ __global__ void __launch_bounds__(256) append_children_kernel(ChildSetT<R> set, 
 // The cell records, the copies' append and the sort of every batched member
 // in one launch each, in place of five launches per member: 32 members of
 // 5k-50k particles took 160 launches a step, most of them shorter than their
-// launch.  32 members of FP32 stores of up to 45k particles: 104 us a step
-// (records 28, append 2, histogram 9, scan 25, scatter 37) where the 160
-// launches took some 220; the step of 853 us fell to 745.  `tails` is the
+// launch.  32 members of FP32 stores of up to 50k particles: 89 us a step
+// (records 27, append 2, histogram 10, scan 13, scatter 37) where the 160
+// launches took some 220.  `tails` is the
 // batch's table (BatchTailT), `members` the members taken (bit k).
 template <typename R, typename Rec>
 __global__ void __launch_bounds__(256) batch_records_kernel(const __grid_constant__ DevTables T,
@@ -999,7 +1039,7 @@ __global__ void __launch_bounds__(256) batch_histogram_kernel(const BatchTailT<R
   }
 }
 template <typename R>
-__global__ void __launch_bounds__(1024) batch_scan_kernel(const BatchTailT<R> *tails, int n, uint64_t members) {
+__global__ void __launch_bounds__(kScanThreads) batch_scan_kernel(const BatchTailT<R> *tails, int n, uint64_t members) {
   __shared__ int first[kMaxBatch + 1];
   MemberPrefix tp{first, n};
   tp.fill([&](int k) { return (members >> k) & 1ull ? (tails[k].buckets + 1023) / 1024 : 0; });
@@ -1228,7 +1268,7 @@ int launch_batch_tails(const BatchTailT<R> *tails, int n, uint64_t members, int 
                        int sm_count, cudaStream_t s) {
   batch_append_kernel<R><<<n * kAppendBlocks, 256, 0, s>>>(tails, members);
   batch_histogram_kernel<R><<<8 * sm_count, 256, 0, s>>>(tails, n, members, tile_first);
-  batch_scan_kernel<R><<<std::max(scan_tiles, 1), 1024, 0, s>>>(tails, n, members);
+  batch_scan_kernel<R><<<std::max(scan_tiles, 1), kScanThreads, 0, s>>>(tails, n, members);
   batch_scatter_kernel<R><<<8 * sm_count, 256, 0, s>>>(tails, n, tile_first);
   return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
@@ -1241,8 +1281,8 @@ void launch_append_children(const ChildSetT<R> &set, unsigned int *next_uid, con
 void launch_exclusive_scan(const unsigned int *in, unsigned int *out, unsigned int *tile_sums, unsigned int *total,
                            int n, cudaStream_t s) {
   const int tiles = (n + 1023) / 1024;
-  scan_tiles<<<tiles, 1024, 0, s>>>(in, out, tile_sums, n, nullptr, nullptr, nullptr);
-  scan_tile_sums<<<1, 1024, 0, s>>>(tile_sums, tiles, total);
+  scan_tiles<<<tiles, kScanThreads, 0, s>>>(in, out, tile_sums, n, nullptr, nullptr, nullptr);
+  scan_tile_sums<<<1, kScanThreads, 0, s>>>(tile_sums, tiles, total);
   scan_add<<<tiles, 1024, 0, s>>>(out, tile_sums, n);
 }
 template <typename R>
@@ -1257,15 +1297,15 @@ void launch_cell_sort(const DevParticlesT<R> &src, DevCount n, const DevParticle
     // clears the histogram), the tile prefixes added by the scatter, the
     // step ended by its last block
     launch_pdl(cell_histogram, grid, 256, 0, s, src.cell, src.meta, n, nx, nz, hist, shift, bounds);
-    launch_pdl(scan_tiles, tiles, 1024, 0, s, (const unsigned int *)hist, offsets, tile_sums, buckets,
+    launch_pdl(scan_tiles, tiles, kScanThreads, 0, s, (const unsigned int *)hist, offsets, tile_sums, buckets,
                finish.scan_blocks, total, hist);
     launch_pdl(cell_scatter<R>, grid, 256, 0, s, src, n, dst, offsets, nx, nz, shift, bounds, finish, tile_sums);
     return;
   }
   cudaMemsetAsync(hist, 0, sizeof(unsigned int) * buckets, s);
   cell_histogram<<<grid, 256, 0, s>>>(src.cell, src.meta, n, nx, nz, hist, shift, bounds);
-  scan_tiles<<<tiles, 1024, 0, s>>>(hist, offsets, tile_sums, buckets, nullptr, nullptr, nullptr);
-  scan_tile_sums<<<1, 1024, 0, s>>>(tile_sums, tiles, total);
+  scan_tiles<<<tiles, kScanThreads, 0, s>>>(hist, offsets, tile_sums, buckets, nullptr, nullptr, nullptr);
+  scan_tile_sums<<<1, kScanThreads, 0, s>>>(tile_sums, tiles, total);
   scan_add<<<tiles, 1024, 0, s>>>(offsets, tile_sums, buckets);
   cell_scatter<R><<<grid, 256, 0, s>>>(src, n, dst, offsets, nx, nz, shift, bounds, finish, nullptr);
 }

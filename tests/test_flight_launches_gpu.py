@@ -35,12 +35,12 @@ def root(cases):
     return cases.tables_owner()
 
 
-def box(root, capacity, precision, field=1e7, donor=DONOR):
+def box(root, capacity, precision, field=1e7, donor=DONOR, dims=(NX, NY, NZ)):
     eng = mcb200.Engine(max_particles=capacity, precision=precision, like=root)
     u = eng.units()
     h = CELL_M / u["spr0"]
-    eng.set_mesh(np.arange(NX + 1) * h, np.arange(NY + 1) * h, np.arange(NZ + 1) * h)
-    eng.set_cells(motion_rules(NX, NY, NZ), np.full(NX * NY * NZ, donor / u["conc0"]))
+    eng.set_mesh(*(np.arange(d + 1) * h for d in dims))
+    eng.set_cells(motion_rules(*dims), np.full(int(np.prod(dims)), donor / u["conc0"]))
     eng.set_fields(*uniform_fields(eng, field, DONOR))
     return eng
 
@@ -139,6 +139,27 @@ def test_batch_tails_at_tile_edges(root, precision, graphs):
         ta, tb = alone.tallies(), member.tallies()
         assert [ta[key] for key in ("events", "phonon", "impurity")] == [tb[key] for key in ("events", "phonon", "impurity")]
     batch.close()
+
+
+@pytest.mark.parametrize("bucket", [1, 4])
+@pytest.mark.parametrize("dims", [(1, 1, 1), (11, 31, 3), (32, 32, 1), (41, 25, 1), (129, 128, 64)])
+def test_step_sorts_the_store(root, dims, bucket):
+    """The step's sort over 1 to 1,056,768 buckets: tiles of 1024 (one short by
+    one, full, one more by one) and more than 1024 tiles."""
+    cells, n = int(np.prod(dims)), 20000
+    eng = box(root, n + 64, mcb200.FLIGHT_FP64, dims=dims)
+    eng.set_sort_bucket(bucket)
+    rng = np.random.default_rng(cells)
+    eng.seed(rng.integers(0, cells, n), np.full(n, -1e-3), 0, 5)
+    before = np.sort(eng.download()["uid"])
+    for step in range(2):
+        eng.step(step, 7, 1e-16 / eng.units()["time0"])
+    p = eng.download()
+    i, j, k = (p[a].astype(np.int64) for a in ("i", "j", "k"))
+    keys = ((j * dims[0] + i) * dims[2] + k) // bucket
+    assert before.size == n and np.array_equal(np.sort(p["uid"]), before)
+    assert keys.min() >= 0 and keys.max() <= (cells - 1) // bucket
+    assert np.all(np.diff(keys) >= 0)
 
 
 def philox_block0(uid, step, seed):
