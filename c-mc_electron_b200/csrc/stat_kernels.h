@@ -14,7 +14,8 @@ struct StatScales {
 };
 
 struct StatBuffers {
-  long long *node = nullptr;                 // [2 types][5: qvx qvy qvz q qE][nodes]
+  long long *node = nullptr;                 // [2 types][nodes][5: qvx qvy qvz q qE]
+  double *values = nullptr;                  // [nodes] fixed-point sums' values on their way to the host
   unsigned long long *cell_count = nullptr;  // [cells]
   double *pot_sum = nullptr;                 // [nodes]
   double *qc_pot_sum = nullptr;              // [nodes] the electrons' potential (quantum-corrected when on)
@@ -23,7 +24,14 @@ struct StatBuffers {
 
 template <typename R>
 void launch_statistic(const DevParticlesT<R> &P, DevCount n, const DevMesh &M, const DevTables &T, const StatScales &S,
-                      const StatBuffers &B, int grid, cudaStream_t s);
+                      const StatBuffers &B, int sm_count, cudaStream_t s);
+// out[p] = (64-bit whole number at sums + stride * p) / scale, p < n.
+void launch_fixed_values(int n, const void *sums, int stride, double scale, double *out, cudaStream_t s);
+// The counters (as whole numbers), contact[kMaxContacts][6], lcurrent[rows]
+// and rcurrent[rows] of y (values) to out, pinned host memory for up to
+// kSmallTallies doubles.
+constexpr int kSmallTallies = kCntNumCounters + kMaxContacts * 6 + 2 * 1024;  // a mesh has at most 1024 rows of nodes
+void launch_small_tallies(const DevTallies &y, int rows, double *out, cudaStream_t s);
 void launch_add_potential(int nodes, const double *pot, double *sum, cudaStream_t s);
 
 // Induced (Ramo-Shockley) current of one contact over the store: the sum
