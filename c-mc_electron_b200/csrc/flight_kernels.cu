@@ -36,7 +36,7 @@ namespace mcb200 {
 template <typename R>
 constexpr int kFlightBlocks = sizeof(R) == 4 ? MCB200_FLIGHT_BLOCKS_F32 : MCB200_FLIGHT_BLOCKS_F64;
 // The flight without draws fits FP32 in 80 registers (2M electrons: 610 us at
-// two blocks per SM, 560 at three).
+// two blocks per SM, 541 at three).
 template <typename R>
 constexpr int kNoDrawBlocks = sizeof(R) == 4 ? 3 : MCB200_FLIGHT_BLOCKS_F64;
 // Threads per block of the flight kernels (a tuning define like the above).
@@ -347,6 +347,14 @@ __device__ __forceinline__ int drift_block(const FlightCtxT<R> &F, FlyerT<R> &f,
   return 0;
 }
 
+// The warp's particles that drifted to the step's end: a pass of the event
+// loop each.
+__device__ __forceinline__ void count_drifted(const DevTallies &Y, unsigned int done) {
+  if ((threadIdx.x & 31u) != 0 || done == 0) return;
+  atomicAdd(&Y.counters[kCntEvents], (unsigned long long)done);
+  if constexpr (MCB200_FLIGHT_EVENT_STATS != 0) atomicAdd(&Y.counters[kStatStepEnd], (unsigned long long)done);
+}
+
 // Places the block's marked threads: each gets a consecutive index from *counter.
 __device__ __forceinline__ unsigned place_in_list(bool mine, unsigned int *counter) {
   __shared__ unsigned warp_base[kFlightThreads / 32 + 1];
@@ -391,7 +399,7 @@ __global__ void __launch_bounds__(kFlightThreads, kDriftBlocks<R>) drift_kernel(
     if (unfinished) list[at] = (uint32_t)p;
   }
   done = __reduce_add_sync(0xffffffffu, done);
-  if ((threadIdx.x & 31u) == 0 && done) atomicAdd(&F.Y.counters[kCntEvents], (unsigned long long)done);
+  count_drifted(F.Y, done);
 }
 
 template <typename R, bool kDraws, bool kResume>
@@ -566,7 +574,7 @@ __global__ void __launch_bounds__(kFlightThreads, kDriftBlocks<R>) batch_drift_k
     bool unfinished;
     const StoreIO<R, false> io{b.P, FlightListsT<R>{}, b.dt, b.step};
     const unsigned done = __reduce_add_sync(0xffffffffu, drift_block(F, f, io, p, p < count, unfinished));
-    if ((threadIdx.x & 31u) == 0 && done) atomicAdd(&b.Y.counters[kCntEvents], (unsigned long long)done);
+    count_drifted(b.Y, done);
     const unsigned at = place_in_list(unfinished, b.lists.count);
     if (unfinished) b.lists.list[at] = (uint32_t)p;
   }

@@ -296,6 +296,8 @@ __device__ __forceinline__ void FlyerT<R>::final_states(unsigned owners) {
           }
           at = first + q;
         }
+        if constexpr (MCB200_FLIGHT_EVENT_STATS != 0)
+          if ((int)lane == src) atomicAdd(&I->Y.counters[kStatStateTries], (unsigned long long)tries);
         real = tries < kMaxStateTries;
         if (real) {
           look_ahead();
