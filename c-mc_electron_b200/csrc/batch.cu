@@ -42,6 +42,7 @@ struct mcb200_batch {
   void *tables = nullptr;          // device: [6][n] BatchInstT (main flight x 2 parities, 4 copy generations)
   void *tails = nullptr;           // device: [2][n] BatchTailT, by store parity
   int *tile_first = nullptr;       // device: [n + 1]
+  unsigned int *counts = nullptr;  // pinned: [n][3], the members' device counts
   int record_tiles = 0, scan_tiles = 0;  // of all members
   uint32_t *steps = nullptr;       // device: step number of each member
   unsigned int *tickets = nullptr;  // device: work counters of the batched launches (main, 4 copy generations, side)
@@ -77,6 +78,7 @@ struct mcb200_batch {
     if (tickets) cudaFree(tickets);
     if (tails) cudaFree(tails);
     if (tile_first) cudaFree(tile_first);
+    if (counts) cudaFreeHost(counts);
     if (ev_flight) cudaEventDestroy(ev_flight);
     for (cudaEvent_t e : ev_member)
       if (e) cudaEventDestroy(e);
@@ -535,6 +537,7 @@ int mcb200_batch_create(mcb200_ctx *const *ctxs, const mcb200_batch_member *memb
                                                                                  : sizeof(BatchTailT<double>))),
        "cudaMalloc");
     ck(cudaMalloc(&b->tile_first, (n + 1) * sizeof(int)), "cudaMalloc");
+    ck(cudaMallocHost(&b->counts, 3 * (size_t)n * sizeof(unsigned int)), "cudaMallocHost");
     std::vector<uint32_t> first_steps(n);
     for (int k = 0; k < n; ++k) first_steps[k] = members[k].first_step;
     b->member_step = first_steps;
@@ -736,10 +739,18 @@ int mcb200_batch_sync(mcb200_batch *b) {
   try {
     ck(cudaSetDevice(b->device), "cudaSetDevice");
     ck(cudaStreamSynchronize(b->stream), "sync");
-    for (mcb200_ctx *c : b->m) {
-      ck(cudaStreamSynchronize(c->stream), "sync");
-      pull_counts(c);
+    for (mcb200_ctx *c : b->m) ck(cudaStreamSynchronize(c->stream), "sync");
+    if (b->steps_done > 0) {  // the tables hold the members' counts
+      const int n = (int)b->m.size();
+      if (b->precision == MCB200_FLIGHT_FP32
+              ? launch_batch_counts(static_cast<const BatchTailT<float> *>(b->tails), n, b->counts, b->stream)
+              : launch_batch_counts(static_cast<const BatchTailT<double> *>(b->tails), n, b->counts, b->stream))
+        throw std::runtime_error("batch counts launch failed");
+      ck(cudaStreamSynchronize(b->stream), "sync");
+      for (int k = 0; k < n; ++k)
+        if (b->m[k]->n_stale) take_counts(b->m[k], b->counts + 3 * k);
     }
+    for (mcb200_ctx *c : b->m) pull_counts(c);  // (reports a store that was full)
     return MCB200_OK;
   } catch (const CapacityError &e) {
     return bfail(b, MCB200_ERR_CAPACITY, e.what());

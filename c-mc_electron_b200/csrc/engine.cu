@@ -37,6 +37,17 @@ __global__ void set_counts_kernel(unsigned int *d, unsigned int n, unsigned int 
   }
 }
 
+// The device counts (n, next uid, store-full flag) read into v.
+void take_counts(mcb200_ctx *c, const unsigned int *v) {
+  c->n = v[0];
+  c->next_uid = v[1];
+  c->n_stale = false;
+  if (v[2]) {
+    ck(cudaMemsetAsync(c->dev_counts + 2, 0, sizeof(unsigned int), c->stream), "memset");
+    c->overflow_pending = true;
+  }
+}
+
 // Host copies of the device counts, after the stream has drained (only when
 // a step may have changed them).  A store-full flag raised by a step is
 // reported here, once.
@@ -45,13 +56,7 @@ void pull_counts(mcb200_ctx *c) {
     ck(cudaMemcpyAsync(c->h_pinned + 32, c->dev_counts, 3 * sizeof(unsigned int), cudaMemcpyDeviceToHost, c->stream),
        "count");
     ck(cudaStreamSynchronize(c->stream), "sync");
-    c->n = c->h_pinned[32];
-    c->next_uid = c->h_pinned[33];
-    c->n_stale = false;
-    if (c->h_pinned[34]) {
-      ck(cudaMemsetAsync(c->dev_counts + 2, 0, sizeof(unsigned int), c->stream), "memset");
-      c->overflow_pending = true;
-    }
+    take_counts(c, c->h_pinned + 32);
   }
   if (c->overflow_pending) {
     c->overflow_pending = false;
@@ -566,8 +571,8 @@ void init_device_context(mcb200_ctx *c, size_t max_particles) {
   c->sink_count = dalloc<unsigned int>(1, c->owned);
   ck(cudaMemsetAsync(c->dev_counts, 0, 4 * sizeof(unsigned int), c->stream), "memset");
   ck(cudaMemsetAsync(c->dev_psteps, 0, sizeof(unsigned long long), c->stream), "memset");
-  ck(cudaMallocHost(&c->h_pinned, 64 * sizeof(unsigned int)), "cudaMallocHost");
-  ck(cudaMallocHost(&c->h_scratch, (16 + kSmallTallies) * sizeof(double)), "cudaMallocHost");
+  ck(cudaMallocHost(&c->h_scratch, (16 + kSmallTallies) * sizeof(double) + 64 * sizeof(unsigned int)), "cudaMallocHost");
+  c->h_pinned = reinterpret_cast<unsigned int *>(c->h_scratch + 16 + kSmallTallies);
   ck(cudaMemsetAsync(c->y.counters, 0, sizeof(unsigned long long) * kCntNumCounters, c->stream), "memset");
   ck(cudaMemsetAsync(c->y.contact, 0, sizeof(long long) * kMaxContacts * 6, c->stream), "memset");
   ck(cudaStreamSynchronize(c->stream), "sync");
@@ -781,10 +786,10 @@ int mcb200_set_mesh(mcb200_ctx *c, int nx, int ny, int nz, const double *lx, con
     c->y.heat_e = dalloc<long long>(nodes, c->mesh_owned);
     c->y.heat_h = dalloc<long long>(nodes, c->mesh_owned);
     c->cell32 = dalloc<float4>(cells * 3, c->mesh_owned);
-    c->cell64 = dalloc<double2>(cells * 3, c->mesh_owned);
+    c->cell64 = reinterpret_cast<double2 *>(c->cell32);  // a step makes the records of its precision
     c->sb.nodes = (int)nodes;
-    c->sb.node = dalloc<long long>(nodes * 10, c->mesh_owned);
-    c->sb.values = dalloc<double>(nodes, c->mesh_owned);
+    c->sb.node = dalloc<long long>(nodes * 11, c->mesh_owned);
+    c->sb.values = reinterpret_cast<double *>(c->sb.node + nodes * 10);
     c->sb.cell_count = dalloc<unsigned long long>(cells, c->mesh_owned);
     c->sb.pot_sum = dalloc<double>(nodes, c->mesh_owned);
     c->sb.qc_pot_sum = dalloc<double>(nodes, c->mesh_owned);

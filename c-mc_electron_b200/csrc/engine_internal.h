@@ -210,7 +210,7 @@ struct mcb200_ctx {
   unsigned int *hist = nullptr, *offsets = nullptr, *tile_sums = nullptr, *total = nullptr;
   int ncells = 0;
   bool heat_tallied = false;         // heat may have been tallied since the last reset
-  unsigned int *h_pinned = nullptr;  // small pinned readback area
+  unsigned int *h_pinned = nullptr;  // small pinned readback area (in h_scratch's allocation)
   MrScratch mr;                      // in mesh_owned
   // effective-potential quantum correction (mcb200_set_quantum_correction);
   // arrays in mesh_owned.  qc_on: solves give electrons the corrected field
@@ -284,7 +284,6 @@ struct mcb200_ctx {
     for (void *p : store_owned) cudaFree(p);
     for (void *p : owned) cudaFree(p);
     if (flush_buf) cudaFree(flush_buf);
-    if (h_pinned) cudaFreeHost(h_pinned);
     if (h_scratch) cudaFreeHost(h_scratch);
     if (h_tally) cudaFreeHost(h_tally);
     for (cudaEvent_t e : ev_tally)
@@ -321,6 +320,7 @@ int fail(mcb200_ctx *c, int code, const std::string &msg);
 // Host copies of the device counts (waits for the stream when a step may
 // have changed them); throws CapacityError once for a store-full flag.
 void pull_counts(mcb200_ctx *c);
+void take_counts(mcb200_ctx *c, const unsigned int *v);
 void push_counts(mcb200_ctx *c);
 // The context stream waits for pending particle statistics (before anything
 // that changes the particle store, resets or reads the statistics).  Never

@@ -117,6 +117,9 @@ int launch_batch_records(const DevTables &T, const BatchTailT<R> *tails, int n, 
 template <typename R>
 int launch_batch_tails(const BatchTailT<R> *tails, int n, uint64_t members, int scan_tiles, int *tile_first,
                        int sm_count, cudaStream_t s);
+// The members' counts (a context's dev_counts[3]) to out, pinned host memory.
+template <typename R>
+int launch_batch_counts(const BatchTailT<R> *tails, int n, unsigned int *out, cudaStream_t s);
 template <typename R>
 void launch_seed(const FlightCtx &F, const DevParticlesT<R> &P, int offset, int n, const int *cell_of,
                  const double *charge, int type, uint32_t uid0, int grid, cudaStream_t s);

@@ -1085,6 +1085,15 @@ __global__ void __launch_bounds__(256) batch_scatter_kernel(const BatchTailT<R> 
   }
 }
 
+// Every member's device counts (n, next uid, store-full flag) into pinned host
+// memory: one launch in place of a copy and a wait per member (20 steps of 32
+// members and their tallies: 12.2 ms with the copies, 11.8 this way).
+template <typename R>
+__global__ void batch_counts_kernel(const BatchTailT<R> *tails, int n, unsigned int *out) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < 3 * n) out[t] = tails[t / 3].finish.n[t % 3];
+}
+
 // ---- initial ensemble ---------------------------------------------------------
 // New particle q (uid = uid0 + q) of carrier `type` in cell cell_of[q]:
 // position uniform in the cell (init_particle_data,
@@ -1290,6 +1299,11 @@ int launch_batch_tails(const BatchTailT<R> *tails, int n, uint64_t members, int 
   return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
 template <typename R>
+int launch_batch_counts(const BatchTailT<R> *tails, int n, unsigned int *out, cudaStream_t s) {
+  batch_counts_kernel<R><<<(3 * n + 63) / 64, 64, 0, s>>>(tails, n, out);
+  return cudaGetLastError() == cudaSuccess ? 0 : 1;
+}
+template <typename R>
 void launch_append_children(const ChildSetT<R> &set, unsigned int *next_uid, const DevParticlesT<R> &dst,
                             const unsigned int *n, int capacity, unsigned int *appended, unsigned int *overflow,
                             int grid, cudaStream_t s) {
@@ -1344,6 +1358,7 @@ void launch_cell_sort(const DevParticlesT<R> &src, DevCount n, const DevParticle
   template int launch_batch_records<R>(const DevTables &, const BatchTailT<R> *, int, uint64_t, int,            \
                                        unsigned int *, int, cudaStream_t);                                      \
   template int launch_batch_tails<R>(const BatchTailT<R> *, int, uint64_t, int, int *, int, cudaStream_t);       \
+  template int launch_batch_counts<R>(const BatchTailT<R> *, int, unsigned int *, cudaStream_t);              \
   template void launch_advance_batch_steps<R>(uint32_t *, BatchInstT<R> *, int, int, cudaStream_t);           \
   template void launch_cell_sort<R>(const DevParticlesT<R> &, DevCount, const DevParticlesT<R> &, int, int, int, \
                                     unsigned int *, unsigned int *, unsigned int *, unsigned int *, int,        \

@@ -440,7 +440,8 @@ int mcb200_batch_set_pairing(mcb200_batch *batch, int enable);
 /* CUDA events after every member's enqueued work (mcb200_mark for a batch). */
 int mcb200_batch_mark(mcb200_batch *batch, int slot);
 int mcb200_batch_elapsed_ms(mcb200_batch *batch, int from, int to, double *ms);
-/* Members, batch steps taken, batched launches made, graphs captured and replayed. */
+/* Members, batch steps taken, batched flight launches (a drift pass, its flight
+ * and the draws' count as one) and paired solves made, graphs captured and replayed. */
 int mcb200_batch_info(const mcb200_batch *batch, int *members, uint64_t *steps_done, uint64_t *launches,
                       uint64_t *graph_captures, uint64_t *graph_replays);
 
