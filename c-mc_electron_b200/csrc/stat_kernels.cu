@@ -49,7 +49,7 @@ __device__ __forceinline__ void group_velocity(const DevTables &T, int itet, int
 // (36 % of issue slots; DRAM at 7 %), with short runs also by their ends.  One
 // wave of blocks, each warp with its share of chunks, and the next particles
 // fetched ahead took 142 us for 2M electrons of a bulk box to 93; shuffles
-// took 231.  A 20 nm FinFET (350k carriers): 53 us, 40 here; a bar of 10k: 9.0, 5.9.
+// took 231.  A 20 nm FinFET (350k carriers): 53 us, 40 here; a bar of 4k: 9.0, 5.9.
 constexpr int kStatThreads = 128, kStatBlocks = 5;  // four warps' 40 rows: 42.5 KB; blocks per SM
 template <typename R>
 __global__ void __launch_bounds__(kStatThreads, kStatBlocks) statistic_kernel(DevParticlesT<R> P, DevCount count, DevMesh M,
