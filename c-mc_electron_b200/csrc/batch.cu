@@ -542,6 +542,7 @@ int mcb200_batch_create(mcb200_ctx *const *ctxs, const mcb200_batch_member *memb
     for (int k = 0; k < n; ++k) first_steps[k] = members[k].first_step;
     b->member_step = first_steps;
     ck(cudaMemcpy(b->steps, first_steps.data(), n * sizeof(uint32_t), cudaMemcpyHostToDevice), "copy");
+    settle_uploads();
     b->snap.assign((size_t)n * kSnapBytes, 0);
     if (b->precision == MCB200_FLIGHT_FP32) build_tables<float>(b);
     else build_tables<double>(b);

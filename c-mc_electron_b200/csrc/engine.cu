@@ -371,6 +371,7 @@ void upload_tables(mcb200_ctx *c) {
   flight_constants(d, d.k64);
   flight_constants(d, d.k32);
   upload_tables32(c, tf, ts, kn);
+  settle_uploads();
   c->ts->vmax = 0;
   for (size_t q = 0; q < t.vt.size(); ++q)
     if (q % 4 != 3) c->ts->vmax = std::max(c->ts->vmax, std::fabs(t.vt[q]));
@@ -812,6 +813,7 @@ int mcb200_set_mesh(mcb200_ctx *c, int nx, int ny, int nz, const double *lx, con
     c->offsets = dalloc<unsigned int>(cells, c->mesh_owned);
     c->tile_sums = dalloc<unsigned int>((cells + 1023) / 1024 + 1, c->mesh_owned);
     ck(cudaStreamSynchronize(c->stream), "sync");
+    settle_uploads();
     c->mesh_set = true;
     c->cells_set = c->fields_set = c->device_set = false;
     c->fb = FieldBuffers{};
@@ -835,15 +837,16 @@ int mcb200_set_cells(mcb200_ctx *c, const int32_t *motion_rule, const int32_t *a
     ck(cudaSetDevice(c->device), "cudaSetDevice");
     const size_t cells = (size_t)c->ncells;
     DevMesh &m = c->mesh;
-    ck(cudaMemcpy(const_cast<int *>(m.motion), motion_rule, cells * 6 * sizeof(int), cudaMemcpyHostToDevice), "copy");
-    auto put_i = [&](const int *dst, const int32_t *src) {
-      if (src) ck(cudaMemcpy(const_cast<int *>(dst), src, cells * sizeof(int), cudaMemcpyHostToDevice), "copy");
-      else ck(cudaMemset(const_cast<int *>(dst), 0, cells * sizeof(int)), "memset");
+    auto put = [&](const void *dst, const void *src, size_t bytes) {
+      if (src) ck(cudaMemcpyAsync(const_cast<void *>(dst), src, bytes, cudaMemcpyHostToDevice, c->stream), "copy");
+      else ck(cudaMemsetAsync(const_cast<void *>(dst), 0, bytes, c->stream), "memset");
     };
-    put_i(m.contact, attached_contact);
-    put_i(m.in_surf, in_surf_region);
-    put_i(m.nearest_surf, nearest_surf);
-    ck(cudaMemcpy(const_cast<double *>(m.da), da, cells * sizeof(double), cudaMemcpyHostToDevice), "copy");
+    put(m.motion, motion_rule, cells * 6 * sizeof(int));
+    put(m.contact, attached_contact, cells * sizeof(int));
+    put(m.in_surf, in_surf_region, cells * sizeof(int));
+    put(m.nearest_surf, nearest_surf, cells * sizeof(int));
+    put(m.da, da, cells * sizeof(double));
+    ck(cudaStreamSynchronize(c->stream), "sync");
     for (int s = 0; s < kMaxSurfaces; ++s) m.surface_dir[s] = (surface_dir && s < n_surface_dir) ? surface_dir[s] : 0;
     m.surface_scatter = (flags & MCB200_FLAG_SURFACE_SCATTER) ? 1 : 0;
     m.surface_impurity = (flags & MCB200_FLAG_SURFACE_IMPURITY) ? 1 : 0;
@@ -885,10 +888,11 @@ int mcb200_set_surface_rates(mcb200_ctx *c, const double *e_rough, const double 
   try {
     ck(cudaSetDevice(c->device), "cudaSetDevice");
     const size_t b = (size_t)c->ncells * sizeof(double);
-    ck(cudaMemcpy(const_cast<double *>(c->mesh.e_rough), e_rough, b, cudaMemcpyHostToDevice), "copy");
-    ck(cudaMemcpy(const_cast<double *>(c->mesh.e_sphon), e_phonon, b, cudaMemcpyHostToDevice), "copy");
-    ck(cudaMemcpy(const_cast<double *>(c->mesh.h_rough), h_rough, b, cudaMemcpyHostToDevice), "copy");
-    ck(cudaMemcpy(const_cast<double *>(c->mesh.h_sphon), h_phonon, b, cudaMemcpyHostToDevice), "copy");
+    ck(cudaMemcpyAsync(const_cast<double *>(c->mesh.e_rough), e_rough, b, cudaMemcpyHostToDevice, c->stream), "copy");
+    ck(cudaMemcpyAsync(const_cast<double *>(c->mesh.e_sphon), e_phonon, b, cudaMemcpyHostToDevice, c->stream), "copy");
+    ck(cudaMemcpyAsync(const_cast<double *>(c->mesh.h_rough), h_rough, b, cudaMemcpyHostToDevice, c->stream), "copy");
+    ck(cudaMemcpyAsync(const_cast<double *>(c->mesh.h_sphon), h_phonon, b, cudaMemcpyHostToDevice, c->stream), "copy");
+    ck(cudaStreamSynchronize(c->stream), "sync");
     return MCB200_OK;
   } catch (const std::exception &e) {
     return fail(c, MCB200_ERR_CUDA, e.what());
@@ -1404,6 +1408,7 @@ int mcb200_set_device(mcb200_ctx *c, const int32_t *material, const double *dono
         f.mg = &c->mg;
       }
     }
+    settle_uploads();
     c->cg_plan = CgPlan{};
     c->cg_plan.method = c->cg_method;
     c->cg_plan.blocks = c->cg_blocks;
@@ -1482,6 +1487,7 @@ int mcb200_set_induced_current(mcb200_ctx *c, int contact) {
     double *zero = dalloc<double>(nodes, tmp);
     ck(cudaMemsetAsync(zero, 0, nodes * sizeof(double), s), "memset");
     w.bc_vapp = dupload(bc, tmp);
+    settle_uploads();
     w.bc_phims = w.vadd = w.pdop = w.density = zero;
     w.potential = dalloc<double>(nodes, tmp);
     ck(cudaMemsetAsync(w.potential, 0, nodes * sizeof(double), s), "memset");
@@ -1715,14 +1721,18 @@ int mcb200_set_quantum_correction(mcb200_ctx *c, const mcb200_quantum_params *p,
       for (size_t i = 0; i < win.size(); ++i) win[i] = make_int2(h.lower[i], h.upper[i]);
       d.window = dupload(win, c->mesh_owned);
       const double *qcl = dupload(h.qcl, c->mesh_owned);
+      const double2 *edge[3];
+      for (int a = 0; a < 3; ++a) {
+        std::vector<double2> e(h.edge[a].size() / 2);
+        for (size_t i = 0; i < e.size(); ++i) e[i] = make_double2(h.edge[a][2 * i], h.edge[a][2 * i + 1]);
+        edge[a] = dupload(e, c->mesh_owned);
+      }
+      settle_uploads();  // the launches below read them on the context's stream
       const int count[3] = {d.px, d.py, d.pz};
       for (int a = 0, at = 0; a < 3; at += count[a], ++a) {
         for (int i = 0; i < count[a]; ++i) d.width[a] = std::max(d.width[a], h.upper[at + i] - h.lower[at + i] + 1);
-        std::vector<double2> e(h.edge[a].size() / 2);
-        for (size_t i = 0; i < e.size(); ++i) e[i] = make_double2(h.edge[a][2 * i], h.edge[a][2 * i + 1]);
         double *diff = dalloc<double>((size_t)count[a] * d.width[a] * kBoxKinds, c->mesh_owned);
-        launch_erf_differences(dupload(e, c->mesh_owned), qcl + at, d.window + at, count[a], d.width[a], diff,
-                               c->stream);
+        launch_erf_differences(edge[a], qcl + at, d.window + at, count[a], d.width[a], diff, c->stream);
         d.erf_diff[a] = diff;
       }
       ck(cudaGetLastError(), "quantum set-up");

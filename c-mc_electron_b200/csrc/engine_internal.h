@@ -54,6 +54,12 @@ T *dupload(const std::vector<T> &v, std::vector<void *> &owned) {
   return p;
 }
 
+// Waits for the legacy stream's uploads and memsets.  A copy from pageable
+// memory returns once its bytes are staged, and a context's own streams do not
+// wait for the legacy stream: without this a kernel on one of them could read
+// an array before its bytes have arrived.
+inline void settle_uploads() { ck(cudaStreamSynchronize(cudaStreamLegacy), "uploads"); }
+
 // Arrays carved from one allocation, each on a 256-byte boundary: a store
 // of a dozen arrays costs one cudaMalloc (a context's set-up otherwise
 // spent tens of milliseconds in allocation calls).

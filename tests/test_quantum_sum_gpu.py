@@ -1,0 +1,54 @@
+"""The effective potential of the quantum correction: its set-up.  The band tables are computed (perf/cases.py)."""
+import importlib.util
+import os
+
+import numpy as np
+import pytest
+
+import mcb200
+
+pytestmark = pytest.mark.gpu
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+@pytest.fixture(scope="module")
+def root():
+    spec = importlib.util.spec_from_file_location("perf_cases", os.path.join(ROOT, "perf", "cases.py"))
+    m = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(m)
+    return m.tables_owner()
+
+
+def graded(root, dims):
+    """An engine on a graded mesh, and its cells' materials and quantum region:
+    silicon under an oxide layer, with a corner of neither."""
+    nx, ny, nz = dims
+    rng = np.random.default_rng(nx)
+    eng = mcb200.Engine(max_particles=64, like=root)
+    eng.set_mesh(*(np.concatenate([[0.0], np.cumsum(rng.uniform(0.3, 0.9, m))]) for m in dims))
+    material = np.full((ny, nx, nz), 3, np.int32)  # cell order (j, i, k)
+    material[:, 0, :] = 2
+    material[0, nx - 1, :nz // 2] = 1
+    region = np.zeros((ny, nx, nz), np.int32)
+    region[ny // 3:, :, nz // 4:] = 1
+    return eng, material.ravel(), region.ravel()
+
+
+def test_set_up_again(root):
+    """A correction set up again, larger, smaller and as before, is the one a
+    new engine has: no launch sees an array that is still on its way."""
+    dims = (24, 40, 22)
+    widths = [((2.0, 2.5, 1.5), (0.5, 0.4, 0.7)), ((3.0, 3.0, 3.0), (0.9, 0.8, 0.7)), ((1.0, 1.0, 1.0), (0.3, 0.3, 0.3)),
+              ((2.0, 2.5, 1.5), (0.5, 0.4, 0.7))]
+    pot = np.random.default_rng(1).normal(size=(dims[0] + 1) * (dims[1] + 1) * (dims[2] + 1)) * 10
+    again, material, region = graded(root, dims)
+    for ratio, theta in widths:
+        new, _, _ = graded(root, dims)
+        got = []
+        for eng in (again, new):
+            eng.set_quantum_correction(material, region, ratio, theta, 3.0, enable=False)
+            got.append(eng.quantum_potential(pot))
+        assert np.all(np.isfinite(got[0])) and np.any(got[0] != pot)
+        assert np.array_equal(got[0].view(np.uint64), got[1].view(np.uint64))
+        new.close()
+    again.close()
