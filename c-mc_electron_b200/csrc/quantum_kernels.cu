@@ -26,14 +26,20 @@ __global__ void erf_differences_kernel(const double2 *edge, const double *target
   out[q] = erf(e.y - target[t]) - erf(e.x - target[t]);
 }
 
-// A group of lanes per quantum node: the window is split over its (x, y)
-// rows, lane g the rows g, g + kLanes, ..., each summed in z order, and the
-// lanes' sums are added in a fixed order.  A term is the product of the
-// three tabulated erf differences in the reference's association
-// ((V + Eb) * dz) * dy) * dx: with the differences evaluated per term (six
-// erf) a FinFET's 50k targets of up to 500 terms took 1.24 ms, and in one
-// thread per target most of the device idled.  Every term reads `pot`, never
-// `out`, so no node sees another's corrected value.
+// A group of lanes per quantum node.  The window's terms are taken in the
+// reference's order (x outer, z inner), eight at a time: lane g forms term
+// f + g, the product of the three tabulated erf differences in the reference's
+// association ((V + Eb) * dz) * dy) * dx, and every lane adds the eight to its
+// running sum one after another, so the sum is the reference's to the last
+// bit (a node outside adds a zero, which changes no sum).  Every term reads
+// `pot`, never `out`, so no node sees another's corrected value.
+//
+// A 20 nm FinFET's 52k targets of up to 500 terms: 145 us; one thread per
+// target, without the shuffles, takes as long there and longer where there are
+// fewer targets (36k: 94 against 136), and six erf per term in place of the
+// tables took 1.24 ms.  (Eight partial sums, each over every eighth row, took
+// 85 us but moved the potential in its last digits, and with it the
+// trajectories of the steps that follow.)
 constexpr int kLanes = 8;
 __global__ void __launch_bounds__(256) effective_potential_kernel(const __grid_constant__ QuantumDevice q,
                                                                   const double *pot, double *out) {
@@ -45,26 +51,33 @@ __global__ void __launch_bounds__(256) effective_potential_kernel(const __grid_c
     const int n = q.list[t];
     const int pk = n % q.pz, r = n / q.pz, pi = r % q.px, pj = r / q.px;
     const int2 wx = q.window[pi], wy = q.window[q.px + pj], wz = q.window[q.px + q.py + pk];
-    const int ny = wy.y - wy.x + 1, rows = (wx.y - wx.x + 1) * ny;
+    const int ny = wy.y - wy.x + 1, nz = wz.y - wz.x + 1, terms = (wx.y - wx.x + 1) * ny * nz;
     const double *ex = q.erf_diff[0] + (size_t)pi * q.width[0] * kBoxKinds;
     const double *ey = q.erf_diff[1] + (size_t)pj * q.width[1] * kBoxKinds;
     const double *ez = q.erf_diff[2] + (size_t)pk * q.width[2] * kBoxKinds;
     double ret = 0.0;
-    for (int row = g; row < rows; row += kLanes) {
-      const int i = row / ny, j = row - i * ny;
-      const size_t base = ((size_t)(wy.x + j) * q.px + wx.x + i) * q.pz + wz.x;
-#pragma unroll 4
-      for (int k = 0; k <= wz.y - wz.x; ++k) {
-        const unsigned box = q.inside[base + k];
-        const double v = pot[base + k] + q.eb[base + k];
+    int i = 0, j = 0, k = g;  // the lane's term
+#pragma unroll 2
+    for (int f = 0; f < terms; f += kLanes) {
+      for (; k >= nz; k -= nz)
+        if (++j == ny) {
+          j = 0;
+          ++i;
+        }
+      double term = 0.0;
+      if (f + g < terms) {
+        const size_t m = ((size_t)(wy.x + j) * q.px + wx.x + i) * q.pz + wz.x + k;
+        const unsigned box = q.inside[m];
+        const double v = pot[m] + q.eb[m];
         const unsigned kinds = box - 1u;
         if (box)
-          ret += v * ez[k * kBoxKinds + ((kinds >> 4) & 3u)] * ey[j * kBoxKinds + ((kinds >> 2) & 3u)] *
+          term = v * ez[k * kBoxKinds + ((kinds >> 4) & 3u)] * ey[j * kBoxKinds + ((kinds >> 2) & 3u)] *
                  ex[i * kBoxKinds + (kinds & 3u)];
       }
-    }
+      k += kLanes;
 #pragma unroll
-    for (int o = kLanes / 2; o > 0; o >>= 1) ret += __shfl_xor_sync(mask, ret, o);
+      for (int s = 0; s < kLanes; ++s) ret += __shfl_sync(mask, term, s, kLanes);
+    }
     if (g == 0) out[n] = ret * 0.125;
   }
 }

@@ -1,4 +1,5 @@
-"""The effective potential of the quantum correction: its set-up.  The band tables are computed (perf/cases.py)."""
+"""The effective potential of the quantum correction: its set-up and the order
+of its sum.  The band tables are computed (perf/cases.py)."""
 import importlib.util
 import os
 
@@ -52,3 +53,32 @@ def test_set_up_again(root):
         assert np.array_equal(got[0].view(np.uint64), got[1].view(np.uint64))
         new.close()
     again.close()
+
+
+@pytest.mark.parametrize("dims, ratio", [((5, 7, 4), (2.0, 2.5, 1.5)), ((9, 4, 11), (1.5, 3.0, 2.0)),
+                                         ((3, 3, 20), (9.0, 9.0, 9.0))])
+def test_sum_in_the_reference_order(root, dims, ratio):
+    """The window is summed in the reference's order (x outer, z inner), one
+    term after another, to the last bit.  The terms themselves come from the
+    potentials of single nodes; a node's potential is +-2^e, so that its term
+    is theirs times a power of two, exactly, and the sum here is the sum there."""
+    px, py, pz = (d + 1 for d in dims)
+    eng, material, region = graded(root, dims)
+    eng.set_quantum_correction(material, region, ratio, (0.5, 0.4, 0.7), 0.0, enable=False)
+    nodes = px * py * pz
+    term = np.empty((nodes, nodes))  # [source][target]
+    for m in range(nodes):
+        term[m] = eng.quantum_potential(np.eye(1, nodes, m)[0]) * 8
+    rng = np.random.default_rng(2)
+    pot = rng.choice([-1.0, 1.0], nodes) * 2.0 ** rng.integers(-8, 9, nodes)
+    got = eng.quantum_potential(pot)
+    want, backwards = np.zeros(nodes), np.zeros(nodes)
+    order = [(j * px + i) * pz + k for i in range(px) for j in range(py) for k in range(pz)]
+    for m in order:
+        want += pot[m] * term[m]
+    for m in reversed(order):
+        backwards += pot[m] * term[m]
+    corrected = got != pot
+    assert corrected.sum() > nodes // 4 and np.any(want != backwards)
+    assert np.array_equal(got[corrected].view(np.uint64), (want / 8)[corrected].view(np.uint64))
+    eng.close()
