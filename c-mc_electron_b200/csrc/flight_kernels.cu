@@ -270,7 +270,9 @@ __device__ __forceinline__ void fly_interleaved(const FlightCtxT<R> &F, const Sy
         }
         if (q >= 0) {
           p = io.load(q, f, state);
-          if (p >= 0 && !(f.left_time > 0)) {
+          // (a resumed particle's draw is due even when its event came at the
+          // very end of the step)
+          if (p >= 0 && state == FlyerT<R>::kGoOn && !(f.left_time > 0)) {
             io.store(p, f, done());
             p = -1;
           }
