@@ -432,14 +432,18 @@ __device__ __forceinline__ bool FlyerT<R>::no_event() const {
     float rate = 0.0f;
     if constexpr (sizeof(R) == 4) {
       const float e = imp_emax < t.e0 ? t.e0 : (imp_emax > t.e3 ? t.e3 : imp_emax);
-      if (e < imp_ecut) rate = __fdividef(imp_a * sqrtf(e), 1.0f + imp_b * e);
+      const float d = 1.0f + imp_b * e;
+      if (e < imp_ecut) rate = __fdividef(imp_a * sqrtf(e), d);
+      if (d > 0x1p126f) return false;  // where the fast quotient is zero: a density next to none
     } else {
       const float e = fminf(fmaxf((float)imp_emax, (float)t.e0), (float)t.e3);
       if (e * (float)F.T.eV0 < 0.120f * (1.0f + 0x1p-16f))
         rate = __fdividef((float)imp_a * sqrtf(2.0f * F.T.k32.meld * e),
                           (float)imp_c * (1.0f + __fdividef(4.0f * e * F.T.k32.melt, (float)imp_b)));
     }
-    if (!(clock(u1) > fmaxf(rate, (float)TB::k(F.T).gamma_floor) * tf32)) return false;
+    // (a rate that is no number, from a density no float holds, is an event)
+    const float c1 = clock(u1);
+    if (!(c1 > rate * tf32 && c1 > (float)TB::k(F.T).gamma_floor * tf32)) return false;
   }
   if (M.surface_scatter && M.in_surf[c]) {
     float u = impurities ? 0.0f : u1;
