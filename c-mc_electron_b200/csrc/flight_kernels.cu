@@ -934,6 +934,14 @@ struct CopyRef {
   }
 };
 
+template <typename R>
+__device__ __forceinline__ int copy_count(const ChildSetT<R> &set) {
+  int total = 0;
+#pragma unroll
+  for (int q = 0; q < kChildGenerations; ++q) total += min((int)*set.g[q].count, set.g[q].capacity);
+  return total;
+}
+
 // Block `block` of `blocks` (256 threads).
 template <typename R>
 __device__ __forceinline__ void append_block(const ChildSetT<R> &set, const unsigned int *next_uid,
@@ -1026,14 +1034,22 @@ __global__ void __launch_bounds__(256) batch_records_kernel(const __grid_constan
     if (c < b.cells) cell_record(T, b.M, static_cast<Rec *>(b.records), c);
   }
 }
-constexpr int kAppendBlocks = 8;  // per member: 32 copies a block, a step of 50k particles makes a few
+// The members' copies, 32 a block, whatever their numbers: ranking a member's
+// copies is quadratic in them, so those of one with many are spread over the
+// grid like those of a step of it alone.  Four members of 500k FP32 carriers
+// with 471, 1857 and 6521 copies each: 20, 75 and 532 us with eight blocks a
+// member, 10, 16 and 80 this way (one member alone: 8, 13, 55).
 template <typename R>
-__global__ void __launch_bounds__(256) batch_append_kernel(const BatchTailT<R> *tails, uint64_t members) {
-  const int k = (int)blockIdx.x / kAppendBlocks;
-  if (!((members >> k) & 1ull)) return;
-  const BatchTailT<R> &b = tails[k];
-  append_block(b.set, b.finish.next_uid, b.src, b.finish.n, b.capacity, b.counters.appended, b.overflow,
-               (int)blockIdx.x % kAppendBlocks, kAppendBlocks);
+__global__ void __launch_bounds__(256) batch_append_kernel(const BatchTailT<R> *tails, int n, uint64_t members) {
+  __shared__ int first[kMaxBatch + 1];
+  MemberPrefix tp{first, n};
+  tp.fill([&](int k) { return (members >> k) & 1ull ? (copy_count(tails[k].set) + 31) / 32 : 0; });
+  for (int t = blockIdx.x; t < first[n]; t += gridDim.x) {
+    const int k = tp.find(t);
+    const BatchTailT<R> &b = tails[k];
+    append_block(b.set, b.finish.next_uid, b.src, b.finish.n, b.capacity, b.counters.appended, b.overflow,
+                 t - first[k], first[k + 1] - first[k]);
+  }
 }
 template <typename R>
 __device__ __forceinline__ int tail_count(const BatchTailT<R> &b) {
@@ -1294,7 +1310,7 @@ int launch_batch_records(const DevTables &T, const BatchTailT<R> *tails, int n, 
 template <typename R>
 int launch_batch_tails(const BatchTailT<R> *tails, int n, uint64_t members, int scan_tiles, int *tile_first,
                        int sm_count, cudaStream_t s) {
-  batch_append_kernel<R><<<n * kAppendBlocks, 256, 0, s>>>(tails, members);
+  batch_append_kernel<R><<<4 * sm_count, 256, 0, s>>>(tails, n, members);
   batch_histogram_kernel<R><<<8 * sm_count, 256, 0, s>>>(tails, n, members, tile_first);
   batch_scan_kernel<R><<<std::max(scan_tiles, 1), kScanThreads, 0, s>>>(tails, n, members);
   batch_scatter_kernel<R><<<8 * sm_count, 256, 0, s>>>(tails, n, tile_first);
