@@ -194,6 +194,7 @@ struct FlightListsT {
   double *left_time;
   uint2 *progress;              // {draws made, events | zero_run << 20}
   uint32_t *info;               // packed flags
+  int *copies;                  // made so far (their streams' numbers)
 };
 
 // Bytes of one particle in the store.

@@ -107,7 +107,7 @@ void alloc_particles(DevParticlesT<R> &d, size_t cap, std::vector<void *> &owned
 template <typename R>
 FlightListsT<R> flight_lists(const DevParticlesT<R> &b, unsigned int *count) {
   return FlightListsT<R>{b.uid, b.meta, count, b.x, b.y, b.z, b.kx, b.ky, b.kz, b.energy,
-                         reinterpret_cast<uint2 *>(b.charge), b.cell};
+                         reinterpret_cast<uint2 *>(b.charge), b.cell, b.itet};
 }
 
 template <typename R>

@@ -1178,8 +1178,8 @@ struct FlyerT {
     m.progress[p] = make_uint2(n, (uint32_t)loop | (uint32_t)zero_run << 20);
     m.info[p] = (get_tet ? 1u : 0u) | (get_ph ? 2u : 0u) | (get_imp ? 4u : 0u) | (get_surf ? 8u : 0u) |
                 (self ? 16u : 0u) | (imp_pending ? 32u : 0u) | (uint32_t)loc_mode << 6 | (uint32_t)draw_kind << 8 |
-                (uint32_t)idir << 10 | (uint32_t)itetdir << 13 | (uint32_t)ev << 15 |
-                (uint32_t)nchild << 20;
+                (uint32_t)idir << 10 | (uint32_t)itetdir << 13 | (uint32_t)ev << 15;
+    m.copies[p] = nchild;
   }
   // After the store's part is loaded.
   __device__ __forceinline__ void resume(const FlightListsT<R> &m, int p) {
@@ -1207,7 +1207,7 @@ struct FlyerT {
     idir = (int)(w >> 10 & 7u);
     itetdir = (int)(w >> 13 & 3u);
     ev = (int)(w >> 15 & 7u);
-    nchild = (int)(w >> 20);
+    nchild = m.copies[p];
     catch_ = too_far = false;
     surf_gamma = imp_gamma = 0;
     load_cell_fields();

@@ -8,6 +8,7 @@ import numpy as np
 import pytest
 
 import mcb200
+from mcb200.workloads import motion_rules, uniform_fields
 from test_flight_launches_gpu import box, by_uid, cases, ensemble, philox_block0, root  # noqa: F401 (fixtures)
 
 pytestmark = pytest.mark.gpu
@@ -71,3 +72,45 @@ def test_draw_due_at_the_end_of_the_step(root, precision):  # noqa: F811
     assert np.any(whole["uid"] == p["uid"][q])
     for k in ("events", "phonon", "impurity"):
         assert tw[k] == parts[0][1][k] + parts[1][1][k], k
+
+
+def test_copies_beyond_4096_in_a_step(root):  # noqa: F811
+    """A carrier that makes thousands of copies between two of its draws (a
+    plane of cells 0.1 pm thick between a mirror and a face that makes copies):
+    each copy has a stream of its own, numbered on through a launch for the
+    draws as in one launch."""
+    precision, (nx, ny, nz), thin, specials = mcb200.FLIGHT_FP64, (4, 6, 4), 3, 8
+    n = SPLIT[precision] + 1
+    widths = np.full(ny, 5e-9)
+    widths[thin] = 1e-13
+
+    def slab(count):
+        eng = mcb200.Engine(max_particles=1 << 22, precision=precision, like=root)
+        u = eng.units()
+        x, y, z = (np.concatenate([[0.0], np.cumsum(w)]) / u["spr0"]
+                   for w in (np.full(nx, 5e-9), widths, np.full(nz, 5e-9)))
+        eng.set_mesh(x, y, z)
+        faces = motion_rules(nx, ny, nz).reshape(ny, nx, nz, 6)
+        reflect, genref, left, right = 2, 8, 2, 3
+        faces[thin - 1, :, :, right] = faces[thin, :, :, left] = faces[thin + 1, :, :, left] = reflect
+        faces[thin, :, :, right] = genref
+        cells = nx * ny * nz
+        eng.set_cells(faces.reshape(-1), np.zeros(cells))
+        eng.set_fields(*uniform_fields(eng, 0.0, 1e23))
+        rng = np.random.default_rng(1)
+        plane = rng.permutation(np.repeat([0, 1, 2, 4, 5], (count - specials) // 5 + 1))[:count - specials]
+        cell = np.concatenate([np.full(specials, thin * nx * nz + 5),
+                               plane * nx * nz + rng.integers(0, nx * nz, count - specials)])
+        eng.seed(cell, np.full(count, -1e-3), 0, 5)
+        return eng, u
+
+    ends = []
+    for count in (n, 300):
+        eng, u = slab(count)
+        eng.step(0, 7, 6e-14 / u["time0"])
+        p, t = by_uid(eng), eng.tallies()
+        ends.append({k: v[(p["uid"] < specials) | (p["uid"] >= count)] for k, v in p.items()})
+        ends[-1]["uid"] = np.where(ends[-1]["uid"] < specials, ends[-1]["uid"], ends[-1]["uid"] - count + specials)
+        assert t["generated"] > specials * 4096 and t["child_overflow"] == 0
+        eng.close()
+    same(*ends)
