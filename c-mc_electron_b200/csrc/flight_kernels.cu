@@ -39,12 +39,6 @@ constexpr int kFlightBlocks = sizeof(R) == 4 ? MCB200_FLIGHT_BLOCKS_F32 : MCB200
 // two blocks per SM, 541 at three).
 template <typename R>
 constexpr int kNoDrawBlocks = sizeof(R) == 4 ? 3 : MCB200_FLIGHT_BLOCKS_F64;
-// Threads per block of the flight kernels (a tuning define like the above).
-#ifndef MCB200_FLIGHT_THREADS
-#define MCB200_FLIGHT_THREADS 256
-#endif
-constexpr int kFlightThreads = MCB200_FLIGHT_THREADS;
-
 // Resident blocks per SM of the drift pass (measured best: FP32 of 4 to 6, 80 us
 // for 2M electrons; FP64 of 2 to 4, 155 us).
 #ifndef MCB200_DRIFT_BLOCKS_F32
@@ -206,7 +200,6 @@ struct ChildIO {
 template <typename R, bool kLaneEvents, bool kDraws, class IO>
 __device__ __forceinline__ void fly_interleaved(const FlightCtxT<R> &F, const SymSmemT<R> &S, const IO &io, int n,
                                                 unsigned int *ticket) {
-  static_assert(kFlightThreads == FlyerT<R>::kRingStride, "one ring column a thread");
   __shared__ R ring[FlyerT<R>::kRing * FlyerT<R>::kRingStride];
   FlyerT<R> f(F, S, ring + threadIdx.x);
   f.n_ph = f.n_imp = 0;
@@ -1124,7 +1117,7 @@ __global__ void batch_counts_kernel(const BatchTailT<R> *tails, int n, unsigned 
 // cell-relative).
 
 template <typename R>
-__global__ void __launch_bounds__(256) seed_kernel(FlightCtx F, DevParticlesT<R> P, int offset, int n,
+__global__ void __launch_bounds__(kFlightThreads) seed_kernel(FlightCtx F, DevParticlesT<R> P, int offset, int n,
                                                    const int *cell_of, const double *charge, int type,
                                                    uint32_t uid0) {
   __shared__ SymSmem S;
@@ -1188,7 +1181,7 @@ __global__ void __launch_bounds__(256) seed_kernel(FlightCtx F, DevParticlesT<R>
 template <typename R>
 void launch_seed(const FlightCtx &F, const DevParticlesT<R> &P, int offset, int n, const int *cell_of,
                  const double *charge, int type, uint32_t uid0, int grid, cudaStream_t s) {
-  if (n > 0) seed_kernel<R><<<grid, 256, 0, s>>>(F, P, offset, n, cell_of, charge, type, uid0);
+  if (n > 0) seed_kernel<R><<<grid, kFlightThreads, 0, s>>>(F, P, offset, n, cell_of, charge, type, uid0);
 }
 // Blocks of the persistent flight kernels: enough to fill every SM at the
 // kernel's occupancy, fewer when there are fewer particles than warps.

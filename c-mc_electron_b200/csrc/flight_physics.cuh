@@ -45,6 +45,14 @@ constexpr int kMaxStateTries = 10000;
 // FP32 flight: consecutive zero-length events after which a particle is
 // taken as stuck (counted in kCntZeroTime and caught).
 constexpr int kMaxZeroTimeEvents = 64;
+// Threads per block of the kernels that fly or seed particles (a tuning define
+// like those of flight_kernels.cu; whole warps, at most 512: a column of the
+// draws' ring each).
+#ifndef MCB200_FLIGHT_THREADS
+#define MCB200_FLIGHT_THREADS 256
+#endif
+constexpr int kFlightThreads = MCB200_FLIGHT_THREADS;
+static_assert(kFlightThreads % 32 == 0 && kFlightThreads <= 512, "whole warps, the ring in shared memory");
 // Opt-in event census (build with -DMCB200_FLIGHT_EVENT_STATS=1): counters
 // 10-15 of the tallies count the flight loop's passes by the event that
 // ended them and the work of the rare shared tails, for the design record
@@ -254,7 +262,7 @@ struct FlyerT {
   // draws of an event pass come at several places, where other lanes may or
   // may not draw; one stock per pass computes the block once for all lanes
   // that need one, instead of at each place for the lanes that do there.
-  static constexpr uint32_t kRing = 8, kRingStride = 256;
+  static constexpr uint32_t kRing = 8, kRingStride = kFlightThreads;
   static constexpr uint32_t kBlockDraws = sizeof(R) == 4 ? 4 : 2;
   __device__ __forceinline__ void stock(uint32_t k) {
 #pragma unroll 1
