@@ -56,7 +56,7 @@ struct DevTables32 {
   const TetFlightT<float> *tf;
   const TetShapeT<float> *ts;
   const float4 *knode;
-  const float *gamtet, *energy, *sumscatt, *scatte, *dose, *scattiie, *scatth, *dosh, *scattiih, *dostetmax;
+  const float *energy, *sumscatt, *scatte, *dose, *scattiie, *scatth, *dosh, *scattiih, *dostetmax;
 };
 
 // Constants in the flight's arithmetic, each rounded as the reference's
@@ -89,7 +89,6 @@ struct DevTables {
   const int4 *tnode;         // [nt] node indices
   const int4 *tneib;         // [nt] neighbour code per face
   const int *ibt;            // [nt]
-  const double *gamtet;      // [nt]
   const double4 *knode;      // [nk] (kx, ky, kz, E)
   const double *energy;      // [kNT]
   const double *sumscatt;    // [kNT][kMNB]

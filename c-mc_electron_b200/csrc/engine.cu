@@ -244,7 +244,6 @@ void upload_tables32(mcb200_ctx *c, const std::vector<TetFlight> &tf, const std:
   d.tf = dupload(tf32, c->ts->owned);
   d.ts = dupload(ts32, c->ts->owned);
   d.knode = dupload(kn32, c->ts->owned);
-  d.gamtet = dupload(to_float(t.gamtet), c->ts->owned);
   d.energy = dupload(to_float(t.energy), c->ts->owned);
   d.sumscatt = dupload(to_float(t.sumscatt), c->ts->owned);
   d.scatte = dupload(to_float(t.scatte), c->ts->owned);
@@ -317,7 +316,6 @@ void upload_tables(mcb200_ctx *c) {
   d.tnode = dupload(tn, c->ts->owned);
   d.tneib = dupload(tb, c->ts->owned);
   d.ibt = dupload(t.ibt, c->ts->owned);
-  d.gamtet = dupload(t.gamtet, c->ts->owned);
   std::vector<double4> kn(t.nk);
   for (int i = 0; i < t.nk; ++i) kn[i] = make_double4(t.xkk[i], t.ykk[i], t.zkk[i], t.eek[i]);
   d.knode = dupload(kn, c->ts->owned);
