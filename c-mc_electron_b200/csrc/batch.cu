@@ -45,7 +45,7 @@ struct mcb200_batch {
   unsigned int *counts = nullptr;  // pinned: [n][3], the members' device counts
   int record_tiles = 0, scan_tiles = 0;  // of all members
   uint32_t *steps = nullptr;       // device: step number of each member
-  unsigned int *tickets = nullptr;  // device: work counters of the batched launches (main, 4 copy generations, side)
+  unsigned int *tickets = nullptr;  // device: work counters of the batched launches (kFlightTickets: flight, draws, 4 copy generations; side)
   bool overlap = true;              // fly the members not solving Poisson beside the solves
   bool pair_solves = true;          // two multigrid solves of the same shape per cooperative launch
   bool smem_table = false;          // batched flights copy the member table into shared memory (else read in place)

@@ -2079,9 +2079,9 @@ StepFinish step_finish(mcb200_ctx *c) {
 template StepCounters step_counters<float>(mcb200_ctx *);
 template StepCounters step_counters<double>(mcb200_ctx *);
 
-// Before the flights of a step: the induced-current tally (when on), work
-// counters, the FP32 per-cell records, and zeroed copy counters of every
-// generation and of the sink.
+// Before the flights of a step: the induced-current tally (when on), and with
+// `records` the per-cell records of the flight's precision and the zeroed work
+// counters, list counts and copy counters (every generation's and the sink's).
 template <typename R>
 void step_prepare(mcb200_ctx *c, bool records) {
   cudaStream_t s = c->stream;

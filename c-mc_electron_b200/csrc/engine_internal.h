@@ -233,7 +233,7 @@ struct mcb200_ctx {
   MgDevice mg{};                            // multigrid hierarchy of the Poisson stencil (mcb200_set_device)
   int cg_method = kCgAuto, cg_blocks = 0;   // mcb200_set_poisson_solver
   bool device_set = false;
-  double *h_scratch = nullptr;  // pinned, 16 doubles
+  double *h_scratch = nullptr;  // pinned: 16 doubles, then the small tallies (kSmallTallies), then h_pinned
   // pipelined contact-tally readback (mcb200_tallies_enqueue / _collect):
   // kTallyRing slots of the contact tallies and the store-full flag, pinned
   static constexpr int kTallyRing = 4;

@@ -54,9 +54,19 @@ constexpr int kDriftBlocks = sizeof(R) == 4 ? MCB200_DRIFT_BLOCKS_F32 : MCB200_D
 // to a launch of their own (draws_apart; tuning defines).  Without the draws
 // the flight's loop has two thirds of the code and no register spills (FP64),
 // or fits three blocks per SM (FP32); the second launch costs the latency of
-// a draw and the rest of its particles' steps, 30-40 us.  Measured, one
-// launch against two: FP64 2M electrons 1326 -> 972 us, 100k 196 -> 173, bar of
-// 4800 worse; FP32 2M 756 -> 666, FinFET of 530k 112 -> 118, 76k 73 -> 83.
+// a draw and the rest of its particles' steps, 30-40 us.  Measured, a whole
+// step in us with one launch and with two (bulk boxes at 1 to 100 kV/cm, n-FinFETs;
+// per cent by which two are slower):
+//   FP64  bulk   5k 92-97 / 118-122 (+23 to +30)   20k 131-140 / 146-155 (+11)
+//                40k +4 to 0   65,536 +1 to -6   100k -2 to -11   400k -14 to -16
+//                2M 1570-1814 / 1213-1362 (-23 to -25)
+//         FinFET 192k -7   487k -14   1.26M -15
+//   FP32  bulk   5k 70-73 / 98-101 (+39)   100k +12 to +23   400k +1 to -1
+//                700k -3 to -8   1M 492-579 / 455-515 (-8 to -11)
+//                2M 907-1070 / 807-923 (-11 to -14)
+//         FinFET 192k +7   285k +5   487k -4   1.26M -11
+// FP64's line lies where a cold box gains nothing yet; FP32's above the crossing
+// (400k-500k), where every ensemble gains: up to it one launch gives away 3-8 %.
 #ifndef MCB200_DRAWS_APART_F32
 #define MCB200_DRAWS_APART_F32 1000000
 #endif

@@ -1,14 +1,16 @@
 // flight_physics.cuh -- per-particle full-band free flight on the device.
 //
-// One thread owns one particle for one time step and runs the reference's
-// event loop (MeshQuantities::particle_fly, src/mcmodel.cpp:1874-2161) with
-// every routine it calls restated as device code below.  Each routine cites
+// A lane flies one particle at a time through the reference's event loop
+// (MeshQuantities::particle_fly, src/mcmodel.cpp:1874-2161), with every
+// routine it calls restated as device code below; final states are drawn by
+// the whole warp for one lane after another.  Each routine cites
 // the reference lines it follows.  Arithmetic is IEEE double in the
 // reference's operand order and this code is compiled without FMA
 // contraction, so with the same random draws (include/mcb200_rng.h) the
 // discrete outcomes (tetrahedron, wedge, cell, event type, final state) are
-// the reference's; only libm transcendentals (log, sin, cos, pow with a
-// negative exponent) may differ from glibc by an ulp.
+// the reference's; only libm transcendentals (log, sincos) and the impurity
+// event's 1 / (q q), the reference's pow(q, -2.0), may differ from glibc by an
+// ulp or so.
 //
 // Device-side differences from the reference, each deliberate:
 //  * no process exit: conditions where the reference calls exit() or loops

@@ -45,11 +45,12 @@ __device__ __forceinline__ void group_velocity(const DevTables &T, int itet, int
 // 10 (2 b + a) + 5 d + t holds tally t of corner (i + a, j + b, k + d).
 // Lane l owns row l, and lanes 0-7 rows 32-39 too.
 //
-// Bound by the latency of about 800 instructions a chunk at 20 warps per SM
-// (36 % of issue slots; DRAM at 7 %), with short runs also by their ends.  One
+// Bound by the latency of about 800 instructions a chunk at 20 warps per SM and
+// by shared memory (issue slots at 47 %, the SM's memory pipes at 77, DRAM at
+// 10), with short runs also by their ends.  One
 // wave of blocks, each warp with its share of chunks, and the next particles
 // fetched ahead took 142 us for 2M electrons of a bulk box to 93; shuffles
-// took 231.  A 20 nm FinFET (350k carriers): 53 us, 40 here; a bar of 4k: 9.0, 5.9.
+// took 231.  A 20 nm FinFET (511k carriers): 53 us, 40 here; a bar of 4k: 9.0, 5.9.
 constexpr int kStatThreads = 128, kStatBlocks = 5;  // four warps' 40 rows: 42.5 KB; blocks per SM
 template <typename R>
 __global__ void __launch_bounds__(kStatThreads, kStatBlocks) statistic_kernel(DevParticlesT<R> P, DevCount count, DevMesh M,

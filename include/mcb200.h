@@ -441,7 +441,8 @@ int mcb200_batch_set_pairing(mcb200_batch *batch, int enable);
 int mcb200_batch_mark(mcb200_batch *batch, int slot);
 int mcb200_batch_elapsed_ms(mcb200_batch *batch, int from, int to, double *ms);
 /* Members, batch steps taken, batched flight launches (a drift pass, its flight
- * and the draws' count as one) and paired solves made, graphs captured and replayed. */
+ * and the draws' count as one; the records, append and sort that members share
+ * are not counted) and paired solves made, graphs captured and replayed. */
 int mcb200_batch_info(const mcb200_batch *batch, int *members, uint64_t *steps_done, uint64_t *launches,
                       uint64_t *graph_captures, uint64_t *graph_replays);
 
@@ -453,7 +454,8 @@ int mcb200_batch_info(const mcb200_batch *batch, int *members, uint64_t *steps_d
  * every step cost 3 % of the step).
  * mcb200_get_timing: out[0..n) = flight-kernel ms and flight-kernel launches
  * of the timed steps, whole-step ms and steps timed, particles flown (all
- * steps), engine kernel launches (all steps). */
+ * steps), engine kernel launches (all steps; those a batch makes for several
+ * members at once are not among a member's). */
 int mcb200_set_timing(mcb200_ctx *ctx, int enable);
 int mcb200_get_timing(const mcb200_ctx *ctx, double *out, int n);
 
