@@ -29,13 +29,20 @@ sort), refresh.  Timed twice: FP32 flight and plain FP64 flight.
 
 --impl reference times the same reference routines on all host cores, one
 process per core.
+
+Where the reference's files are not there, the engine's band tables are
+computed (perf/cases.py; `data` says so) and the reference's routines are
+`unavailable`.
 """
 from __future__ import annotations
 
 import argparse
+import atexit
+import functools
 import json
 import multiprocessing as mp
 import os
+import shutil
 import statistics
 import subprocess
 import sys
@@ -49,6 +56,32 @@ sys.path.insert(0, os.path.join(ROOT, "c-mc_electron_b200"))
 
 METRIC = "particle-steps/s"
 from mcb200.workloads import BULK_BOX as BOX  # noqa: E402
+
+ORACLE = os.path.join(ROOT, "oracle", "_ref", "libref_oracle.so")
+NO_ORACLE = "the reference's sources are not there: its routines were not built (oracle/_ref)"
+
+
+@functools.lru_cache(maxsize=None)
+def table_dir() -> str:
+    """The folder of the band tables: the staged files or, without them, computed ones."""
+    from mcb200 import DEFAULT_TABLE_DIR
+
+    if os.path.exists(os.path.join(DEFAULT_TABLE_DIR, "bs.si.asc")):
+        return DEFAULT_TABLE_DIR
+    sys.path.insert(0, ROOT)
+    from perf import cases
+
+    folder = tempfile.mkdtemp(prefix="mcb200_tables_")
+    atexit.register(shutil.rmtree, folder, ignore_errors=True)
+    cases.write_tables(folder)
+    return folder
+
+
+def data_kind() -> str:
+    from mcb200 import DEFAULT_TABLE_DIR
+
+    return "synthetic" if table_dir() == DEFAULT_TABLE_DIR else "synthetic, band tables computed (pseudopotential)"
+
 
 # read + write of the particle state: 80 B (FP64 plain), 56 B (FP32 flight)
 BYTES_PER_PARTICLE_STEP = {"fp64": 160, "fp32": 112}
@@ -123,7 +156,7 @@ def measure_precision(args, rank: int, world: int, device: int, precision: str):
 
     seed = 1 + rank
     prec = mcb200.FLIGHT_FP32 if precision == "fp32" else mcb200.FLIGHT_FP64
-    eng, dt, fields = bulk_box_engine(args.particles, seed, device, precision=prec)
+    eng, dt, fields = bulk_box_engine(args.particles, seed, device, precision=prec, table_dir=table_dir())
     n0 = eng.num_particles()
     for s in range(args.warmup):
         eng.step(s, seed, dt)
@@ -212,7 +245,8 @@ def finfet_run(args, device: int, precision: str, readback: bool = False, profil
         d = decks.finfet(tmp, total_step=args.warmup + steps + 1, heat_steps=0, stat_step=100000)
         prec = mcb200.FLIGHT_FP32 if precision == "fp32" else mcb200.FLIGHT_FP64
         with ClockSampler(device) as clocks:
-            rep = mcb200.run_deck(d["input"], device=device, precision=prec, max_steps=args.warmup + steps,
+            rep = mcb200.run_deck(d["input"], device=device, precision=prec, table_dir=table_dir(),
+                                  max_steps=args.warmup + steps,
                                   warmup_steps=args.warmup, max_heat_steps=0, poisson_every=FINFET_POISSON_EVERY,
                                   write_outputs=False, readback_every_step=readback,
                                   flush_l2_bytes=0 if (readback or profile_steps) else FLUSH_BYTES,
@@ -262,7 +296,7 @@ def engine_arm(args, rank: int, world: int, device: int):
     return {
         "metric": METRIC, "value": value["fp32"], "unit": "particle-steps/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": r32["timed_device_ms"] / max(r32["timed_steps"], 1),
-        "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32", "data": "synthetic",
+        "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32", "data": data_kind(),
         "config": finfet_config(world),
         "precision": "fp32-flight (FP64 energy / time bookkeeping); fp64_plain: all-FP64 flight",
         "carriers_initial": r32["initial_particles"],
@@ -306,7 +340,7 @@ def batch_arm(args, device: int) -> dict:
     from mcb200 import batching
 
     t0 = time.perf_counter()
-    members, root = batching.build_mix(n=BATCH_MEMBERS, seed=4, precision=mcb200.FLIGHT_FP32)
+    members, root = batching.build_mix(n=BATCH_MEMBERS, seed=4, precision=mcb200.FLIGHT_FP32, table_dir=table_dir())
     setup_s = time.perf_counter() - t0
     batch = mcb200.Batch([(m.eng, m.cfg) for m in members])
     batch.use_graphs(True)
@@ -348,7 +382,7 @@ def batch_arm(args, device: int) -> dict:
            "value": batched, "ms_per_step": ms_b, "unbatched_value": alone, "unbatched_ms_per_step": ms_a,
            "batched_over_unbatched": batched / alone, "steps": BATCH_STEPS, "windows": windows, "autotune": tune,
            "graph_captures": info["graph_captures"], "graph_replays": info["graph_replays"],
-           "setup_s": setup_s, "clocks": clocks.summary(), "dtype": "f32", "data": "synthetic",
+           "setup_s": setup_s, "clocks": clocks.summary(), "dtype": "f32", "data": data_kind(),
            "config": "64 members (seed 4): bulk n-Si boxes 20^3-80x40x50 cells, E_x U[1,100] kV/cm, and "
                      "self-consistent n-FinFETs Lg {15,20,30} nm, Vg U[0,0.8] V, Vd 0.7 V, surface scattering, "
                      "Poisson every 10 steps (staggered), MultipleRefresh every 50; N log-uniform 5k-500k "
@@ -382,7 +416,7 @@ def serve_arm(args, device: int) -> dict:
 
     with tempfile.TemporaryDirectory() as tmp:
         reqs = serving.make_requests(tmp, n=SERVE_REQUESTS, seed=5, rate=4.0)
-        srv = mcb200.Server(device=device, precision=mcb200.FLIGHT_FP32, quantum_steps=SERVE_QUANTUM)
+        srv = mcb200.Server(table_dir(), device=device, precision=mcb200.FLIGHT_FP32, quantum_steps=SERVE_QUANTUM)
         with ClockSampler(device) as clocks:
             res, st, wall = serving.serve(srv, reqs, max_wall_s=900, max_steps=args.serve_max_steps, min_windows=5,
                                           warm_windows_cold=6, warm_windows_warm=2, poisson_every=10,
@@ -443,6 +477,8 @@ FINFET_REQUEST = (300000, 50000)  # electrons, holes requested in the deck
 def cpu_baseline(steps: int = 10):
     """The reference's routines on the engine arm's FinFET (511,200 carriers),
     one core: one Poisson solve and `steps` flights (about 10-15 s)."""
+    if not os.path.exists(ORACLE):
+        return {"unavailable": NO_ORACLE}
     ps, t = _oracle_sample((99, *FINFET_REQUEST, steps))
     return {"value": ps / t, "unit": "particle-steps/s", "cores": 1, "kind": "reference",
             "sample": f"the reference's density_and_field (every {FINFET_POISSON_EVERY} steps) + update_particle on "
@@ -453,6 +489,8 @@ def cpu_baseline(steps: int = 10):
 def reference_arm(args, rank: int, world: int):
     if rank != 0:
         return None
+    if not os.path.exists(ORACLE):
+        return {"impl": "reference", "unavailable": NO_ORACLE}
     cores = len(os.sched_getaffinity(0)) if hasattr(os, "sched_getaffinity") else (os.cpu_count() or 1)
     steps = max(3, min(args.steps, 20))
     ctx = mp.get_context("spawn")
@@ -552,6 +590,8 @@ def main():
     if args.warmup < 3:
         args.warmup = 3
     rank, world, local = dist_init()
+    if args.impl == "engine":
+        table_dir()  # before anything is timed or its clocks are sampled
     if args.impl == "reference":
         out = reference_arm(args, rank, world)
     elif args.workload == "batch":
