@@ -51,7 +51,9 @@ __global__ void __launch_bounds__(256) effective_potential_kernel(const __grid_c
     const int n = q.list[t];
     const int pk = n % q.pz, r = n / q.pz, pi = r % q.px, pj = r / q.px;
     const int2 wx = q.window[pi], wy = q.window[q.px + pj], wz = q.window[q.px + q.py + pk];
-    const int ny = wy.y - wy.x + 1, nz = wz.y - wz.x + 1, terms = (wx.y - wx.x + 1) * ny * nz;
+    // (a window can be empty, its end before its start: under a negative ratio)
+    const int nx = max(wx.y - wx.x + 1, 0), ny = max(wy.y - wy.x + 1, 0), nz = max(wz.y - wz.x + 1, 0);
+    const int terms = nx * ny * nz;
     const double *ex = q.erf_diff[0] + (size_t)pi * q.width[0] * kBoxKinds;
     const double *ey = q.erf_diff[1] + (size_t)pj * q.width[1] * kBoxKinds;
     const double *ez = q.erf_diff[2] + (size_t)pk * q.width[2] * kBoxKinds;

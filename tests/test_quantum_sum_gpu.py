@@ -1,5 +1,6 @@
 """The effective potential of the quantum correction: its set-up and the order
 of its sum.  The band tables are computed (perf/cases.py)."""
+import bisect
 import importlib.util
 import os
 
@@ -81,4 +82,42 @@ def test_sum_in_the_reference_order(root, dims, ratio):
     corrected = got != pot
     assert corrected.sum() > nodes // 4 and np.any(want != backwards)
     assert np.array_equal(got[corrected].view(np.uint64), (want / 8)[corrected].view(np.uint64))
+    eng.close()
+
+
+def widths(dims):
+    rng = np.random.default_rng(dims[0])  # as graded's mesh
+    return [rng.uniform(0.3, 0.9, m) for m in dims]
+
+
+def window(line, reach):
+    """An axis's windows as the set-up's lower_bound / upper_bound walk finds them."""
+    low = up = 0
+    out = []
+    for i, at in enumerate(line):
+        low = bisect.bisect_left(line, at - reach, min(low, i), i)
+        up = bisect.bisect_right(line, at + reach, up)
+        low -= low > 0
+        up -= up == len(line)
+        out.append((low, up))
+    return out
+
+
+@pytest.mark.parametrize("ratio", [(2.0, -6.0, -6.0), (-6.0, 2.0, -6.0), (-6.0, -6.0, -6.0), (2.0, 2.0, -6.0)])
+def test_empty_windows(root, ratio):
+    """Under a negative ratio a window ends before its start, on two axes at
+    once too: it holds no node, and the sum over it is zero."""
+    dims, theta = (8, 11, 9), (0.5, 0.4, 0.7)
+    px, py, pz = (d + 1 for d in dims)
+    eng, material, region = graded(root, dims)
+    eng.set_quantum_correction(material, region, ratio, theta, 0.0, enable=False)
+    pot = np.random.default_rng(3).normal(size=px * py * pz)
+    got = eng.quantum_potential(pot)
+    lines = [np.concatenate([[0.0], np.cumsum(w)]) for w in widths(dims)]
+    empty = [np.array([up < low for low, up in window(list(line), r * t)])
+             for line, r, t in zip(lines, ratio, theta)]
+    none = (empty[1][:, None, None] | empty[0][None, :, None] | empty[2][None, None, :]).ravel()
+    corrected = got != pot
+    assert np.all(np.isfinite(got)) and np.any(none & corrected)
+    assert np.all(got[none & corrected] == 0.0)
     eng.close()
